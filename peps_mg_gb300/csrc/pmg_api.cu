@@ -694,11 +694,12 @@ int Ctx::build(const pmg_config_t *c, cudaStream_t s)
     // A level too large for one CTA is kept on the grid kernels.
     while (tail_l0 <= nl && lv[tail_l0].total > kTailMaxCells) ++tail_l0;
     // Tail block size: about two cells per thread at the largest tail level (barriers of
-    // a 1024-thread CTA dominate the coarsest solve of a few cells).
+    // a large CTA dominate the small levels), and the threads the coarsest solver wants.
     {
         long long cells = 1;
         for (int l = tail_l0; l <= nl; ++l) cells = std::max(cells, (long long)lv[l].n[0] * lv[l].n[1] * lv[l].n[2]);
-        tail_threads = (int)std::min<long long>(1024, std::max<long long>(64, ((cells / 2 + 31) / 32) * 32));
+        tail_threads = (int)std::min<long long>(kTail64Threads, std::max<long long>(64, ((cells / 2 + 31) / 32) * 32));
+        tail_threads = std::max(tail_threads, chip_threads(lv[nl].n[0], lv[nl].n[1], lv[nl].n[2]));
     }
 
     // ---- device arrays -------------------------------------------------------------

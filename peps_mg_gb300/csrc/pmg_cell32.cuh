@@ -546,9 +546,11 @@ __device__ void tail32_run(const TailDesc<float> &D, const LevelK<float> *Ls, co
         const LevelK<double> &C = D.C64;
         float *x = xs[D.nl];
         const float *b = bs[D.nl];
-        if (C.sz * (C.nz + 2) <= kWarpCoarseMax) {
-            // small coarsest level: shared memory, one warp, no block barriers per iteration
-            __shared__ double cs[5][kWarpCoarseMax];
+        const int chip = chip_threads(C.nx, C.ny, C.nz);
+        if (chip > 0 && (D.coarse_solver != 0 || chip <= (int)blockDim.x)) {
+            // small coarsest level: in shared memory; levels of at most 64 cells take the FMA
+            // form of the RBGS solver (the FP32 cycle is not bound to the reference's bits)
+            __shared__ double cs[5][kChipCoarseMax];
             const int total = (int)(C.sz * (C.nz + 2));
             for (int q = threadIdx.x; q < total; q += blockDim.x) cs[1][q] = 0.0;
             __syncthreads();
@@ -556,14 +558,19 @@ __device__ void tail32_run(const TailDesc<float> &D, const LevelK<float> *Ls, co
                 cs[1][lin(i, j, k, C.sy, C.sz)] = (double)b[lin(i, j, k, L.sy, L.sz)];
             });
             __syncthreads();
-            int iters = 0;
-            if (threadIdx.x < 32)
-                iters = coarse_solve_warp_f64(C, cs[0], cs[1], cs[2], cs[3], cs[4], D.coarse_solver, D.coarse_maxit,
-                                              D.tol, D.omega64, D.omw64, D.abort);
+            int iters = 0, xs64 = 0;
+            if (D.coarse_solver != 0) {
+                if (threadIdx.x < 32)
+                    iters = coarse_cg_warp_f64(C, cs[0], cs[1], cs[2], cs[3], cs[4], D.coarse_maxit, D.tol, D.abort);
+            } else if (C.nx * C.ny * C.nz <= 64) {
+                iters = coarse_rbgs_chip<false>(C, cs, D.coarse_maxit, D.tol, D.omega64, D.omw64, D.abort, &xs64);
+            } else {
+                iters = coarse_rbgs_chip<true>(C, cs, D.coarse_maxit, D.tol, D.omega64, D.omw64, D.abort, &xs64);
+            }
             if (threadIdx.x == 0 && D.iters_out) *D.iters_out = iters;
             __syncthreads();
             for_cells(L.nx, L.ny, L.nz, [&](int i, int j, int k) {
-                x[lin(i, j, k, L.sy, L.sz)] = (float)cs[0][lin(i, j, k, C.sy, C.sz)];
+                x[lin(i, j, k, L.sy, L.sz)] = (float)cs[xs64][lin(i, j, k, C.sy, C.sz)];
             });
         } else {
             for_cells(L.nx, L.ny, L.nz, [&](int i, int j, int k) {

@@ -16,7 +16,7 @@ namespace pmg {
 namespace {
 
 constexpr int kBX = 32, kBY = 8;          // 256-thread CTAs for the grid kernels
-constexpr int kTailThreads = 1024;        // single-CTA persistent tail
+constexpr int kTailThreads = kTail64Threads;   // single-CTA persistent tail
 constexpr int kMaxGridZ = 65535;
 
 __device__ __forceinline__ int tid_in_block()
@@ -353,8 +353,25 @@ __global__ void __launch_bounds__(kTailThreads) k_tail_f64(const TailDesc<double
     }
     // coarsest level, src/multigrid.f90:1819-1851
     {
-        const int iters = coarse_solve_f64(D.C64, D.cx64, D.cb64, D.cp64, D.cap64, D.crr64, D.coarse_solver,
-                                           D.coarse_maxit, D.tol, D.omega64, D.omw64, sw, D.abort);
+        const LevelK<double> &C = D.C64;
+        const int chip = chip_threads(C.nx, C.ny, C.nz);
+        int iters;
+        if (D.coarse_solver == 0 && chip > 0 && chip <= (int)blockDim.x) {
+            __shared__ double cs[5][kChipCoarseMax];
+            const int total = (int)(C.sz * (C.nz + 2));
+            const long long csy = C.sy, csz = C.sz;
+            for (int q = threadIdx.x; q < total; q += blockDim.x) {
+                const int i = q % (int)csy, j = (q / (int)csy) % (C.ny + 2), k = q / (int)csz;
+                const bool in = i >= 1 && i <= C.nx && j >= 1 && j <= C.ny && k >= 1 && k <= C.nz;
+                cs[1][q] = in ? D.cb64[q] : 0.0;
+            }
+            int xs;
+            iters = coarse_rbgs_chip<true>(C, cs, D.coarse_maxit, D.tol, D.omega64, D.omw64, D.abort, &xs);
+            for (int q = threadIdx.x; q < total; q += blockDim.x) D.cx64[q] = cs[xs][q];
+        } else {
+            iters = coarse_solve_f64(C, D.cx64, D.cb64, D.cp64, D.cap64, D.crr64, D.coarse_solver, D.coarse_maxit,
+                                     D.tol, D.omega64, D.omw64, sw, D.abort);
+        }
         if (threadIdx.x == 0 && D.iters_out) *D.iters_out = iters;
         __syncthreads();
     }

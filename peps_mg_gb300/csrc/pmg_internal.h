@@ -23,6 +23,10 @@ struct Launch {
     bool collapse[3];   // one CTA spans the whole axis
 };
 
+// Largest block of the FP64 tail: 16 warps keep the SM's FP64 unit busy (it takes one warp
+// instruction per 19 clocks), and 512 threads leave the on-chip coarsest solver its registers.
+constexpr int kTail64Threads = 512;
+
 // Single-CTA persistent coarse tail (levels l0..nl): the CGA mapping, and the
 // coarsest-level solve of every method.
 template <typename T>

@@ -670,7 +670,7 @@ int Ctx::build_mixed()
     // The FP32 cycle hands every level of at most kTail32Cells cells (and the levels the
     // aggregation method already assigns to the tail) to the single-CTA tail kernel: such
     // levels are latency bound on the grid kernels (a few microseconds of work behind
-    // each launch and each plane step), and one 1024-thread CTA runs them back to back.
+    // each launch and each plane step), and one CTA runs them back to back.
     tail32_l0 = tail_l0;
     if (deep_tail)
         while (tail32_l0 > 1 && (long long)lv[tail32_l0 - 1].n[0] * lv[tail32_l0 - 1].n[1] * lv[tail32_l0 - 1].n[2] <=
@@ -680,6 +680,7 @@ int Ctx::build_mixed()
         long long cells = 1;
         for (int l = tail32_l0; l <= nl; ++l) cells = std::max(cells, (long long)lv[l].n[0] * lv[l].n[1] * lv[l].n[2]);
         tail32_threads = (int)std::min<long long>(kTail32Threads, std::max<long long>(64, ((cells / 2 + 31) / 32) * 32));
+        tail32_threads = std::max(tail32_threads, chip_threads(lv[nl].n[0], lv[nl].n[1], lv[nl].n[2]));
     }
     MixedState *m = new (std::nothrow) MixedState();
     if (!m) return PMG_ENOMEM;

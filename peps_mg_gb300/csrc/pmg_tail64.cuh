@@ -209,15 +209,6 @@ __device__ int coarse_solve_f64(const LevelK<double> &L, double *x, const double
     return iters;
 }
 
-// Coarsest-level solve by ONE warp on a level held in shared memory (at most
-// kWarpCoarseMax stored values, ghosts included), for the FP32 cycle of the mixed solver:
-// the iterations of coarse_solve_f64 (RBGS or CG, the same exit tests; levels of at most
-// 64 cells take a register fast path with reordered arithmetic), the sums in a 32-lane
-// butterfly order (every lane obtains the same bits, so the exit decision is uniform),
-// and __syncwarp instead of block barriers.  x, b, p, ap, rr are shared
-// arrays of the level's layout; only the calling warp touches them.
-constexpr int kWarpCoarseMax = 1000;
-
 __device__ __forceinline__ double warp_sum_f64(double v)
 {
 #pragma unroll
@@ -225,9 +216,222 @@ __device__ __forceinline__ double warp_sum_f64(double v)
     return v;
 }
 
-__device__ int coarse_solve_warp_f64(const LevelK<double> &L, double *x, const double *b, double *p, double *ap,
-                                     double *rr, int solver, int maxit, double tol, double omega, double omw,
-                                     const volatile int *abort = nullptr)
+// ---------------------------------------------------------------------------------------
+// RBGS coarsest-level solve on chip (rbgs_solver_poisson_matrix, src/rbgs_poisson_matrix.f90
+// :69-171, from x = 0): the sweeps and the convergence test run side by side.
+//
+// One FP64 warp instruction occupies this part's FP64 unit for 19 clocks and takes 64 to
+// complete, however many lanes are active and whether or not the next one depends on it
+// (measured with clock64), so an iteration's length is its chain of FP64 instructions and
+// the work has to be spread over several warps: one cell per thread.
+//  * Threads [0, P) sweep: thread s updates the s-th cell of each colour (coefficients, c0,
+//    its reciprocal and b in registers), out of place into the other of two buffers.
+//  * Threads [P, P + R) form the residual norm of the iterate before, during the sweep: the
+//    residuals and their squares beside the first colour, the sum and the exit test beside
+//    the second.  An iterate that passes is the one returned; the sweep under way is dropped.
+//  * Two barriers per iteration (P + R threads); other threads of the block wait at the end.
+// The sum's order is fixed by the level alone (R depends on nothing else).  The test
+// sqrt(rn / r0) <= tol is decided by integer comparison with tol^2 r0 unless rn lies within
+// 2^-40 of it, where it is evaluated as written.
+//
+// REF: the reference's operation order, bit for bit (the division by quot_f64's rule).
+// Otherwise (the FP32 cycle's coarsest level of at most 64 cells): the neighbour sum as a
+// tree of FMAs and x = (omega/c0)(b - t) + (1-omega) x, for the shorter chain.
+//
+// Measured (2.07 GHz, whole V-cycle solves): coarsest level 7 x 5 x 3, 36 iterations, the
+// 224 x 160 x 96 mixed solve 5.29 -> 3.00 ms; 8 x 6 x 4, about 52 iterations, the 256 x 192 x
+// 128 mixed solve from host arrays 14.9 -> 8.2 ms; 4^3, 34 iterations, the 64^3 FP64 solve
+// 6.96 -> 5.58 ms (before: one warp, or a 64-thread block with both phases in turn and an
+// IEEE division per update).
+// ---------------------------------------------------------------------------------------
+__device__ __forceinline__ void bar_named(int id, int threads)
+{
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
+// cs: five shared arrays of the level's (nx+2)(ny+2)(nz+2) layout; cs[1] holds b (ghosts
+// zero), the others are scratch.  All threads of the block call it (at least chip_threads of
+// them).  Returns the iteration counter; *xsel = the array that holds the solution.
+template <bool REF>
+__device__ int coarse_rbgs_chip(const LevelK<double> &L, double (*cs)[kChipCoarseMax], int maxit, double tol,
+                                double omega, double omw, const volatile int *abort, int *xsel)
+{
+    __shared__ double s_part[16];
+    __shared__ int s_flag, s_iters, s_x;
+    const int nx = L.nx, ny = L.ny, nz = L.nz, n = nx * ny * nz;
+    const int sy = L.sy, sz = (int)L.sz;
+    const int total = sz * (nz + 2);
+    const int tid = threadIdx.x;
+    for (int q = tid; q < total; q += blockDim.x) cs[0][q] = cs[2][q] = 0.0;
+    if (tid == 0) {
+        s_flag = 0;
+        s_iters = 0;
+        s_x = 0;
+    }
+    for (int q = tid; q < n; q += blockDim.x) {
+        const int i = q % nx + 1, r2 = q / nx, j = r2 % ny + 1, k = r2 / ny + 1;
+        const double c0 = diag_f64(L, i, j, k);
+        cs[3][i + sy * j + sz * k] = c0;
+        cs[4][i + sy * j + sz * k] = REF ? recip_f64(c0) : __ddiv_rn(omega, c0);
+    }
+    __syncthreads();
+    if (n == 1) {
+        const int c = 1 + sy + sz;
+        if (tid == 0) cs[0][c] = __ddiv_rn(cs[1][c], cs[3][c]);
+        __syncthreads();
+        *xsel = 0;
+        return 0;
+    }
+    const ChipRoles ro = chip_roles(nx, ny, nz);
+    const int nthr = ro.P + ro.R;
+    if (tid < ro.P) {
+        // ---- sweeps ----
+        const int hx = (nx + 1) / 2;
+        const int t = tid % hx, r2 = tid / hx, j = r2 % ny + 1, k = r2 / ny + 1;
+        const bool slot = tid < hx * ny * nz;
+        int p[2];
+        bool has[2];
+        double cxm[2], cxp[2], c0[2], y[2], b[2];
+        const double cym = slot ? L.cym[j] : 0.0, cyp = slot ? L.cyp[j] : 0.0;
+        const double czm = slot ? L.czm[k] : 0.0, czp = slot ? L.czp[k] : 0.0;
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {      // first colour: i + j + k odd (src/rbgs_poisson_matrix.f90:242)
+            const int i = 2 * t + 1 + ((j + k + c) & 1);
+            has[c] = slot && i <= nx;
+            p[c] = has[c] ? i + sy * j + sz * k : 1 + sy + sz;
+            cxm[c] = has[c] ? L.cxm[i] : 0.0;
+            cxp[c] = has[c] ? L.cxp[i] : 0.0;
+            c0[c] = cs[3][p[c]];
+            y[c] = cs[4][p[c]];
+            b[c] = cs[1][p[c]];
+        }
+        const bool omega1 = omega == 1.0;
+        auto update = [&](int c, const double *nb, const double *own, double *out) {
+            const int q = p[c];
+            double v;
+            if (REF) {
+                double s = __dmul_rn(cxm[c], nb[q - 1]);
+                s = __dadd_rn(s, __dmul_rn(cxp[c], nb[q + 1]));
+                s = __dadd_rn(s, __dmul_rn(cym, nb[q - sy]));
+                s = __dadd_rn(s, __dmul_rn(cyp, nb[q + sy]));
+                s = __dadd_rn(s, __dmul_rn(czm, nb[q - sz]));
+                s = __dadd_rn(s, __dmul_rn(czp, nb[q + sz]));
+                const double d = __dsub_rn(b[c], s);
+                if (omega1)
+                    v = add_zero_times_f64(quot_f64(d, c0[c], y[c]), own[q]);
+                else
+                    v = __dadd_rn(quot_f64(__dmul_rn(omega, d), c0[c], y[c]), __dmul_rn(omw, own[q]));
+            } else {
+                const double tx = fma(cxp[c], nb[q + 1], __dmul_rn(cxm[c], nb[q - 1]));
+                const double ty = fma(cyp, nb[q + sy], __dmul_rn(cym, nb[q - sy]));
+                const double tz = fma(czp, nb[q + sz], __dmul_rn(czm, nb[q - sz]));
+                const double s = __dadd_rn(__dadd_rn(tx, ty), tz);
+                v = fma(y[c], __dsub_rn(b[c], s), __dmul_rn(omw, own[q]));
+            }
+            if (has[c]) out[q] = v;
+        };
+        bar_named(1, nthr);                // |r0| is formed beside nothing
+        int cur = 0;
+        for (int it = 0; it <= maxit; ++it) {
+            const double *x = cs[cur ? 2 : 0];
+            double *xn = cs[cur ? 0 : 2];
+            if (it < maxit) update(0, x, x, xn);
+            bar_named(1, nthr);
+            if (it < maxit) update(1, xn, x, xn);
+            bar_named(1, nthr);
+            if (s_flag) break;
+            cur ^= 1;
+        }
+    } else if (tid < nthr) {
+        // ---- norms ----
+        const int rt = tid - ro.P, lane = tid & 31, warp = rt >> 5, nw = ro.R >> 5;
+        auto squares = [&](const double *x) {
+            double acc = 0.0;
+            for (int u = 0; u < ro.NN; ++u) {
+                const int q = rt + u * ro.R;
+                if (q >= n) break;
+                const int i = q % nx + 1, r2 = q / nx, j = r2 % ny + 1, k = r2 / ny + 1;
+                const int c = i + sy * j + sz * k;
+                double r;
+                if (REF) {
+                    r = __dmul_rn(cs[3][c], x[c]);
+                    r = __dadd_rn(r, __dmul_rn(L.cxm[i], x[c - 1]));
+                    r = __dadd_rn(r, __dmul_rn(L.cxp[i], x[c + 1]));
+                    r = __dadd_rn(r, __dmul_rn(L.cym[j], x[c - sy]));
+                    r = __dadd_rn(r, __dmul_rn(L.cyp[j], x[c + sy]));
+                    r = __dadd_rn(r, __dmul_rn(L.czm[k], x[c - sz]));
+                    r = __dadd_rn(r, __dmul_rn(L.czp[k], x[c + sz]));
+                    r = __dsub_rn(cs[1][c], r);
+                    acc = __dadd_rn(acc, __dmul_rn(r, r));
+                } else {
+                    const double tx = fma(L.cxp[i], x[c + 1], __dmul_rn(L.cxm[i], x[c - 1]));
+                    const double ty = fma(L.cyp[j], x[c + sy], __dmul_rn(L.cym[j], x[c - sy]));
+                    const double tz = fma(L.czp[k], x[c + sz], __dmul_rn(L.czm[k], x[c - sz]));
+                    r = __dsub_rn(cs[1][c], fma(cs[3][c], x[c], __dadd_rn(__dadd_rn(tx, ty), tz)));
+                    acc = fma(r, r, acc);
+                }
+            }
+            return acc;
+        };
+        // the sum of the threads' values, on lane 0 of the first norm warp
+        auto sum = [&](double acc) {
+            acc = warp_sum_f64(acc);
+            if (nw > 1) {
+                if (lane == 0) s_part[warp] = acc;
+                bar_named(2, ro.R);
+                if (warp == 0) {
+                    acc = lane < nw ? s_part[lane] : 0.0;
+                    for (int o = 8; o > 0; o >>= 1)
+                        if (nw > o) acc = __dadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, o));
+                }
+            }
+            return acc;
+        };
+        const double r0 = sum(squares(cs[0]));
+        // rn <= lo passes, rn > hi does not, between them the test is evaluated; positive
+        // doubles compare as integers, NaN above every hi
+        const double thr = __dmul_rn(__dmul_rn(tol, tol), r0);
+        const bool plain = thr >= 1e-250 && thr <= 1e250;
+        const long long lo = plain ? __double_as_longlong(__dmul_rn(thr, 1.0 - 0x1p-40)) : -1;
+        const long long hi = plain ? __double_as_longlong(__dmul_rn(thr, 1.0 + 0x1p-40)) : 0x7fffffffffffffffLL;
+        bar_named(1, nthr);
+        int cur = 0;
+        for (int it = 0; it <= maxit; ++it) {
+            double acc = 0.0;
+            if (it > 0) acc = squares(cs[cur ? 2 : 0]);
+            bar_named(1, nthr);
+            if (it > 0) {
+                const double rn = sum(acc);
+                if (rt == 0) {
+                    const long long v = __double_as_longlong(rn);
+                    const bool pass = v <= lo || (v <= hi && sqrt(__ddiv_rn(rn, r0)) <= tol);
+                    // the flag is polled every 16 iterations
+                    const bool stop = !pass && (it & 15) == 0 && abort && *abort;
+                    if (pass || stop || it == maxit) {
+                        s_iters = pass || stop ? it - 1 : maxit;
+                        s_x = cur ? 2 : 0;
+                        s_flag = 1;
+                    }
+                }
+            }
+            bar_named(1, nthr);
+            if (s_flag) break;
+            cur ^= 1;
+        }
+    }
+    __syncthreads();
+    *xsel = s_x;
+    return s_iters;
+}
+
+// CG coarsest-level solve by ONE warp on a level held in shared memory (at most
+// kChipCoarseMax stored values, ghosts included), for the FP32 cycle of the mixed solver:
+// the iterations of coarse_solve_f64 and its exit test, the sums in a 32-lane butterfly
+// order (every lane obtains the same bits, so the exit decision is uniform), and __syncwarp
+// instead of block barriers.  x, b, p, ap, rr are shared arrays of the level's layout; only
+// the calling warp touches them.
+__device__ int coarse_cg_warp_f64(const LevelK<double> &L, double *x, const double *b, double *p, double *ap,
+                                  double *rr, int maxit, double tol, const volatile int *abort = nullptr)
 {
     const int lane = threadIdx.x & 31;
     const int nx = L.nx, ny = L.ny, n = L.nx * L.ny * L.nz;
@@ -285,121 +489,38 @@ __device__ int coarse_solve_warp_f64(const LevelK<double> &L, double *x, const d
         __syncwarp();
     };
     int it = 0;
-    if (solver == 0 && n <= 64) {
-        // at most two cells per lane: their offsets, coefficients, omega/c0 and b stay in
-        // registers.  Each dependent FP64 operation costs on the order of a hundred
-        // cycles here, so the arithmetic is arranged for short chains: the neighbour sum
-        // as a tree of FMAs, the update x = (omega/c0)(b - t) + (1-omega) x, and the exit
-        // test sqrt(|r|^2/|r0|^2) <= tol as |r|^2 <= tol^2 |r0|^2 (no division or square
-        // root per iteration).  The same RBGS iteration as the reference's solver; the
-        // FP32 cycle that calls it is not bound to the reference's bits.
-        long long cidx[2];
-        double cw[2][6], c0v[2], wv[2], bv[2];
-        bool has[2], odd[2];
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            const int q = lane + 32 * u;
-            has[u] = q < n;
-            const int qq = has[u] ? q : 0;
-            const int i = qq % nx + 1, r2 = qq / nx, j = r2 % ny + 1, k = r2 / ny + 1;
-            cidx[u] = lin(i, j, k, L.sy, L.sz);
-            odd[u] = ((i + j + k) & 1) != 0;
-            cw[u][0] = L.cxm[i];
-            cw[u][1] = L.cxp[i];
-            cw[u][2] = L.cym[j];
-            cw[u][3] = L.cyp[j];
-            cw[u][4] = L.czm[k];
-            cw[u][5] = L.czp[k];
-            c0v[u] = diag_f64(L, i, j, k);
-            wv[u] = __ddiv_rn(omega, c0v[u]);
-            bv[u] = b[cidx[u]];
+    residual(false);
+    interior(0, 0.0, p, nullptr, rr, nullptr);
+    const double r0 = dot(rr, rr);
+    // Fused passes: A p with the sum Ap.p, and the x/r update with the sum r.r.  Each
+    // lane visits its cells in the order dot() does, so the sums are dot()'s; temp1
+    // (r.r of the unchanged r) is the previous iteration's temp2.
+    double t1 = r0;
+    for (it = 0; it < maxit; ++it) {
+        double pap = 0.0;
+        for (int q = lane; q < n; q += 32) {
+            const int i = q % nx + 1, r2 = q / nx, j = r2 % ny + 1, k = r2 / ny + 1;
+            const long long c = lin(i, j, k, L.sy, L.sz);
+            const double v = ax_cell_f64(L, p, i, j, k);
+            ap[c] = v;
+            pap = __dadd_rn(pap, __dmul_rn(v, p[c]));
         }
-        const long long sy = L.sy, sz = L.sz;
-        auto nbsum = [&](int u) {
-            const long long c = cidx[u];
-            const double tx = fma(cw[u][1], x[c + 1], __dmul_rn(cw[u][0], x[c - 1]));
-            const double ty = fma(cw[u][3], x[c + sy], __dmul_rn(cw[u][2], x[c - sy]));
-            const double tz = fma(cw[u][5], x[c + sz], __dmul_rn(cw[u][4], x[c - sz]));
-            return __dadd_rn(__dadd_rn(tx, ty), tz);
-        };
-        auto norm = [&]() {
-            double acc = 0.0;
-#pragma unroll
-            for (int u = 0; u < 2; ++u)
-                if (has[u]) {
-                    const double r = __dsub_rn(bv[u], fma(c0v[u], x[cidx[u]], nbsum(u)));
-                    acc = fma(r, r, acc);
-                }
-            return warp_sum_f64(acc);
-        };
-        const double r0 = norm();
-        const double thr = __dmul_rn(__dmul_rn(tol, tol), r0);
-        for (it = 0; it < maxit; ++it) {
-#pragma unroll
-            for (int colour = 0; colour < 2; ++colour) {
-                // first colour: (i + j + k) odd (src/rbgs_poisson_matrix.f90:242)
-#pragma unroll
-                for (int u = 0; u < 2; ++u)
-                    if (has[u] && odd[u] == (colour == 0)) {
-                        const double old = x[cidx[u]];
-                        const double t = nbsum(u);
-                        x[cidx[u]] = fma(wv[u], __dsub_rn(bv[u], t), __dmul_rn(omw, old));
-                    }
-                __syncwarp();
-            }
-            if (norm() <= thr) break;
-            if ((it & 15) == 15 && warp_abort(abort)) break;
+        const double alpha = __ddiv_rn(t1, warp_sum_f64(pap));
+        double rr2 = 0.0;
+        for (int q = lane; q < n; q += 32) {
+            const int i = q % nx + 1, r2 = q / nx, j = r2 % ny + 1, k = r2 / ny + 1;
+            const long long c = lin(i, j, k, L.sy, L.sz);
+            x[c] = __dadd_rn(x[c], __dmul_rn(alpha, p[c]));
+            const double v = __dsub_rn(rr[c], __dmul_rn(alpha, ap[c]));
+            rr[c] = v;
+            rr2 = __dadd_rn(rr2, __dmul_rn(v, v));
         }
-    } else if (solver == 0) {
-        const int hx = (nx + 1) / 2, nq = hx * ny * L.nz;
-        const double r0 = residual(true);
-        for (it = 0; it < maxit; ++it) {
-            for (int colour = 0; colour < 2; ++colour) {
-                for (int q = lane; q < nq; q += 32) {
-                    const int t = q % hx, r2 = q / hx, j = r2 % ny + 1, k = r2 / ny + 1;
-                    const int i = 2 * t + 1 + ((j + k + colour) & 1);
-                    if (i <= nx) x[lin(i, j, k, L.sy, L.sz)] = rbgs_cell_f64(L, x, b, i, j, k, omega, omw);
-                }
-                __syncwarp();
-            }
-            const double rn = residual(true);
-            if (sqrt(__ddiv_rn(rn, r0)) <= tol) break;
-            if ((it & 15) == 15 && warp_abort(abort)) break;
-        }
-    } else {
-        residual(false);
-        interior(0, 0.0, p, nullptr, rr, nullptr);
-        const double r0 = dot(rr, rr);
-        // Fused passes: A p with the sum Ap.p, and the x/r update with the sum r.r.  Each
-        // lane visits its cells in the order dot() does, so the sums are dot()'s; temp1
-        // (r.r of the unchanged r) is the previous iteration's temp2.
-        double t1 = r0;
-        for (it = 0; it < maxit; ++it) {
-            double pap = 0.0;
-            for (int q = lane; q < n; q += 32) {
-                const int i = q % nx + 1, r2 = q / nx, j = r2 % ny + 1, k = r2 / ny + 1;
-                const long long c = lin(i, j, k, L.sy, L.sz);
-                const double v = ax_cell_f64(L, p, i, j, k);
-                ap[c] = v;
-                pap = __dadd_rn(pap, __dmul_rn(v, p[c]));
-            }
-            const double alpha = __ddiv_rn(t1, warp_sum_f64(pap));
-            double rr2 = 0.0;
-            for (int q = lane; q < n; q += 32) {
-                const int i = q % nx + 1, r2 = q / nx, j = r2 % ny + 1, k = r2 / ny + 1;
-                const long long c = lin(i, j, k, L.sy, L.sz);
-                x[c] = __dadd_rn(x[c], __dmul_rn(alpha, p[c]));
-                const double v = __dsub_rn(rr[c], __dmul_rn(alpha, ap[c]));
-                rr[c] = v;
-                rr2 = __dadd_rn(rr2, __dmul_rn(v, v));
-            }
-            const double t2 = warp_sum_f64(rr2);
-            __syncwarp();
-            if (sqrt(__ddiv_rn(t2, r0)) < tol) break;
-            interior(2, __ddiv_rn(t2, t1), p, nullptr, rr, nullptr);
-            t1 = t2;
-            if ((it & 15) == 15 && warp_abort(abort)) break;
-        }
+        const double t2 = warp_sum_f64(rr2);
+        __syncwarp();
+        if (sqrt(__ddiv_rn(t2, r0)) < tol) break;
+        interior(2, __ddiv_rn(t2, t1), p, nullptr, rr, nullptr);
+        t1 = t2;
+        if ((it & 15) == 15 && warp_abort(abort)) break;
     }
     return it;
 }

@@ -1,0 +1,83 @@
+"""The FP64 path's division by the diagonal (quot_f64 in pmg_common.cuh: a product with the
+rounded reciprocal and two FMAs) against the correctly rounded quotient, in exact rational
+arithmetic: random operands, and operands whose quotient lies as close to a rounding boundary
+as a quotient can, including divisors whose reciprocal does (which the kernel's table rejects).
+"""
+from fractions import Fraction
+
+import numpy as np
+import pytest
+
+
+def rn(v):
+    """Round a rational to the nearest double (normal range), ties to even."""
+    if v == 0:
+        return Fraction(0)
+    a = abs(v)
+    e = a.numerator.bit_length() - a.denominator.bit_length()
+    if Fraction(2) ** e > a:
+        e -= 1
+    unit = Fraction(2) ** (e - 52)
+    n, rest = divmod(a, unit)
+    if rest * 2 > unit or (rest * 2 == unit and n % 2):
+        n += 1
+    return n * unit * (1 if v > 0 else -1)
+
+
+def recip(c):
+    """recip_f64 on a mantissa c in [1, 2): y, or None where the table holds a NaN."""
+    y = rn(1 / c)
+    off = abs(1 - c * y)
+    assert rn(off) == off            # one FMA forms it exactly
+    return y if off <= rn(c * Fraction(1, 2 ** 54) * (1 - Fraction(1, 2 ** 40))) else None
+
+
+def quot(d, c, y):
+    q0 = rn(d * y)
+    r = rn(d - c * q0)
+    return rn(q0 + r * y)
+
+
+def near_boundary(rng, count):
+    """(d, c) with mantissas in [1, 2) and d / c within a few units of 2^-106 / c of a
+    midpoint between doubles: M C + N = D 2^s for odd C, small N and M the midpoint."""
+    out = []
+    while len(out) < count:
+        C = int(rng.integers(2 ** 52, 2 ** 53)) | 1
+        N = int(rng.integers(1, 12)) * int(rng.choice([-1, 1]))
+        s = int(rng.choice([53, 54]))
+        M = (-N * pow(C, -1, 2 ** s)) % 2 ** s
+        if not M & 1:
+            continue
+        D, rest = divmod(M * C + N, 2 ** s)
+        if rest == 0 and 2 ** 52 <= D < 2 ** 53:
+            out.append((Fraction(D, 2 ** 52), Fraction(C, 2 ** 52)))
+    return out
+
+
+@pytest.mark.parametrize("kind", ["random", "boundary", "extreme"])
+def test_quotient_is_correctly_rounded(kind):
+    rng = np.random.Generator(np.random.PCG64(11))
+    one = 2 ** 52
+    if kind == "random":
+        pairs = [(Fraction(int(a), one), Fraction(int(b), one)) for a, b in rng.integers(one, 2 * one, size=(2000, 2))]
+    elif kind == "boundary":
+        pairs = near_boundary(rng, 2000)
+    else:
+        ends = [one + k for k in range(12)] + [2 * one - 1 - k for k in range(12)]
+        ends += [3 * one // 2 + k for k in range(-3, 4)]
+        pairs = [(Fraction(a, one), Fraction(b, one)) for a in ends for b in ends]
+    used = 0
+    for d, c in pairs:
+        y = recip(c)
+        if y is None:
+            continue
+        used += 1
+        assert quot(d, c, y) == rn(d / c), (d, c)
+    if kind != "extreme":                # a few of whose divisors lie just below a power of two
+        assert used == len(pairs)
+
+
+def test_reciprocal_table_rejects_the_exceptional_divisor():
+    """The divisor with all mantissa bits set: its reciprocal lies next to a midpoint."""
+    assert recip(Fraction(2 ** 53 - 1, 2 ** 52)) is None
