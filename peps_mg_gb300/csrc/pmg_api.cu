@@ -437,6 +437,15 @@ bool host_setup()
 // host-side uses (level queries, the FP32 tables of the mixed path).  The layout: per level
 // and axis cm, cp (and sx for x), then per transfer and axis w, pp, pn, each table padded to
 // an even length (16-byte alignment).
+// Every v[0..n) positive, finite and within 2^+-e: what the integer-pipe products of the FP64
+// kernels (pmg_mul64.cuh) ask of a level's tables.
+static bool exponents_within(const double *v, int n, int e)
+{
+    for (int i = 0; i < n; ++i)
+        if (!(v[i] > 0.0) || !std::isfinite(v[i]) || std::abs(std::ilogb(v[i])) > e) return false;
+    return true;
+}
+
 int Ctx::setup_tables()
 {
     const bool meshes_given = preset_levels || host_setup();
@@ -472,6 +481,8 @@ int Ctx::setup_tables()
                 H.w[l][d] = tab(lv[l].n[d]);
                 H.pp[l][d] = tab(lv[l].n[d]);
                 H.pn[l][d] = tab(lv[l].n[d]);
+                H.ps[l][d] = tab(lv[l].n[d]);
+                H.pr[l][d] = tab(lv[l].n[d]);
             }
     }
     std::vector<double> hm((size_t)mo, 0.0);
@@ -530,6 +541,10 @@ int Ctx::setup_tables()
         k.cxm = d_tables + H.cm[l][0]; k.cxp = d_tables + H.cp[l][0]; k.sx = d_tables + H.sx[l];
         k.cym = d_tables + H.cm[l][1]; k.cyp = d_tables + H.cp[l][1];
         k.czm = d_tables + H.cm[l][2]; k.czp = d_tables + H.cp[l][2];
+        k.mul64 = 1;
+        for (int d = 0; d < 3; ++d)
+            for (long long o : {H.cm[l][d], H.cp[l][d]})
+                if (!exponents_within(tables_host.data() + o + 1, L.n[d], 390)) k.mul64 = 0;
         if (l < nl) {
             const Level &C = lv[l + 1];
             XferK<double> &x = X[l];
@@ -543,6 +558,12 @@ int Ctx::setup_tables()
             x.pxp = d_tables + H.pp[l][0]; x.pxn = d_tables + H.pn[l][0];
             x.pyp = d_tables + H.pp[l][1]; x.pyn = d_tables + H.pn[l][1];
             x.pzp = d_tables + H.pp[l][2]; x.pzn = d_tables + H.pn[l][2];
+            x.sx = d_tables + H.ps[l][0]; x.sy = d_tables + H.ps[l][1]; x.szz = d_tables + H.ps[l][2];
+            x.rx = d_tables + H.pr[l][0]; x.ry = d_tables + H.pr[l][1]; x.rz = d_tables + H.pr[l][2];
+            x.mul64 = 1;
+            for (int d = 0; d < 3; ++d)
+                for (long long o : {H.w[l][d], H.pp[l][d], H.pn[l][d], H.ps[l][d]})
+                    if (!exponents_within(tables_host.data() + o + 1, L.n[d], 120)) x.mul64 = 0;
         }
     }
     if (host_setup()) {
@@ -565,6 +586,11 @@ int Ctx::setup_tables()
                     std::copy(w.begin(), w.end(), hb.begin() + H.w[l][d]);
                     std::copy(dp.begin(), dp.end(), hb.begin() + H.pp[l][d]);
                     std::copy(dn.begin(), dn.end(), hb.begin() + H.pn[l][d]);
+                    for (int f = 1; f <= lv[l].n[d]; ++f) {
+                        const double ps = s1 ? dn[f] + dn[f] : (f & 1) ? dp[f] + dp[f + 1] : dn[f] + dn[f - 1];
+                        hb[H.ps[l][d] + f] = ps;
+                        hb[H.pr[l][d] + f] = 1.0 / ps;
+                    }
                 }
         }
         if (std::memcmp(hb.data(), tables_host.data(), hb.size() * sizeof(double)) != 0) {
@@ -750,12 +776,13 @@ int Ctx::build(const pmg_config_t *c, cudaStream_t s)
     }
     if (precision == PMG_FP64_FAST) PMG_TRY(setup_fast64());
     if (precision == PMG_FP64) {
-        // per-cell diagonal tables of the plain FP64 path (the grid kernels read c0 instead
-        // of summing five 1-D table entries per cell; the values are diag_f64's bits)
+        // per-cell diagonal tables of the plain FP64 path and of its reciprocal (the grid
+        // kernels read c0 instead of summing five 1-D table entries per cell, the values are
+        // diag_f64's bits, and divide by it with two FMAs)
         c0t.assign((size_t)nl + 1, nullptr);
         for (int l = 0; l <= nl; ++l) {
-            PMG_CUDA(dev_malloc(&c0t[l], lv[l].total * sizeof(double)), "diagonal table");
-            PMG_CUDA(cudaMemsetAsync(c0t[l], 0, lv[l].total * sizeof(double), stream), "diagonal table");
+            PMG_CUDA(dev_malloc(&c0t[l], 2 * lv[l].total * sizeof(double)), "diagonal table");
+            PMG_CUDA(cudaMemsetAsync(c0t[l], 0, 2 * lv[l].total * sizeof(double), stream), "diagonal table");
             PMG_TRY(f64_diag_table(K[l], c0t[l], stream));
         }
         // complete before any other stream (a decomposed solve's) reads the tables

@@ -25,6 +25,7 @@ struct LevelK {
     int sy;
     long long sz;
     const T *cxm, *cxp, *sx, *cym, *cyp, *czm, *czp;
+    int mul64;     // FP64: every coefficient's exponent lies within 2^+-390 (pmg_mul64.cuh)
 };
 
 // Transfer between fine level l and coarse level l+1 (restriction and prolongation).
@@ -41,6 +42,10 @@ struct XferK {
     int stx, sty, stz;
     const T *wx, *wy, *wz;
     const T *pxp, *pxn, *pyp, *pyn, *pzp, *pzn;
+    // FP64 only: per axis and fine index, the sum of the two prolongation weights and its
+    // reciprocal; mul64: every weight's exponent lies within 2^+-120 (pmg_mul64.cuh)
+    const T *sx, *sy, *szz, *rx, *ry, *rz;
+    int mul64;
 };
 
 __host__ __device__ inline long long lin(int i, int j, int k, int sy, long long sz)
@@ -103,8 +108,8 @@ __device__ __forceinline__ double diag_f64(const LevelK<double> &L, int i, int j
 //    (1 - c y = m delta, formed exactly by one FMA).  Otherwise q0 is a neighbour of the
 //    boundary, r is exact, and the perturbation |r delta| < m 2^-108 stays below the
 //    smallest distance 2^-106 / m of a quotient (of unit 2^-53) from a boundary, m < 2;
-//  * over- and underflow: c's exponent lies within 2^+-400 and d's within 2^+-500 (or d is
-//    zero, where the signs come out right for the operator's negative c).
+//  * over- and underflow: c's exponent lies within 2^+-400 and d's within 2^+-500, or d is
+//    zero (a zero with the quotient's sign).
 // Anything else takes the IEEE division.
 __device__ __forceinline__ double recip_f64(double c)
 {
@@ -113,19 +118,21 @@ __device__ __forceinline__ double recip_f64(double c)
     const unsigned e = ((unsigned)hi >> 20) & 0x7ffu;
     const double m54 = __hiloint2double((hi & 0xfffff) | (969 << 20), __double2loint(c));   // m 2^-54
     const double off = fabs(__fma_rn(-c, y, 1.0));
-    const bool ok = hi < 0 && e - 623u <= 800u && off <= __dmul_rn(m54, 1.0 - 0x1p-40);
+    const bool ok = e - 623u <= 800u && off <= __dmul_rn(m54, 1.0 - 0x1p-40);
     return ok ? y : __longlong_as_double(0x7ff8000000000000LL);
 }
 
-// d / c, c negative, y = recip_f64(c)
+// d / c, y = recip_f64(c)
 __device__ __forceinline__ double quot_f64(double d, double c, double y)
 {
     const double q0 = __dmul_rn(d, y);
     const double r = __fma_rn(-c, q0, d);
     double q = __fma_rn(r, y, q0);
     const unsigned dh = (unsigned)__double2hiint(d), dl = (unsigned)__double2loint(d);
-    const bool ok = (((dh >> 20) & 0x7ffu) - 523u <= 1000u || ((dh << 1) | dl) == 0u) &&
-                    (((unsigned)__double2hiint(q) >> 20) & 0x7ffu) != 0x7ffu;
+    const bool zero = ((dh << 1) | dl) == 0u;
+    if (zero) q = __hiloint2double((int)((dh ^ (unsigned)__double2hiint(c)) & 0x80000000u), 0);
+    const bool ok = (((dh >> 20) & 0x7ffu) - 523u <= 1000u || zero) &&
+                    (((unsigned)__double2hiint(y) >> 20) & 0x7ffu) != 0x7ffu;
     if (!ok) q = __ddiv_rn(d, c);
     return q;
 }

@@ -7,8 +7,11 @@
 // column (the CGPSA per-axis step-down), without changing any cell's arithmetic.
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "../../include/peps_mg.h"
 #include "pmg_internal.h"
+#include "pmg_mul64.cuh"
 #include "pmg_tail64.cuh"
 
 namespace pmg {
@@ -29,60 +32,133 @@ __device__ __forceinline__ int block_lin()
     return blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
 }
 
-// The diagonal c0 of cell p: read from the level's per-cell table (TAB; the values
-// k_diag_f64 stored, diag_f64's bits) or formed from the 1-D tables.  The table takes four
-// of the 28 FP64 instructions of an RBGS update off a pipe that bounds these kernels.
-template <bool TAB>
+// How a grid kernel forms its arithmetic:
+//  kPlain  the diagonal summed from the 1-D tables, products on the FP64 unit (contexts
+//          without the per-cell tables: the level operations of mixed and FP64-fast ones);
+//  kTab    the diagonal read from the level's per-cell table;
+//  kInt    that, products on the integer pipe (pmg_mul64.cuh) and the division by the table's
+//          reciprocal: levels whose coefficients fit mul64's range, which all but meshes with
+//          spacings beyond 2^+-190 do.
+// The bits are the same.  These kernels are bound by the FP64 unit (19 clocks per warp
+// instruction and SM), so kInt takes the products off it: an RBGS update keeps 8 of 21 FP64
+// instructions (15 with the reciprocal alone), a residual 7 of 14, A p with its dot product 7
+// of 16.  Measured: a half-sweep at 384^3 1.15 -> 0.53 ms, a residual at 324 x 258 x 194 0.474
+// -> 0.252 ms, A p at 224 x 160 x 128 159 -> 103 us; the FP64 unit is 80% busy in the sweep.
+enum ArithMode { kPlain = 0, kTab = 1, kInt = 2 };
+
+template <int MODE>
 __device__ __forceinline__ double diag_at(const LevelK<double> &L, const double *c0t, long long p, int i, int j,
                                           int k)
 {
-    return TAB ? c0t[p] : diag_f64(L, i, j, k);
+    return MODE != kPlain ? c0t[p] : diag_f64(L, i, j, k);
+}
+
+template <int MODE>
+__device__ __forceinline__ double prod(double c, double x)
+{
+    return MODE == kInt ? mul64(mul64_factor(c), x) : __dmul_rn(c, x);
+}
+
+// A term of a dot product: one FMA (the sums' order is this file's own, so their bits are too).
+__device__ __forceinline__ double add_prod(double acc, double a, double b) { return __fma_rn(a, b, acc); }
+
+// ax_cell_c0_f64 (pmg_common.cuh) with the products of MODE
+template <int MODE>
+__device__ __forceinline__ double ax_cell(const LevelK<double> &L, const double *x, const double *c0t, long long p,
+                                          int i, int j, int k)
+{
+    double t = prod<MODE>(diag_at<MODE>(L, c0t, p, i, j, k), x[p]);
+    t = __dadd_rn(t, prod<MODE>(L.cxm[i], x[p - 1]));
+    t = __dadd_rn(t, prod<MODE>(L.cxp[i], x[p + 1]));
+    t = __dadd_rn(t, prod<MODE>(L.cym[j], x[p - L.sy]));
+    t = __dadd_rn(t, prod<MODE>(L.cyp[j], x[p + L.sy]));
+    t = __dadd_rn(t, prod<MODE>(L.czm[k], x[p - L.sz]));
+    t = __dadd_rn(t, prod<MODE>(L.czp[k], x[p + L.sz]));
+    return t;
+}
+
+// The planes k0 .. k1 of this CTA: consecutive chunks of the nz planes.
+__device__ __forceinline__ void plane_chunk(int nz, int &k0, int &k1)
+{
+    const int kc = (nz + gridDim.z - 1) / gridDim.z;
+    k0 = 1 + kc * blockIdx.z;
+    k1 = min(nz, k0 + kc - 1);
+}
+
+// f(i, j, k, p) on the cells of this thread.
+template <typename F>
+__device__ __forceinline__ void each_cell(const LevelK<double> &L, F f)
+{
+    int k0, k1;
+    plane_chunk(L.nz, k0, k1);
+    for (int j = blockIdx.y * blockDim.y + threadIdx.y + 1; j <= L.ny; j += gridDim.y * blockDim.y)
+        for (int i = blockIdx.x * blockDim.x + threadIdx.x + 1; i <= L.nx; i += gridDim.x * blockDim.x)
+            for (int k = k0; k <= k1; ++k) f(i, j, k, lin(i, j, k, L.sy, L.sz));
 }
 
 // One colour of the red-black sweep.  colour 0 is the reference's first half-sweep:
 // ista = 1 + mod(j+k, 2) (src/rbgs_poisson_matrix.f90:242); colour 1 the second
 // (:260).  Thread t of a row updates i = 2t + ista.
-template <bool TAB, bool OMEGA1>
+template <int MODE, bool OMEGA1>
 __global__ void __launch_bounds__(kBX *kBY) k_rbgs_f64(LevelK<double> L, double *__restrict__ x,
                                                        const double *__restrict__ b, double omega, double omw,
                                                        int colour, const double *__restrict__ c0t)
 {
-    for (int k = blockIdx.z + 1; k <= L.nz; k += gridDim.z)
-        for (int j = blockIdx.y * blockDim.y + threadIdx.y + 1; j <= L.ny; j += gridDim.y * blockDim.y) {
-            const int ista = 1 + ((j + k + colour) & 1);
-            for (int i = ista + 2 * (blockIdx.x * blockDim.x + threadIdx.x); i <= L.nx;
-                 i += 2 * gridDim.x * blockDim.x) {
+    const long long total = L.sz * (L.nz + 2);
+    int k0, k1;
+    plane_chunk(L.nz, k0, k1);
+    for (int j = blockIdx.y * blockDim.y + threadIdx.y + 1; j <= L.ny; j += gridDim.y * blockDim.y)
+        for (int t = blockIdx.x * blockDim.x + threadIdx.x; 2 * t < L.nx; t += gridDim.x * blockDim.x)
+            for (int k = k0; k <= k1; ++k) {
+                const int i = 2 * t + 1 + ((j + k + colour) & 1);
+                if (i > L.nx) continue;
                 const long long p = lin(i, j, k, L.sy, L.sz);
-                x[p] = rbgs_cell_c0_f64<OMEGA1>(L, x, b, i, j, k, omega, omw, diag_at<TAB>(L, c0t, p, i, j, k));
+                if (MODE == kInt) {
+                    double s = prod<MODE>(L.cxm[i], x[p - 1]);
+                    s = __dadd_rn(s, prod<MODE>(L.cxp[i], x[p + 1]));
+                    s = __dadd_rn(s, prod<MODE>(L.cym[j], x[p - L.sy]));
+                    s = __dadd_rn(s, prod<MODE>(L.cyp[j], x[p + L.sy]));
+                    s = __dadd_rn(s, prod<MODE>(L.czm[k], x[p - L.sz]));
+                    s = __dadd_rn(s, prod<MODE>(L.czp[k], x[p + L.sz]));
+                    const double d = __dsub_rn(b[p], s);
+                    if (OMEGA1)
+                        x[p] = add_zero_times_f64(quot64(d, c0t[p], c0t[p + total]), x[p]);
+                    else
+                        x[p] = __dadd_rn(quot64(mul64_vv(omega, d), c0t[p], c0t[p + total]), mul64_vv(omw, x[p]));
+                } else {
+                    x[p] = rbgs_cell_c0_f64<OMEGA1>(L, x, b, i, j, k, omega, omw, diag_at<MODE>(L, c0t, p, i, j, k));
+                }
             }
-        }
 }
 
-// c0t = the diagonal of every interior cell (diag_f64); the ghosts are left as they are.
+// c0t = the diagonal of every interior cell (diag_f64), then as many values again its
+// reciprocals (recip_f64); the ghosts are left as they are.
 __global__ void __launch_bounds__(kBX *kBY) k_diag_f64(LevelK<double> L, double *__restrict__ c0t)
 {
+    const long long total = L.sz * (L.nz + 2);
     for (int k = blockIdx.z + 1; k <= L.nz; k += gridDim.z)
         for (int j = blockIdx.y * blockDim.y + threadIdx.y + 1; j <= L.ny; j += gridDim.y * blockDim.y)
-            for (int i = blockIdx.x * blockDim.x + threadIdx.x + 1; i <= L.nx; i += gridDim.x * blockDim.x)
-                c0t[lin(i, j, k, L.sy, L.sz)] = diag_f64(L, i, j, k);
+            for (int i = blockIdx.x * blockDim.x + threadIdx.x + 1; i <= L.nx; i += gridDim.x * blockDim.x) {
+                const long long p = lin(i, j, k, L.sy, L.sz);
+                const double c0 = diag_f64(L, i, j, k);
+                c0t[p] = c0;
+                c0t[p + total] = recip_f64(c0);
+            }
 }
 
 // r = b - A x on the interior (src/multigrid.f90:1795-1805); optional per-block sum of r^2.
-template <bool NORM, bool TAB>
+template <bool NORM, int MODE>
 __global__ void __launch_bounds__(kBX *kBY) k_residual_f64(LevelK<double> L, double *__restrict__ r,
                                                            const double *__restrict__ x,
                                                            const double *__restrict__ b, double *partials,
                                                            const double *__restrict__ c0t)
 {
     double acc = 0.0;
-    for (int k = blockIdx.z + 1; k <= L.nz; k += gridDim.z)
-        for (int j = blockIdx.y * blockDim.y + threadIdx.y + 1; j <= L.ny; j += gridDim.y * blockDim.y)
-            for (int i = blockIdx.x * blockDim.x + threadIdx.x + 1; i <= L.nx; i += gridDim.x * blockDim.x) {
-                const long long p = lin(i, j, k, L.sy, L.sz);
-                const double v = __dsub_rn(b[p], ax_cell_c0_f64(L, x, i, j, k, diag_at<TAB>(L, c0t, p, i, j, k)));
-                r[p] = v;
-                if (NORM) acc = __dadd_rn(acc, __dmul_rn(v, v));
-            }
+    each_cell(L, [&](int i, int j, int k, long long p) {
+        const double v = __dsub_rn(b[p], ax_cell<MODE>(L, x, c0t, p, i, j, k));
+        r[p] = v;
+        if (NORM) acc = add_prod(acc, v, v);
+    });
     if (NORM) {
         __shared__ double sw[kBX * kBY / 32];
         const double s = block_sum(acc, sw);
@@ -90,16 +166,11 @@ __global__ void __launch_bounds__(kBX *kBY) k_residual_f64(LevelK<double> L, dou
     }
 }
 
-template <bool TAB>
+template <int MODE>
 __global__ void __launch_bounds__(kBX *kBY) k_mvmul_f64(LevelK<double> L, double *__restrict__ y,
                                                         const double *__restrict__ x, const double *__restrict__ c0t)
 {
-    for (int k = blockIdx.z + 1; k <= L.nz; k += gridDim.z)
-        for (int j = blockIdx.y * blockDim.y + threadIdx.y + 1; j <= L.ny; j += gridDim.y * blockDim.y)
-            for (int i = blockIdx.x * blockDim.x + threadIdx.x + 1; i <= L.nx; i += gridDim.x * blockDim.x) {
-                const long long p = lin(i, j, k, L.sy, L.sz);
-                y[p] = ax_cell_c0_f64(L, x, i, j, k, diag_at<TAB>(L, c0t, p, i, j, k));
-            }
+    each_cell(L, [&](int i, int j, int k, long long p) { y[p] = ax_cell<MODE>(L, x, c0t, p, i, j, k); });
 }
 
 __global__ void __launch_bounds__(kBX *kBY) k_dot_f64(LevelK<double> L, const double *__restrict__ x,
@@ -126,15 +197,142 @@ __global__ void __launch_bounds__(1024) k_reduce_f64(const double *__restrict__ 
     if (threadIdx.x == 0) *out = s;
 }
 
+// M64: products on the integer pipe; otherwise (weights beyond mul64's range) restrict_cell_f64.
+// A thread takes the coarse cells of one column (i, j) over a chunk of planes, so the weights'
+// x-y products are formed once, and the full weights, their sum and its reciprocal only where
+// the plane's weights change: on a uniform z axis a coarse cell keeps 9 of 43 FP64
+// instructions (324 x 258 x 194, stretched: 192 -> 122 us).
+template <bool M64>
 __global__ void __launch_bounds__(kBX *kBY) k_restrict_f64(XferK<double> X, const double *__restrict__ vf,
                                                            double *__restrict__ vc)
 {
-    for (int k = blockIdx.z + 1; k <= X.ncz; k += gridDim.z)
-        for (int j = blockIdx.y * blockDim.y + threadIdx.y + 1; j <= X.ncy; j += gridDim.y * blockDim.y)
-            for (int i = blockIdx.x * blockDim.x + threadIdx.x + 1; i <= X.ncx; i += gridDim.x * blockDim.x)
-                vc[lin(i, j, k, X.csy, X.csz)] = restrict_cell_f64(X, vf, i, j, k);
+    int k0, k1;
+    plane_chunk(X.ncz, k0, k1);
+    for (int j = blockIdx.y * blockDim.y + threadIdx.y + 1; j <= X.ncy; j += gridDim.y * blockDim.y)
+        for (int i = blockIdx.x * blockDim.x + threadIdx.x + 1; i <= X.ncx; i += gridDim.x * blockDim.x) {
+            if (!M64) {
+                for (int k = k0; k <= k1; ++k) vc[lin(i, j, k, X.csy, X.csz)] = restrict_cell_f64(X, vf, i, j, k);
+                continue;
+            }
+            const int ip = i * X.stx, iz = ip - (X.stx - 1);
+            const int jp = j * X.sty, jz = jp - (X.sty - 1);
+            const double xz = X.wx[iz], xp = X.wx[ip], yz = X.wy[jz], yp = X.wy[jp];
+            const double xy[4] = {__dmul_rn(xz, yz), __dmul_rn(xp, yz), __dmul_rn(xz, yp), __dmul_rn(xp, yp)};
+            // child c of a plane: (ip|iz, jp|jz) in the reference's order (restrict_cell_f64)
+            const long long o[4] = {lin(ip, jp, 0, X.fsy, X.fsz), lin(iz, jp, 0, X.fsy, X.fsz),
+                                    lin(ip, jz, 0, X.fsy, X.fsz), lin(iz, jz, 0, X.fsy, X.fsz)};
+            double wz0 = 0.0, wz1 = 0.0, vol = 1.0, y = 1.0;
+            Mul64 w[8];
+            for (int k = k0; k <= k1; ++k) {
+                const int kp = k * X.stz, kz = kp - (X.stz - 1);
+                const double zz = X.wz[kz], zp = X.wz[kp];
+                if (k == k0 || __double_as_longlong(zz) != __double_as_longlong(wz0) ||
+                    __double_as_longlong(zp) != __double_as_longlong(wz1)) {
+                    wz0 = zz;
+                    wz1 = zp;
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) {
+                        const double v = mul64(mul64_factor(xy[c & 3]), c < 4 ? zz : zp);
+                        vol = c == 0 ? v : __dadd_rn(vol, v);
+                        w[c] = mul64_factor(v);
+                    }
+                    y = recip_f64(vol);
+                }
+                // v11* meets the plane kp's children first (src/multigrid.f90:1483-1490)
+                double s = 0.0;
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                    const double v = mul64(w[c], vf[o[c & 3] + X.fsz * (c < 4 ? kp : kz)]);
+                    s = c == 0 ? v : __dadd_rn(s, v);
+                }
+                vc[lin(i, j, k, X.csy, X.csz)] = quot64(s, vol, y);
+            }
+        }
 }
 
+// Coarse index, neighbour and the own and the neighbour's 1-D weight of fine index f along
+// one axis (stride 2: odd f is the low child, even f the high one; stride 1: the high child,
+// src/multigrid.f90:1594-1649).
+__device__ __forceinline__ void side64(int st, int f, const double *pp, const double *pn, int &c, int &nb, double &wa,
+                                       double &wb)
+{
+    if (st == 2) {
+        c = (f + 1) >> 1;
+        nb = (f & 1) ? c - 1 : c + 1;
+        wa = (f & 1) ? pp[f] : pn[f];
+        wb = (f & 1) ? pp[f + 1] : pn[f - 1];
+    } else {
+        c = nb = f;
+        wa = wb = pn[f];
+    }
+}
+
+// Prolongation on the integer pipe: a thread takes the fine cells of one column over a chunk
+// of fine planes (coalesced, where a thread per coarse cell writes every second cell).  The
+// x-y products of the weights are formed once per column; the eight weights, the denominator
+// and its reciprocal only where the plane's weights change, which on a uniform z axis is at
+// the chunk's first plane and at the boundaries.  A fine cell then keeps 10 (14 where the
+// weights change) of about 40 FP64 instructions; where they change the integer products (19)
+// bound it.  324 x 258 x 194, stretched: 1.43 -> 0.60 ms.  Terms and order: prolong_child_f64.
+template <bool ADD>
+__global__ void __launch_bounds__(kBX *kBY) k_prolong_m64(XferK<double> X, const double *__restrict__ vc,
+                                                          double *__restrict__ vf)
+{
+    const int nfx = X.ncx * X.stx, nfy = X.ncy * X.sty, nfz = X.ncz * X.stz;
+    int k0, k1;
+    plane_chunk(nfz, k0, k1);
+    for (int jf = blockIdx.y * blockDim.y + threadIdx.y + 1; jf <= nfy; jf += gridDim.y * blockDim.y)
+        for (int fi = blockIdx.x * blockDim.x + threadIdx.x + 1; fi <= nfx; fi += gridDim.x * blockDim.x) {
+            int i, in, j, jn;
+            double ax, bx, ay, by;
+            side64(X.stx, fi, X.pxp, X.pxn, i, in, ax, bx);
+            side64(X.sty, jf, X.pyp, X.pyn, j, jn, ay, by);
+            const Mul64 axy = mul64_factor(__dmul_rn(ax, ay)), bxy = mul64_factor(__dmul_rn(bx, ay));
+            const Mul64 axby = mul64_factor(__dmul_rn(ax, by)), bxby = mul64_factor(__dmul_rn(bx, by));
+            const Mul64 sxy = mul64_factor(__dmul_rn(X.sx[fi], X.sy[jf]));
+            const double rxy = __dmul_rn(X.rx[fi], X.ry[jf]);
+            const double *v0 = vc + lin(i, j, 0, X.csy, X.csz), *vx = vc + lin(in, j, 0, X.csy, X.csz);
+            const double *vy = vc + lin(i, jn, 0, X.csy, X.csz), *vxy = vc + lin(in, jn, 0, X.csy, X.csz);
+            double *out = vf + lin(fi, jf, 0, X.fsy, X.fsz);
+            double az = 0.0, bz = 0.0, den = 1.0, y = 1.0;
+            Mul64 w[8];
+            for (int kf = k0; kf <= k1; ++kf) {
+                int k, kn;
+                double a, b;
+                side64(X.stz, kf, X.pzp, X.pzn, k, kn, a, b);
+                if (kf == k0 || __double_as_longlong(a) != __double_as_longlong(az) ||
+                    __double_as_longlong(b) != __double_as_longlong(bz)) {
+                    az = a;
+                    bz = b;
+                    w[0] = mul64_factor(mul64(axy, a));
+                    w[1] = mul64_factor(mul64(bxy, a));
+                    w[2] = mul64_factor(mul64(axby, a));
+                    w[3] = mul64_factor(mul64(axy, b));
+                    w[4] = mul64_factor(mul64(bxby, a));
+                    w[5] = mul64_factor(mul64(bxy, b));
+                    w[6] = mul64_factor(mul64(axby, b));
+                    w[7] = mul64_factor(mul64(bxby, b));
+                    den = mul64(sxy, X.szz[kf]);
+                    const double y0 = __dmul_rn(rxy, X.rz[kf]);
+                    y = __fma_rn(y0, __fma_rn(-den, y0, 1.0), y0);
+                }
+                const long long o = X.csz * k, on = X.csz * kn;
+                double t = mul64(w[0], v0[o]);
+                t = __dadd_rn(t, mul64(w[1], vx[o]));
+                t = __dadd_rn(t, mul64(w[2], vy[o]));
+                t = __dadd_rn(t, mul64(w[3], v0[on]));
+                t = __dadd_rn(t, mul64(w[4], vxy[o]));
+                t = __dadd_rn(t, mul64(w[5], vx[on]));
+                t = __dadd_rn(t, mul64(w[6], vy[on]));
+                t = __dadd_rn(t, mul64(w[7], vxy[on]));
+                const double v = quot64_near(t, den, y);
+                const long long q = X.fsz * kf;
+                out[q] = ADD ? __dadd_rn(out[q], v) : v;
+            }
+        }
+}
+
+// Prolongation with the products on the FP64 unit (weights beyond mul64's range).
 template <bool ADD>
 __global__ void __launch_bounds__(kBX *kBY) k_prolong_f64(XferK<double> X, const double *__restrict__ vc,
                                                           double *__restrict__ vf)
@@ -218,22 +416,19 @@ __device__ __forceinline__ double cg_sum_partials(const double *partials, double
 }
 
 // r = b - A x, p = r (src/cg_poisson_matrix.f90:80-91), rsd0tol = temp1 = r.r (:94, :107)
-template <bool TAB>
+template <int MODE>
 __global__ void __launch_bounds__(kBX *kBY) k_cg_init(LevelK<double> L, double *__restrict__ r,
                                                       double *__restrict__ p, const double *__restrict__ x,
                                                       const double *__restrict__ b, double *partials, CgState *st,
                                                       const double *__restrict__ c0t)
 {
     double acc = 0.0;
-    for (int k = blockIdx.z + 1; k <= L.nz; k += gridDim.z)
-        for (int j = blockIdx.y * blockDim.y + threadIdx.y + 1; j <= L.ny; j += gridDim.y * blockDim.y)
-            for (int i = blockIdx.x * blockDim.x + threadIdx.x + 1; i <= L.nx; i += gridDim.x * blockDim.x) {
-                const long long q = lin(i, j, k, L.sy, L.sz);
-                const double v = __dsub_rn(b[q], ax_cell_c0_f64(L, x, i, j, k, diag_at<TAB>(L, c0t, q, i, j, k)));
-                r[q] = v;
-                p[q] = v;
-                acc = __dadd_rn(acc, __dmul_rn(v, v));
-            }
+    each_cell(L, [&](int i, int j, int k, long long q) {
+        const double v = __dsub_rn(b[q], ax_cell<MODE>(L, x, c0t, q, i, j, k));
+        r[q] = v;
+        p[q] = v;
+        acc = add_prod(acc, v, v);
+    });
     __shared__ double sw[kBX * kBY / 32];
     const double s = block_sum(acc, sw);
     if (cg_arrive_last(st, s, partials)) {
@@ -250,21 +445,18 @@ __global__ void __launch_bounds__(kBX *kBY) k_cg_init(LevelK<double> L, double *
 }
 
 // Ap = A p (src/poisson_matrix_operator.f90:146-159), temp2 = Ap.p (:112), alpha (:114)
-template <bool TAB>
+template <int MODE>
 __global__ void __launch_bounds__(kBX *kBY) k_cg_apdot(LevelK<double> L, const double *__restrict__ p,
                                                        double *__restrict__ ap, double *partials, CgState *st,
                                                        const double *__restrict__ c0t)
 {
     if (st->done) return;
     double acc = 0.0;
-    for (int k = blockIdx.z + 1; k <= L.nz; k += gridDim.z)
-        for (int j = blockIdx.y * blockDim.y + threadIdx.y + 1; j <= L.ny; j += gridDim.y * blockDim.y)
-            for (int i = blockIdx.x * blockDim.x + threadIdx.x + 1; i <= L.nx; i += gridDim.x * blockDim.x) {
-                const long long q = lin(i, j, k, L.sy, L.sz);
-                const double v = ax_cell_c0_f64(L, p, i, j, k, diag_at<TAB>(L, c0t, q, i, j, k));
-                ap[q] = v;
-                acc = __dadd_rn(acc, __dmul_rn(v, p[q]));
-            }
+    each_cell(L, [&](int i, int j, int k, long long q) {
+        const double v = ax_cell<MODE>(L, p, c0t, q, i, j, k);
+        ap[q] = v;
+        acc = add_prod(acc, v, p[q]);
+    });
     __shared__ double sw[kBX * kBY / 32];
     const double s = block_sum(acc, sw);
     if (cg_arrive_last(st, s, partials)) {
@@ -287,15 +479,12 @@ __global__ void __launch_bounds__(kBX *kBY) k_cg_update(LevelK<double> L, double
     if (st->done) return;
     const double alpha = st->alpha;
     double acc = 0.0;
-    for (int k = blockIdx.z + 1; k <= L.nz; k += gridDim.z)
-        for (int j = blockIdx.y * blockDim.y + threadIdx.y + 1; j <= L.ny; j += gridDim.y * blockDim.y)
-            for (int i = blockIdx.x * blockDim.x + threadIdx.x + 1; i <= L.nx; i += gridDim.x * blockDim.x) {
-                const long long q = lin(i, j, k, L.sy, L.sz);
-                x[q] = __dadd_rn(x[q], __dmul_rn(alpha, p[q]));
-                const double v = __dsub_rn(r[q], __dmul_rn(alpha, ap[q]));
-                r[q] = v;
-                acc = __dadd_rn(acc, __dmul_rn(v, v));
-            }
+    each_cell(L, [&](int, int, int, long long q) {
+        x[q] = __dadd_rn(x[q], mul64_vv(alpha, p[q]));
+        const double v = __dsub_rn(r[q], mul64_vv(alpha, ap[q]));
+        r[q] = v;
+        acc = add_prod(acc, v, v);
+    });
     __shared__ double sw[kBX * kBY / 32];
     const double s = block_sum(acc, sw);
     if (cg_arrive_last(st, s, partials)) {
@@ -320,12 +509,7 @@ __global__ void __launch_bounds__(kBX *kBY) k_cg_p(LevelK<double> L, double *__r
 {
     if (st->done) return;
     const double beta = st->beta;
-    for (int k = blockIdx.z + 1; k <= L.nz; k += gridDim.z)
-        for (int j = blockIdx.y * blockDim.y + threadIdx.y + 1; j <= L.ny; j += gridDim.y * blockDim.y)
-            for (int i = blockIdx.x * blockDim.x + threadIdx.x + 1; i <= L.nx; i += gridDim.x * blockDim.x) {
-                const long long q = lin(i, j, k, L.sy, L.sz);
-                p[q] = __dadd_rn(r[q], __dmul_rn(beta, p[q]));
-            }
+    each_cell(L, [&](int, int, int, long long q) { p[q] = __dadd_rn(r[q], mul64_vv(beta, p[q])); });
 }
 
 // ------------------------------------------------------------------------------------
@@ -445,6 +629,7 @@ __global__ void __launch_bounds__(256) k_hierarchy(const HierDesc *__restrict__ 
         const int nc = H.n[l + 1][d];
         const double *dmc = meshes + H.mesh_off[l + 1][d];
         double *w = tables + H.w[l][d], *pp = tables + H.pp[l][d], *pn = tables + H.pn[l][d];
+        double *ps = tables + H.ps[l][d], *pr = tables + H.pr[l][d];
         if (l >= H.lvc[d]) {   // the axis is no longer coarsened: stride 1 (src/multigrid.f90:1415-1458)
             for (int i = threadIdx.x; i <= n + 1; i += blockDim.x) {
                 w[i] = dm[i];
@@ -460,6 +645,14 @@ __global__ void __launch_bounds__(256) k_hierarchy(const HierDesc *__restrict__ 
                 pn[f - 1] = __dmul_rn(0.5, dm[f]);
                 pn[f] = __dadd_rn(__dmul_rn(1.0, dm[f + 1]), __dmul_rn(0.5, dm[f]));
             }
+        }
+        __syncthreads();
+        // the prolongation's denominator along the axis (own + neighbour's weight of each
+        // fine cell, as side64 takes them) and its reciprocal
+        const bool one = l >= H.lvc[d];
+        for (int f = threadIdx.x + 1; f <= n; f += blockDim.x) {
+            ps[f] = one ? __dadd_rn(pn[f], pn[f]) : (f & 1) ? __dadd_rn(pp[f], pp[f + 1]) : __dadd_rn(pn[f], pn[f - 1]);
+            pr[f] = __ddiv_rn(1.0, ps[f]);
         }
     }
 }
@@ -484,26 +677,56 @@ void grid_for_cells(const LevelK<double> &L, const Launch &ln, dim3 *grid, dim3 
     *block = dim3(kBX, kBY, 1);
 }
 
+// The grid of the column kernels (each_cell and its kin): the tiles of the (i, j) plane and
+// chunks of planes, of at most 8 so that a thread's column set-up is shared, as long as the
+// grid fills every SM a few times over.
+static dim3 grid_columns(int nx_threads, int ny, int nz, const Launch &ln)
+{
+    dim3 g = grid3(nx_threads, ny, nz, ln);
+    if (ln.collapse[2]) return g;
+    const long long want = 152 * 16;
+    const long long ctas = (long long)g.x * g.y * nz;
+    const int kc = (int)(ctas / want < 1 ? 1 : ctas / want > 8 ? 8 : ctas / want);
+    const int gz = (nz + kc - 1) / kc;
+    g.z = (unsigned)(gz < kMaxGridZ ? gz : kMaxGridZ);
+    return g;
+}
+
+static int arith_mode(const LevelK<double> &L, const double *c0t)
+{
+    return !c0t ? kPlain : L.mul64 ? kInt : kTab;
+}
+
+// Calls f(std::integral_constant<int, MODE>) for the level's arithmetic.
+template <typename F>
+static void with_mode(int mode, F f)
+{
+    if (mode == kInt)
+        f(std::integral_constant<int, kInt>());
+    else if (mode == kTab)
+        f(std::integral_constant<int, kTab>());
+    else
+        f(std::integral_constant<int, kPlain>());
+}
+
 static void launch_rbgs_colour(const LevelK<double> &L, dim3 g, double *x, const double *b, double omega,
                                double omw, int colour, const double *c0t, cudaStream_t s)
 {
     const dim3 bl(kBX, kBY, 1);
     // omega == 1 exactly: 1 * v is v for every double, so the OMEGA1 kernel's bits are the same
-    if (c0t && omega == 1.0)
-        k_rbgs_f64<true, true><<<g, bl, 0, s>>>(L, x, b, omega, omw, colour, c0t);
-    else if (c0t)
-        k_rbgs_f64<true, false><<<g, bl, 0, s>>>(L, x, b, omega, omw, colour, c0t);
-    else if (omega == 1.0)
-        k_rbgs_f64<false, true><<<g, bl, 0, s>>>(L, x, b, omega, omw, colour, nullptr);
-    else
-        k_rbgs_f64<false, false><<<g, bl, 0, s>>>(L, x, b, omega, omw, colour, nullptr);
+    with_mode(arith_mode(L, c0t), [&](auto m) {
+        if (omega == 1.0)
+            k_rbgs_f64<decltype(m)::value, true><<<g, bl, 0, s>>>(L, x, b, omega, omw, colour, c0t);
+        else
+            k_rbgs_f64<decltype(m)::value, false><<<g, bl, 0, s>>>(L, x, b, omega, omw, colour, c0t);
+    });
 }
 
 int f64_rbgs_sweeps(const LevelK<double> &L, const Launch &ln, double *x, const double *b, int iters,
                     double omega, cudaStream_t s, const double *c0t)
 {
     const double omw = 1.0 - omega;   // (1.0d0-omega), src/rbgs_poisson_matrix.f90:250
-    const dim3 g = grid3((L.nx + 1) / 2, L.ny, L.nz, ln);
+    const dim3 g = grid_columns((L.nx + 1) / 2, L.ny, L.nz, ln);
     for (int it = 0; it < iters; ++it)
         for (int c = 0; c < 2; ++c) launch_rbgs_colour(L, g, x, b, omega, omw, c, c0t, s);
     count_launches(2LL * iters);
@@ -513,7 +736,7 @@ int f64_rbgs_sweeps(const LevelK<double> &L, const Launch &ln, double *x, const 
 int f64_rbgs_colour(const LevelK<double> &L, const Launch &ln, double *x, const double *b, double omega, int colour,
                     cudaStream_t s, const double *c0t)
 {
-    const dim3 g = grid3((L.nx + 1) / 2, L.ny, L.nz, ln);
+    const dim3 g = grid_columns((L.nx + 1) / 2, L.ny, L.nz, ln);
     launch_rbgs_colour(L, g, x, b, omega, 1.0 - omega, colour & 1, c0t, s);
     count_launches(1);
     return cuda_status(cudaGetLastError(), "rbgs half-sweep");
@@ -530,18 +753,14 @@ int f64_diag_table(const LevelK<double> &L, double *c0t, cudaStream_t s)
 int f64_residual(const LevelK<double> &L, const Launch &ln, double *r, const double *x, const double *b,
                  double *partials, int *npart, cudaStream_t s, const double *c0t)
 {
-    const dim3 g = grid3(L.nx, L.ny, L.nz, ln), bl(kBX, kBY, 1);
-    if (partials) {
-        if (c0t)
-            k_residual_f64<true, true><<<g, bl, 0, s>>>(L, r, x, b, partials, c0t);
+    const dim3 g = grid_columns(L.nx, L.ny, L.nz, ln), bl(kBX, kBY, 1);
+    with_mode(arith_mode(L, c0t), [&](auto m) {
+        if (partials)
+            k_residual_f64<true, decltype(m)::value><<<g, bl, 0, s>>>(L, r, x, b, partials, c0t);
         else
-            k_residual_f64<true, false><<<g, bl, 0, s>>>(L, r, x, b, partials, nullptr);
-        *npart = (int)(g.x * g.y * g.z);
-    } else if (c0t) {
-        k_residual_f64<false, true><<<g, bl, 0, s>>>(L, r, x, b, nullptr, c0t);
-    } else {
-        k_residual_f64<false, false><<<g, bl, 0, s>>>(L, r, x, b, nullptr, nullptr);
-    }
+            k_residual_f64<false, decltype(m)::value><<<g, bl, 0, s>>>(L, r, x, b, nullptr, c0t);
+    });
+    if (partials) *npart = (int)(g.x * g.y * g.z);
     count_launches(1);
     return cuda_status(cudaGetLastError(), "residual");
 }
@@ -549,11 +768,8 @@ int f64_residual(const LevelK<double> &L, const Launch &ln, double *r, const dou
 int f64_mv_mul(const LevelK<double> &L, const Launch &ln, double *y, const double *x, cudaStream_t s,
                const double *c0t)
 {
-    const dim3 g = grid3(L.nx, L.ny, L.nz, ln), bl(kBX, kBY, 1);
-    if (c0t)
-        k_mvmul_f64<true><<<g, bl, 0, s>>>(L, y, x, c0t);
-    else
-        k_mvmul_f64<false><<<g, bl, 0, s>>>(L, y, x, nullptr);
+    const dim3 g = grid_columns(L.nx, L.ny, L.nz, ln), bl(kBX, kBY, 1);
+    with_mode(arith_mode(L, c0t), [&](auto m) { k_mvmul_f64<decltype(m)::value><<<g, bl, 0, s>>>(L, y, x, c0t); });
     count_launches(1);
     return cuda_status(cudaGetLastError(), "mv_mul");
 }
@@ -577,8 +793,11 @@ int f64_reduce(const double *partials, int n, double *out, cudaStream_t s)
 
 int f64_restrict(const XferK<double> &X, const Launch &ln, const double *vf, double *vc, cudaStream_t s)
 {
-    const dim3 g = grid3(X.ncx, X.ncy, X.ncz, ln), bl(kBX, kBY, 1);
-    k_restrict_f64<<<g, bl, 0, s>>>(X, vf, vc);
+    const dim3 g = grid_columns(X.ncx, X.ncy, X.ncz, ln), bl(kBX, kBY, 1);
+    if (X.mul64)
+        k_restrict_f64<true><<<g, bl, 0, s>>>(X, vf, vc);
+    else
+        k_restrict_f64<false><<<g, bl, 0, s>>>(X, vf, vc);
     count_launches(1);
     return cuda_status(cudaGetLastError(), "restriction");
 }
@@ -586,11 +805,20 @@ int f64_restrict(const XferK<double> &X, const Launch &ln, const double *vf, dou
 int f64_prolong(const XferK<double> &X, const Launch &ln, const double *vc, double *vf, bool add,
                 cudaStream_t s)
 {
-    const dim3 g = grid3(X.ncx, X.ncy, X.ncz, ln), bl(kBX, kBY, 1);
-    if (add)
-        k_prolong_f64<true><<<g, bl, 0, s>>>(X, vc, vf);
-    else
-        k_prolong_f64<false><<<g, bl, 0, s>>>(X, vc, vf);
+    const dim3 bl(kBX, kBY, 1);
+    if (X.mul64) {
+        const dim3 g = grid_columns(X.ncx * X.stx, X.ncy * X.sty, X.ncz * X.stz, ln);
+        if (add)
+            k_prolong_m64<true><<<g, bl, 0, s>>>(X, vc, vf);
+        else
+            k_prolong_m64<false><<<g, bl, 0, s>>>(X, vc, vf);
+    } else {
+        const dim3 g = grid3(X.ncx, X.ncy, X.ncz, ln);
+        if (add)
+            k_prolong_f64<true><<<g, bl, 0, s>>>(X, vc, vf);
+        else
+            k_prolong_f64<false><<<g, bl, 0, s>>>(X, vc, vf);
+    }
     count_launches(1);
     return cuda_status(cudaGetLastError(), "prolongation");
 }
@@ -644,10 +872,9 @@ int f64_cg_partials(const LevelK<double> &L, const Launch &ln)
 int f64_cg_init(const LevelK<double> &L, const Launch &ln, double *r, double *p, const double *x, const double *b,
                 double *partials, CgState *st, cudaStream_t s, const double *c0t)
 {
-    if (c0t)
-        k_cg_init<true><<<cg_grid(L, ln), dim3(kBX, kBY, 1), 0, s>>>(L, r, p, x, b, partials, st, c0t);
-    else
-        k_cg_init<false><<<cg_grid(L, ln), dim3(kBX, kBY, 1), 0, s>>>(L, r, p, x, b, partials, st, nullptr);
+    with_mode(arith_mode(L, c0t), [&](auto m) {
+        k_cg_init<decltype(m)::value><<<cg_grid(L, ln), dim3(kBX, kBY, 1), 0, s>>>(L, r, p, x, b, partials, st, c0t);
+    });
     count_launches(1);
     return cuda_status(cudaGetLastError(), "cg init");
 }
@@ -657,10 +884,8 @@ int f64_cg_iteration(const LevelK<double> &L, const Launch &ln, double *x, doubl
                      const double *c0t)
 {
     const dim3 g = cg_grid(L, ln), bl(kBX, kBY, 1);
-    if (c0t)
-        k_cg_apdot<true><<<g, bl, 0, s>>>(L, p, ap, partials, st, c0t);
-    else
-        k_cg_apdot<false><<<g, bl, 0, s>>>(L, p, ap, partials, st, nullptr);
+    with_mode(arith_mode(L, c0t),
+              [&](auto m) { k_cg_apdot<decltype(m)::value><<<g, bl, 0, s>>>(L, p, ap, partials, st, c0t); });
     k_cg_update<<<g, bl, 0, s>>>(L, x, r, p, ap, partials, st, tol, check ? 1 : 0, iter);
     k_cg_p<<<g, bl, 0, s>>>(L, p, r, st);
     count_launches(3);

@@ -66,6 +66,7 @@ struct HierDesc {
     long long mesh_off[kMaxLevels][3];
     long long cm[kMaxLevels][3], cp[kMaxLevels][3], sx[kMaxLevels];
     long long w[kMaxLevels][3], pp[kMaxLevels][3], pn[kMaxLevels][3];
+    long long ps[kMaxLevels][3], pr[kMaxLevels][3];
 };
 
 // ---- FP64 (bitwise) launchers, pmg_f64.cu -------------------------------------
@@ -79,7 +80,8 @@ int f64_rbgs_sweeps(const LevelK<double> &L, const Launch &ln, double *x, const 
 // (src/rbgs_poisson_matrix.f90:242, :260; colour carries a rank's parity offset).
 int f64_rbgs_colour(const LevelK<double> &L, const Launch &ln, double *x, const double *b, double omega, int colour,
                     cudaStream_t s, const double *c0t = nullptr);
-// c0t = diag_f64 of every interior cell of level L (an array of the level's layout).
+// c0t = diag_f64 of every interior cell of level L (an array of the level's layout), followed
+// by an array of its reciprocals (recip_f64).
 int f64_diag_table(const LevelK<double> &L, double *c0t, cudaStream_t s);
 // r = b - A x (interior); if partials != nullptr also writes per-block sums of r^2
 // and returns the number of partials in *npart.

@@ -1,0 +1,163 @@
+// pmg_mul64.cuh -- FP64 products on the integer pipe, bit for bit.
+//
+// The bitwise FP64 kernels are bound by this part's FP64 unit: one warp instruction per 19
+// clocks per SM, whether add, multiply or FMA, while integer and FP32 instructions issue at
+// two to four per clock beside it.  A 53 x 53 bit product rounded to nearest even takes about
+// 35 integer instructions (four high and three low 32-bit products, a shift by at most one
+// place, a round-up by the carry of the first dropped bit): 13 to 17 clocks per SM that
+// overlap with the FP64 unit's (measured: 7 products and 8 additions per cell 167 clocks
+// instead of 300).  So the kernels below form their products here and leave the FP64 unit
+// the additions and the two FMAs of a division.
+//
+// mul64(f, x) returns RN(f x) for every double x, f a factor decoded once by mul64_factor:
+//  * x normal with an exponent within 2^+-500, f's exponent within 2^+-400 (the callers
+//    check the operator's tables once per level): the integer product;
+//  * x = +-0: a zero with the product's sign;
+//  * everything else (subnormal, huge, infinite, NaN): __dmul_rn, in a function of its own --
+//    in line, the compiler turns the branch into a multiplication that every thread executes.
+#pragma once
+
+namespace pmg {
+namespace {
+
+struct Mul64 {
+    unsigned h, l;   // the 53-bit significand, shifted up to bit 63
+    unsigned e;      // sign and exponent, at their place in the high word, less 1024 << 20
+                     // (the bias, and 1 for the implicit bit that mul64_core's sum brings)
+};
+
+__device__ __forceinline__ Mul64 mul64_factor(double f)
+{
+    const unsigned fh = (unsigned)__double2hiint(f), fl = (unsigned)__double2loint(f);
+    Mul64 r;
+    r.h = __funnelshift_l(fl, (fh & 0xfffffu) | 0x100000u, 11);
+    r.l = fl << 11;
+    r.e = (fh & 0xfff00000u) - (1024u << 20);
+    return r;
+}
+
+__device__ __noinline__ double mul64_slow(unsigned h, unsigned l, unsigned e, double x)
+{
+    const unsigned fh = ((h >> 11) & 0xfffffu) + e + (1024u << 20);
+    return __dmul_rn(__hiloint2double((int)fh, (int)__funnelshift_r(l, h, 11)), x);
+}
+
+__device__ __noinline__ double mul64_slow_vv(double a, double b) { return __dmul_rn(a, b); }
+
+__device__ __noinline__ double div64_slow(double d, double c) { return __ddiv_rn(d, c); }
+
+// Exponent field in [523, 1523].
+__device__ __forceinline__ bool mul64_in_range(unsigned xh)
+{
+    return xh + xh - (523u << 21) < (1001u << 21);
+}
+
+__device__ __forceinline__ bool is_zero64(unsigned xh, unsigned xl) { return ((xh << 1) | xl) == 0u; }
+
+// f x for x in range.
+__device__ __forceinline__ double mul64_core(const Mul64 &f, unsigned xh, unsigned xl)
+{
+    const unsigned mh = (xh & 0xfffffu) | 0x100000u;
+    // words 1, 2 and 3 of the 128-bit product (m1, h0, h1); word 0 only settles ties
+    unsigned m1, h0, h1;
+    {
+        const unsigned p0h = __umulhi(xl, f.l), p1l = xl * f.h, p1h = __umulhi(xl, f.h);
+        const unsigned p2l = mh * f.l, p2h = __umulhi(mh, f.l), p3l = mh * f.h, p3h = __umulhi(mh, f.h);
+        asm("add.cc.u32 %0, %3, %4;\n\t"
+            "addc.cc.u32 %1, %5, %6;\n\t"
+            "addc.u32 %2, %7, 0;\n\t"
+            "add.cc.u32 %0, %0, %8;\n\t"
+            "addc.cc.u32 %1, %1, %9;\n\t"
+            "addc.u32 %2, %2, 0;"
+            : "=&r"(m1), "=&r"(h0), "=&r"(h1)
+            : "r"(p0h), "r"(p1l), "r"(p1h), "r"(p3l), "r"(p3h), "r"(p2l), "r"(p2h));
+    }
+    // the significand is bits 52 .. 0 of (h1, h0) when bit 52 is set, else one place lower
+    const unsigned top = h1 & 0x100000u;
+    if (!top) {
+        h1 = __funnelshift_l(h0, h1, 1);
+        h0 = __funnelshift_l(m1, h0, 1);
+        m1 <<= 1;
+    }
+    // the first dropped bit rounds up, except on a tie (word 0 zero too) with an even
+    // significand; factors of few bits, such as those of uniform meshes, tie often
+    if (m1 == 0x80000000u && (h0 & 1u) == 0u && xl * f.l == 0u) m1 = 0u;
+    unsigned rl, rh;
+    asm("{\n\t.reg .u32 t;\n\t"
+        "add.cc.u32 t, %2, 0x80000000;\n\t"
+        "addc.cc.u32 %0, %3, 0;\n\t"
+        "addc.u32 %1, %4, %5;\n\t}"
+        : "=&r"(rl), "=r"(rh)
+        : "r"(m1), "r"(h0), "r"(h1), "r"((xh & 0xfff00000u) + f.e + top));
+    return __hiloint2double((int)rh, (int)rl);
+}
+
+__device__ __forceinline__ double mul64(const Mul64 &f, double x)
+{
+    const unsigned xh = (unsigned)__double2hiint(x), xl = (unsigned)__double2loint(x);
+    double r = mul64_core(f, xh, xl);
+    if (!mul64_in_range(xh)) {
+        if (is_zero64(xh, xl))
+            r = __hiloint2double((int)((xh ^ (f.e + (1024u << 20))) & 0x80000000u), 0);
+        else
+            r = mul64_slow(f.h, f.l, f.e, x);
+    }
+    return r;
+}
+
+// a b of two variable operands (a sum of squares, a dot product).
+__device__ __forceinline__ double mul64_vv(double a, double b)
+{
+    const unsigned ah = (unsigned)__double2hiint(a), al = (unsigned)__double2loint(a);
+    const unsigned bh = (unsigned)__double2hiint(b), bl = (unsigned)__double2loint(b);
+    double r = mul64_core(mul64_factor(a), bh, bl);
+    const bool ia = mul64_in_range(ah), ib = mul64_in_range(bh);
+    if (!(ia && ib)) {
+        const bool za = is_zero64(ah, al), zb = is_zero64(bh, bl);
+        if ((za || zb) && (ia || za) && (ib || zb))
+            r = __hiloint2double((int)((ah ^ bh) & 0x80000000u), 0);
+        else
+            r = mul64_slow_vv(a, b);
+    }
+    return r;
+}
+
+// d / c with y = recip_f64(c) as quot_f64 (pmg_common.cuh), the first product here.
+__device__ __forceinline__ double quot64(double d, double c, double y)
+{
+    const unsigned dh = (unsigned)__double2hiint(d), dl = (unsigned)__double2loint(d);
+    const double q0 = mul64_core(mul64_factor(y), dh, dl);
+    const double r = __fma_rn(-c, q0, d);
+    double q = __fma_rn(r, y, q0);
+    if (!mul64_in_range(dh) || ((unsigned)__double2hiint(y) & 0x7ff00000u) == 0x7ff00000u) {
+        if (is_zero64(dh, dl) && ((unsigned)__double2hiint(y) & 0x7ff00000u) != 0x7ff00000u)
+            q = __hiloint2double((int)((dh ^ (unsigned)__double2hiint(c)) & 0x80000000u), 0);
+        else
+            q = div64_slow(d, c);
+    }
+    return q;
+}
+
+// d / c with y the result of one Newton step on a y0 within 2^-48 of 1/c (relative), for a c
+// that changes from cell to cell: y = RN((1/c)(1 - e)), e < 2^-95, so it may miss the rounded
+// reciprocal only next to a midpoint and |delta| <= 2^-54 (1 + 2^-40) in the argument at
+// recip_f64.  That argument then holds for every d and c whose significands lie below
+// 2 (1 - 2^-20); others, and operands out of range, take the IEEE division.
+__device__ __forceinline__ double quot64_near(double d, double c, double y)
+{
+    const unsigned dh = (unsigned)__double2hiint(d), dl = (unsigned)__double2loint(d);
+    const unsigned ch = (unsigned)__double2hiint(c);
+    const double q0 = mul64_core(mul64_factor(y), dh, dl);
+    const double r = __fma_rn(-c, q0, d);
+    double q = __fma_rn(r, y, q0);
+    if (!mul64_in_range(dh) || (dh & 0xfffffu) == 0xfffffu || (ch & 0xfffffu) == 0xfffffu) {
+        if (is_zero64(dh, dl))
+            q = __hiloint2double((int)((dh ^ ch) & 0x80000000u), 0);
+        else
+            q = div64_slow(d, c);
+    }
+    return q;
+}
+
+}  // namespace
+}  // namespace pmg
