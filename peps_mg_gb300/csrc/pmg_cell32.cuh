@@ -522,11 +522,61 @@ __device__ void t32_sweeps(const LevelK<float> &L, float *x, const float *b, int
         }
 }
 
-// The single-CTA FP32 coarse tail for one problem on the level descriptors Ls / Xs and
-// arrays xs / bs (the global arrays of D, or shared-memory copies).
-__device__ void tail32_run(const TailDesc<float> &D, const LevelK<float> *Ls, const XferK<float> *Xs,
-                           float *const *xs, float *const *bs, double *sw)
+// The coarsest level of the FP32 tail, solved in FP64 (b converted up, x converted down), so
+// that its convergence test against the FP64 tolerance is attainable.
+__device__ void tail32_coarsest(const TailDesc<float> &D, const LevelK<float> &L, float *x, const float *b, double *sw)
 {
+    const LevelK<double> &C = D.C64;
+    const int chip = chip_threads(C.nx, C.ny, C.nz);
+    const bool fma_form = C.nx * C.ny * C.nz <= 64;
+    if (chip > 0 && (D.coarse_solver != 0 || (chip <= (int)blockDim.x && (fma_form || C.mul64)))) {
+        // small coarsest level: in shared memory; levels of at most 64 cells take the FMA
+        // form of the RBGS solver (the FP32 cycle is not bound to the reference's bits)
+        __shared__ double cs[5][kChipCoarseMax];
+        const int total = (int)(C.sz * (C.nz + 2));
+        for (int q = threadIdx.x; q < total; q += blockDim.x) cs[1][q] = 0.0;
+        __syncthreads();
+        for_cells(L.nx, L.ny, L.nz, [&](int i, int j, int k) {
+            cs[1][lin(i, j, k, C.sy, C.sz)] = (double)b[lin(i, j, k, L.sy, L.sz)];
+        });
+        __syncthreads();
+        int iters = 0, xs64 = 0;
+        if (D.coarse_solver != 0) {
+            if (threadIdx.x < 32)
+                iters = coarse_cg_warp_f64(C, cs[0], cs[1], cs[2], cs[3], cs[4], D.coarse_maxit, D.tol, D.abort);
+        } else if (fma_form) {
+            iters = coarse_rbgs_chip<false, false>(C, cs, D.coarse_maxit, D.tol, D.omega64, D.omw64, D.abort, &xs64);
+        } else if (C.nx * C.ny * C.nz <= 128) {
+            iters = coarse_rbgs_chip<true, false>(C, cs, D.coarse_maxit, D.tol, D.omega64, D.omw64, D.abort, &xs64);
+        } else {
+            iters = coarse_rbgs_chip<true, true>(C, cs, D.coarse_maxit, D.tol, D.omega64, D.omw64, D.abort, &xs64);
+        }
+        if (threadIdx.x == 0 && D.iters_out) *D.iters_out = iters;
+        __syncthreads();
+        for_cells(L.nx, L.ny, L.nz, [&](int i, int j, int k) {
+            x[lin(i, j, k, L.sy, L.sz)] = (float)cs[xs64][lin(i, j, k, C.sy, C.sz)];
+        });
+    } else {
+        for_cells(L.nx, L.ny, L.nz, [&](int i, int j, int k) {
+            D.cb64[lin(i, j, k, C.sy, C.sz)] = (double)b[lin(i, j, k, L.sy, L.sz)];
+        });
+        __syncthreads();
+        const int iters = coarse_solve_f64(C, D.cx64, D.cb64, D.cp64, D.cap64, D.crr64, D.coarse_solver,
+                                           D.coarse_maxit, D.tol, D.omega64, D.omw64, sw, D.abort);
+        for_cells(L.nx, L.ny, L.nz, [&](int i, int j, int k) {
+            x[lin(i, j, k, L.sy, L.sz)] = (float)D.cx64[lin(i, j, k, C.sy, C.sz)];
+        });
+        if (threadIdx.x == 0 && D.iters_out) *D.iters_out = iters;
+    }
+    __syncthreads();
+}
+
+// The single-CTA FP32 coarse tail for one problem on its global arrays.
+__device__ void tail32_body(const TailDesc<float> &D, double *sw)
+{
+    const LevelK<float> *Ls = D.L;
+    const XferK<float> *Xs = D.X;
+    float *const *xs = D.x, *const *bs = D.b;
     const float omega = D.omega, omw = D.omw;
     for (int l = D.l0; l < D.nl; ++l) {
         const LevelK<float> L = Ls[l];
@@ -539,53 +589,7 @@ __device__ void tail32_run(const TailDesc<float> &D, const LevelK<float> *Ls, co
         });
         __syncthreads();
     }
-    // coarsest level: solved in FP64 (b converted up, x converted down), so its
-    // convergence test against the FP64 tolerance is attainable
-    {
-        const LevelK<float> L = Ls[D.nl];
-        const LevelK<double> &C = D.C64;
-        float *x = xs[D.nl];
-        const float *b = bs[D.nl];
-        const int chip = chip_threads(C.nx, C.ny, C.nz);
-        if (chip > 0 && (D.coarse_solver != 0 || chip <= (int)blockDim.x)) {
-            // small coarsest level: in shared memory; levels of at most 64 cells take the FMA
-            // form of the RBGS solver (the FP32 cycle is not bound to the reference's bits)
-            __shared__ double cs[5][kChipCoarseMax];
-            const int total = (int)(C.sz * (C.nz + 2));
-            for (int q = threadIdx.x; q < total; q += blockDim.x) cs[1][q] = 0.0;
-            __syncthreads();
-            for_cells(L.nx, L.ny, L.nz, [&](int i, int j, int k) {
-                cs[1][lin(i, j, k, C.sy, C.sz)] = (double)b[lin(i, j, k, L.sy, L.sz)];
-            });
-            __syncthreads();
-            int iters = 0, xs64 = 0;
-            if (D.coarse_solver != 0) {
-                if (threadIdx.x < 32)
-                    iters = coarse_cg_warp_f64(C, cs[0], cs[1], cs[2], cs[3], cs[4], D.coarse_maxit, D.tol, D.abort);
-            } else if (C.nx * C.ny * C.nz <= 64) {
-                iters = coarse_rbgs_chip<false>(C, cs, D.coarse_maxit, D.tol, D.omega64, D.omw64, D.abort, &xs64);
-            } else {
-                iters = coarse_rbgs_chip<true>(C, cs, D.coarse_maxit, D.tol, D.omega64, D.omw64, D.abort, &xs64);
-            }
-            if (threadIdx.x == 0 && D.iters_out) *D.iters_out = iters;
-            __syncthreads();
-            for_cells(L.nx, L.ny, L.nz, [&](int i, int j, int k) {
-                x[lin(i, j, k, L.sy, L.sz)] = (float)cs[xs64][lin(i, j, k, C.sy, C.sz)];
-            });
-        } else {
-            for_cells(L.nx, L.ny, L.nz, [&](int i, int j, int k) {
-                D.cb64[lin(i, j, k, C.sy, C.sz)] = (double)b[lin(i, j, k, L.sy, L.sz)];
-            });
-            __syncthreads();
-            const int iters = coarse_solve_f64(C, D.cx64, D.cb64, D.cp64, D.cap64, D.crr64, D.coarse_solver,
-                                               D.coarse_maxit, D.tol, D.omega64, D.omw64, sw, D.abort);
-            for_cells(L.nx, L.ny, L.nz, [&](int i, int j, int k) {
-                x[lin(i, j, k, L.sy, L.sz)] = (float)D.cx64[lin(i, j, k, C.sy, C.sz)];
-            });
-            if (threadIdx.x == 0 && D.iters_out) *D.iters_out = iters;
-        }
-        __syncthreads();
-    }
+    tail32_coarsest(D, Ls[D.nl], xs[D.nl], bs[D.nl], sw);
     for (int l = D.nl - 1; l >= D.l0; --l) {
         const LevelK<float> L = Ls[l];
         const XferK<float> X = Xs[l];
@@ -597,56 +601,188 @@ __device__ void tail32_run(const TailDesc<float> &D, const LevelK<float> *Ls, co
     }
 }
 
-__device__ void tail32_body(const TailDesc<float> &D, double *sw) { tail32_run(D, D.L, D.X, D.x, D.b, sw); }
+// ---------------------------------------------------------------------------------------
+// The tail with x and b of every tail level, the residual of one and the levels' tables in
+// shared memory `sm` (offsets in D, each array in the level's unpadded (nx+2)(ny+2)(nz+2)
+// layout): b of the first tail level comes in from global memory and x of that level goes
+// back, every other access stays on chip.
+//
+// A launch meets each of its loops once or a few times with a cold instruction cache, so what
+// bounds it is the code's length and the divisions of the index arithmetic, not the
+// arithmetic: the residual-restriction is a loop over fine cells and one over coarse cells
+// (instead of eight stencils in line), the prolongation one over fine cells (instead of eight
+// children in line), and cell indices come from a multiplication (fastdiv).  Same operations
+// per cell, in the same order, as rbgs32, resrestrict_cell32 and prolong_add_cell32.
+// Measured (levels 16^3 .. 2^3, 10 coarsest iterations): 77 -> 57 us a launch, of which the
+// 16^3 level's eight half-sweeps take 13 us and the coarsest solve 16 us.
+// ---------------------------------------------------------------------------------------
+struct Tail32Level {
+    LevelK<float> L;
+    XferK<float> X;
+    float *x, *b;
+    unsigned dhx, dnx, dny;      // fastdiv's factors of (nx+1)/2, nx and ny
+};
 
-// The tail with x and b of every tail level copied into shared memory `sm` (D.sm_floats
-// floats, each array in the level's unpadded (nx+2)(ny+2)(nz+2) layout): b of the first
-// tail level comes in from global memory and x of that level goes back, every other
-// access stays on chip.
+// q / d for q < 2^18 and d <= 2^12, m = fastdiv_factor(d): 2^32/d rounded up, and 0 for d = 1
+__device__ __forceinline__ unsigned fastdiv_factor(unsigned d) { return d > 1 ? 0xffffffffu / d + 1u : 0u; }
+__device__ __forceinline__ int fastdiv(int q, unsigned m) { return m ? (int)__umulhi((unsigned)q, m) : q; }
+
+// f(i, j, k, p) for every interior cell of the level
+template <typename F>
+__device__ __forceinline__ void tail32_cells(const Tail32Level &T, F f)
+{
+    const int nx = T.L.nx, ny = T.L.ny, n = nx * ny * T.L.nz, sy = T.L.sy, sz = (int)T.L.sz;
+    for (int q = threadIdx.x; q < n; q += blockDim.x) {
+        const int rr = fastdiv(q, T.dnx), kk = fastdiv(rr, T.dny);
+        const int i = q - rr * nx + 1, j = rr - kk * ny + 1, k = kk + 1;
+        f(i, j, k, i + sy * j + sz * k);
+    }
+}
+
+__device__ __forceinline__ float tail32_nbsum(const LevelK<float> &L, const float *x, int p, int i, int j, int k)
+{
+    const int sy = L.sy, sz = (int)L.sz;
+    float t = L.cxm[i] * x[p - 1];
+    t = fmaf(L.cxp[i], x[p + 1], t);
+    t = fmaf(L.cym[j], x[p - sy], t);
+    t = fmaf(L.cyp[j], x[p + sy], t);
+    t = fmaf(L.czm[k], x[p - sz], t);
+    t = fmaf(L.czp[k], x[p + sz], t);
+    return t;
+}
+
+__device__ __noinline__ void tail32_sweeps(const Tail32Level &T, int iters, float omega, float omw, bool zero_start)
+{
+    const LevelK<float> &L = T.L;
+    float *x = T.x;
+    const float *b = T.b;
+    const int hx = (L.nx + 1) / 2, nq = hx * L.ny * L.nz, ny = L.ny, nx = L.nx, sy = L.sy, sz = (int)L.sz;
+    for (int h = 0; h < 2 * iters; ++h) {
+        const bool first = zero_start && h == 0;    // x = 0 (the arrays were cleared)
+#pragma unroll 1
+        for (int q = threadIdx.x; q < nq; q += blockDim.x) {
+            const int rr = fastdiv(q, T.dhx), kk = fastdiv(rr, T.dny);
+            const int t = q - rr * hx, j = rr - kk * ny + 1, k = kk + 1;
+            const int i = 2 * t + 1 + ((j + k + h) & 1);
+            if (i > nx) continue;
+            const int p = i + sy * j + sz * k;
+            const float c0 = diag32(L, i, j, k);
+            if (first)
+                x[p] = __fdividef(omega * b[p], c0);
+            else
+                x[p] = fmaf(omw, x[p], __fdividef(omega * (b[p] - tail32_nbsum(L, x, p, i, j, k)), c0));
+        }
+        __syncthreads();
+    }
+}
+
 __device__ void tail32_body_smem(const TailDesc<float> &D, double *sw, float *sm)
 {
-    __shared__ LevelK<float> sL[kMaxLevels];
-    __shared__ XferK<float> sX[kMaxLevels];
-    __shared__ float *sxp[kMaxLevels], *sbp[kMaxLevels];
-    if (threadIdx.x == 0) {
-        int off = 0;
-        for (int l = D.l0; l <= D.nl; ++l) {
-            LevelK<float> L = D.L[l];
-            L.sy = L.nx + 2;
-            L.sz = (long long)L.sy * (L.ny + 2);
-            const int tot = (int)(L.sz * (L.nz + 2));
-            sL[l] = L;
-            sxp[l] = sm + off;
-            off += (tot + 3) & ~3;
-            sbp[l] = sm + off;
-            off += (tot + 3) & ~3;
+    __shared__ Tail32Level T[kMaxLevels];
+    const int l0 = D.l0, nl = D.nl;
+    if ((int)threadIdx.x >= l0 && (int)threadIdx.x <= nl) {
+        const int l = threadIdx.x;
+        Tail32Level t;
+        t.L = D.L[l];
+        t.L.sy = t.L.nx + 2;
+        t.L.sz = (long long)t.L.sy * (t.L.ny + 2);
+        // the tables' shared copies
+        auto at = [&](const float *&p) { p = sm + D.sm_tab + (p - D.tab); };
+        at(t.L.cxm);
+        at(t.L.cxp);
+        at(t.L.sx);
+        at(t.L.cym);
+        at(t.L.cyp);
+        at(t.L.czm);
+        at(t.L.czp);
+        if (l < nl) {
+            t.X = D.X[l];
+            t.X.fsy = t.L.sy;
+            t.X.fsz = t.L.sz;
+            t.X.csy = D.L[l + 1].nx + 2;
+            t.X.csz = (long long)t.X.csy * (D.L[l + 1].ny + 2);
+            at(t.X.wx);
+            at(t.X.wy);
+            at(t.X.wz);
+            at(t.X.pxp);
+            at(t.X.pxn);
+            at(t.X.pyp);
+            at(t.X.pyn);
+            at(t.X.pzp);
+            at(t.X.pzn);
         }
-        for (int l = D.l0; l < D.nl; ++l) {
-            XferK<float> X = D.X[l];
-            X.fsy = sL[l].sy;
-            X.fsz = sL[l].sz;
-            X.csy = sL[l + 1].sy;
-            X.csz = sL[l + 1].sz;
-            sX[l] = X;
-        }
+        t.x = sm + D.sm_x[l];
+        t.b = sm + D.sm_b[l];
+        t.dhx = fastdiv_factor((t.L.nx + 1) / 2);
+        t.dnx = fastdiv_factor(t.L.nx);
+        t.dny = fastdiv_factor(t.L.ny);
+        T[l] = t;
     }
-    for (int q = threadIdx.x; q < D.sm_floats; q += blockDim.x) sm[q] = 0.f;
+    for (int q = threadIdx.x; q < D.sm_tab; q += blockDim.x) sm[q] = 0.f;
+    for (int q = threadIdx.x; q < D.sm_floats - D.sm_tab; q += blockDim.x) sm[D.sm_tab + q] = D.tab[q];
     __syncthreads();
-    const LevelK<float> &G = D.L[D.l0];
-    const LevelK<float> &S = sL[D.l0];
+    const float omega = D.omega, omw = D.omw;
+    float *r = sm + D.sm_r;
     {
-        const float *gb = D.b[D.l0];
-        float *sb = sbp[D.l0];
-        for_cells(G.nx, G.ny, G.nz,
-                  [&](int i, int j, int k) { sb[lin(i, j, k, S.sy, S.sz)] = gb[lin(i, j, k, G.sy, G.sz)]; });
+        const LevelK<float> &G = D.L[l0];
+        const int gsy = G.sy;
+        const long long gsz = G.sz;
+        const float *gb = D.b[l0];
+        tail32_cells(T[l0], [&](int i, int j, int k, int p) { T[l0].b[p] = gb[lin(i, j, k, gsy, gsz)]; });
     }
     __syncthreads();
-    tail32_run(D, sL, sX, sxp, sbp, sw);
+    for (int l = l0; l < nl; ++l) {
+        const Tail32Level &F = T[l];
+        tail32_sweeps(F, D.maxit, omega, omw, true);
+        tail32_cells(F, [&](int i, int j, int k, int p) {
+            r[p] = F.b[p] - fmaf(diag32(F.L, i, j, k), F.x[p], tail32_nbsum(F.L, F.x, p, i, j, k));
+        });
+        __syncthreads();
+        const XferK<float> &X = F.X;
+        float *bc = T[l + 1].b;
+        tail32_cells(T[l + 1], [&](int i, int j, int k, int p) {
+            const int ip = i * X.stx, iz = ip - (X.stx - 1);
+            const int jp = j * X.sty, jz = jp - (X.sty - 1);
+            const int kp = k * X.stz, kz = kp - (X.stz - 1);
+            const float xz = X.wx[iz], xp = X.wx[ip], yz = X.wy[jz], yp = X.wy[jp], zz = X.wz[kz], zp = X.wz[kp];
+            float vol = 0.f, s = 0.f;
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                const int q = ((c & 1) ? iz : ip) + X.fsy * ((c & 2) ? jz : jp) + (int)X.fsz * ((c & 4) ? kz : kp);
+                const float wv = ((c & 1) ? xp : xz) * ((c & 2) ? yp : yz) * ((c & 4) ? zp : zz);
+                vol += wv;
+                s = fmaf(wv, r[q], s);
+            }
+            bc[p] = __fdividef(s, vol);
+        });
+        __syncthreads();
+    }
+    tail32_coarsest(D, T[nl].L, T[nl].x, T[nl].b, sw);
+    for (int l = nl - 1; l >= l0; --l) {
+        const Tail32Level &F = T[l];
+        const XferK<float> &X = F.X;
+        const float *xc = T[l + 1].x;
+        tail32_cells(F, [&](int fi, int jf, int kf, int p) {
+            int i, in, j, jn, k, kn;
+            float ax, bx, ay, by, az, bz;
+            side_weights(X.stx, fi, X.pxp, X.pxn, &i, &in, &ax, &bx);
+            side_weights(X.sty, jf, X.pyp, X.pyn, &j, &jn, &ay, &by);
+            side_weights(X.stz, kf, X.pzp, X.pzn, &k, &kn, &az, &bz);
+            const int csy = X.csy, csz = (int)X.csz;
+            const float *v0 = xc + csy * j + csz * k, *vy = xc + csy * jn + csz * k;
+            const float *vz = xc + csy * j + csz * kn, *vyz = xc + csy * jn + csz * kn;
+            F.x[p] += prolong_child32(ax, bx, ay, by, az, bz, v0[i], v0[in], vy[i], vz[i], vy[in], vz[in], vyz[i],
+                                      vyz[in]);
+        });
+        __syncthreads();
+        tail32_sweeps(F, D.maxit, omega, omw, false);
+    }
     {
-        float *gx = D.x[D.l0];
-        const float *sx = sxp[D.l0];
-        for_cells(G.nx, G.ny, G.nz,
-                  [&](int i, int j, int k) { gx[lin(i, j, k, G.sy, G.sz)] = sx[lin(i, j, k, S.sy, S.sz)]; });
+        const LevelK<float> &G = D.L[l0];
+        const int gsy = G.sy;
+        const long long gsz = G.sz;
+        float *gx = D.x[l0];
+        tail32_cells(T[l0], [&](int i, int j, int k, int p) { gx[lin(i, j, k, gsy, gsz)] = T[l0].x[p]; });
     }
     __syncthreads();
 }

@@ -97,7 +97,7 @@ __device__ __forceinline__ double diag_f64(const LevelK<double> &L, int i, int j
     return -s;
 }
 
-// Division by the diagonal with its reciprocal at hand.  An IEEE division costs this part's
+// Division by the diagonal with its reciprocal at hand (quot64, pmg_mul64.cuh).  An IEEE division costs this part's
 // FP64 pipe (one warp instruction per 19 clocks per SM, each 64 clocks long) seven to nine
 // operations; a product and two FMAs give the same bits when y = RN(1/c) (Markstein's
 // theorem): q0 = RN(d y), r = d - c q0 (exact), q = RN(q0 + r y).  With c = m 2^k, m in
@@ -120,21 +120,6 @@ __device__ __forceinline__ double recip_f64(double c)
     const double off = fabs(__fma_rn(-c, y, 1.0));
     const bool ok = e - 623u <= 800u && off <= __dmul_rn(m54, 1.0 - 0x1p-40);
     return ok ? y : __longlong_as_double(0x7ff8000000000000LL);
-}
-
-// d / c, y = recip_f64(c)
-__device__ __forceinline__ double quot_f64(double d, double c, double y)
-{
-    const double q0 = __dmul_rn(d, y);
-    const double r = __fma_rn(-c, q0, d);
-    double q = __fma_rn(r, y, q0);
-    const unsigned dh = (unsigned)__double2hiint(d), dl = (unsigned)__double2loint(d);
-    const bool zero = ((dh << 1) | dl) == 0u;
-    if (zero) q = __hiloint2double((int)((dh ^ (unsigned)__double2hiint(c)) & 0x80000000u), 0);
-    const bool ok = (((dh >> 20) & 0x7ffu) - 523u <= 1000u || zero) &&
-                    (((unsigned)__double2hiint(y) >> 20) & 0x7ffu) != 0x7ffu;
-    if (!ok) q = __ddiv_rn(d, c);
-    return q;
 }
 
 // q + 0 * x with the bits of the two FP64 operations, on the integer pipe: for finite x the

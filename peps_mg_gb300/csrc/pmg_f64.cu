@@ -239,13 +239,13 @@ __global__ void __launch_bounds__(kBX *kBY) k_restrict_f64(XferK<double> X, cons
                     y = recip_f64(vol);
                 }
                 // v11* meets the plane kp's children first (src/multigrid.f90:1483-1490)
-                double s = 0.0;
+                double v[8], s[8];
 #pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                    const double v = mul64(w[c], vf[o[c & 3] + X.fsz * (c < 4 ? kp : kz)]);
-                    s = c == 0 ? v : __dadd_rn(s, v);
-                }
-                vc[lin(i, j, k, X.csy, X.csz)] = quot64(s, vol, y);
+                for (int c = 0; c < 8; ++c) v[c] = vf[o[c & 3] + X.fsz * (c < 4 ? kp : kz)];
+                mul64n<8>(w, v, s);
+#pragma unroll
+                for (int c = 1; c < 8; ++c) s[0] = __dadd_rn(s[0], s[c]);
+                vc[lin(i, j, k, X.csy, X.csz)] = quot64(s[0], vol, y);
             }
         }
 }
@@ -317,15 +317,12 @@ __global__ void __launch_bounds__(kBX *kBY) k_prolong_m64(XferK<double> X, const
                     y = __fma_rn(y0, __fma_rn(-den, y0, 1.0), y0);
                 }
                 const long long o = X.csz * k, on = X.csz * kn;
-                double t = mul64(w[0], v0[o]);
-                t = __dadd_rn(t, mul64(w[1], vx[o]));
-                t = __dadd_rn(t, mul64(w[2], vy[o]));
-                t = __dadd_rn(t, mul64(w[3], v0[on]));
-                t = __dadd_rn(t, mul64(w[4], vxy[o]));
-                t = __dadd_rn(t, mul64(w[5], vx[on]));
-                t = __dadd_rn(t, mul64(w[6], vy[on]));
-                t = __dadd_rn(t, mul64(w[7], vxy[on]));
-                const double v = quot64_near(t, den, y);
+                const double v8[8] = {v0[o], vx[o], vy[o], v0[on], vxy[o], vx[on], vy[on], vxy[on]};
+                double t[8];
+                mul64n<8>(w, v8, t);
+#pragma unroll
+                for (int u = 1; u < 8; ++u) t[0] = __dadd_rn(t[0], t[u]);
+                const double v = quot64_near(t[0], den, y);
                 const long long q = X.fsz * kf;
                 out[q] = ADD ? __dadd_rn(out[q], v) : v;
             }
@@ -540,7 +537,7 @@ __global__ void __launch_bounds__(kTailThreads) k_tail_f64(const TailDesc<double
         const LevelK<double> &C = D.C64;
         const int chip = chip_threads(C.nx, C.ny, C.nz);
         int iters;
-        if (D.coarse_solver == 0 && chip > 0 && chip <= (int)blockDim.x) {
+        if (D.coarse_solver == 0 && C.mul64 && chip > 0 && chip <= (int)blockDim.x) {
             __shared__ double cs[5][kChipCoarseMax];
             const int total = (int)(C.sz * (C.nz + 2));
             const long long csy = C.sy, csz = C.sz;
@@ -550,7 +547,10 @@ __global__ void __launch_bounds__(kTailThreads) k_tail_f64(const TailDesc<double
                 cs[1][q] = in ? D.cb64[q] : 0.0;
             }
             int xs;
-            iters = coarse_rbgs_chip<true>(C, cs, D.coarse_maxit, D.tol, D.omega64, D.omw64, D.abort, &xs);
+            if (C.nx * C.ny * C.nz > 128)
+                iters = coarse_rbgs_chip<true, true>(C, cs, D.coarse_maxit, D.tol, D.omega64, D.omw64, D.abort, &xs);
+            else
+                iters = coarse_rbgs_chip<true, false>(C, cs, D.coarse_maxit, D.tol, D.omega64, D.omw64, D.abort, &xs);
             for (int q = threadIdx.x; q < total; q += blockDim.x) D.cx64[q] = cs[xs][q];
         } else {
             iters = coarse_solve_f64(C, D.cx64, D.cb64, D.cp64, D.cap64, D.crr64, D.coarse_solver, D.coarse_maxit,

@@ -46,9 +46,12 @@ struct TailDesc {
     LevelK<double> C64;
     double *cx64, *cb64, *cp64, *cap64, *crr64;
     double omega64, omw64;
-    // FP32 tail only: floats of dynamic shared memory holding x and b of every tail level
-    // (0 = the tail works on the global arrays)
+    // FP32 tail only: floats of dynamic shared memory holding x and b of every tail level (at
+    // sm_x, sm_b), the residual of one (sm_r) and the tail levels' tables (sm_tab, copied from
+    // `tab`); 0 = the tail works on the global arrays
     int sm_floats;
+    int sm_x[kMaxLevels], sm_b[kMaxLevels], sm_r, sm_tab;
+    const T *tab;
     // host abort flag of the context (pmg_set_abort; mapped host memory), or nullptr
     const volatile int *abort;
 };

@@ -845,11 +845,23 @@ int Ctx::upload_tail32(int maxit, double omega, double tol)
     // whose tails share one launch)
     D.sm_floats = 0;
     if (deep_tail) {
-        long long fl = 0;
+        long long fl = 0, largest = 0;
+        auto room = [&](long long n) {
+            const long long o = fl;
+            fl += (n + 3) & ~3LL;
+            return (int)o;
+        };
         for (int l = tail32_l0; l <= nl; ++l) {
             const long long tot = (long long)(lv[l].n[0] + 2) * (lv[l].n[1] + 2) * (lv[l].n[2] + 2);
-            fl += 2 * ((tot + 3) & ~3LL);
+            D.sm_x[l] = room(tot);
+            D.sm_b[l] = room(tot);
+            if (l < nl) largest = std::max(largest, tot);
         }
+        D.sm_r = room(largest);
+        // the tables of levels tail32_l0 .. nl are the end of the table blob
+        D.tab = m->K[tail32_l0].cxm;
+        D.sm_tab = (int)fl;
+        fl += (m->tables + m->tables_host.size()) - D.tab;
         if (fl * (long long)sizeof(float) <= kTail32SmemBytes) D.sm_floats = (int)fl;
     }
     tail32_smem = D.sm_floats * (int)sizeof(float);

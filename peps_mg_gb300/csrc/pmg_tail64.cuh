@@ -6,6 +6,7 @@
 #pragma once
 
 #include "pmg_common.cuh"
+#include "pmg_mul64.cuh"
 
 namespace pmg {
 namespace {
@@ -234,15 +235,18 @@ __device__ __forceinline__ double warp_sum_f64(double v)
 // sqrt(rn / r0) <= tol is decided by integer comparison with tol^2 r0 unless rn lies within
 // 2^-40 of it, where it is evaluated as written.
 //
-// REF: the reference's operation order, bit for bit (the division by quot_f64's rule).
+// REF: the reference's operation order, bit for bit (the level's mul64 flag must be set).  The
+// sweeps multiply on the FP64 unit: a lone warp is bound by fetching its instructions, and the
+// integer products' forty each made an iteration at 4^3 cells 1.9 us instead of 1.4.  INT_NORM
+// (levels of more than 128 cells, where the unit is shared by many warps) takes the norm's
+// products to the integer pipe.
 // Otherwise (the FP32 cycle's coarsest level of at most 64 cells): the neighbour sum as a
 // tree of FMAs and x = (omega/c0)(b - t) + (1-omega) x, for the shorter chain.
 //
-// Measured (2.07 GHz, whole V-cycle solves): coarsest level 7 x 5 x 3, 36 iterations, the
-// 224 x 160 x 96 mixed solve 5.29 -> 3.00 ms; 8 x 6 x 4, about 52 iterations, the 256 x 192 x
-// 128 mixed solve from host arrays 14.9 -> 8.2 ms; 4^3, 34 iterations, the 64^3 FP64 solve
-// 6.96 -> 5.58 ms (before: one warp, or a 64-thread block with both phases in turn and an
-// IEEE division per update).
+// Measured per iteration (one warp before, or a 64-thread block with both phases in turn and
+// an IEEE division per update): FMA form 2^3 cells 1.0 us and 4^3 1.15 us (4.6 us before);
+// REF 2^3 1.35 us, 4^3 1.4 us, 7 x 5 x 3 1.8 us (about 9 before), 8 x 6 x 4 2.2 us (about 14),
+// 8^3 4.8 us.
 // ---------------------------------------------------------------------------------------
 __device__ __forceinline__ void bar_named(int id, int threads)
 {
@@ -252,7 +256,7 @@ __device__ __forceinline__ void bar_named(int id, int threads)
 // cs: five shared arrays of the level's (nx+2)(ny+2)(nz+2) layout; cs[1] holds b (ghosts
 // zero), the others are scratch.  All threads of the block call it (at least chip_threads of
 // them).  Returns the iteration counter; *xsel = the array that holds the solution.
-template <bool REF>
+template <bool REF, bool INT_NORM>
 __device__ int coarse_rbgs_chip(const LevelK<double> &L, double (*cs)[kChipCoarseMax], int maxit, double tol,
                                 double omega, double omw, const volatile int *abort, int *xsel)
 {
@@ -292,15 +296,15 @@ __device__ int coarse_rbgs_chip(const LevelK<double> &L, double (*cs)[kChipCoars
         int p[2];
         bool has[2];
         double cxm[2], cxp[2], c0[2], y[2], b[2];
-        const double cym = slot ? L.cym[j] : 0.0, cyp = slot ? L.cyp[j] : 0.0;
-        const double czm = slot ? L.czm[k] : 0.0, czp = slot ? L.czp[k] : 0.0;
+        const double cym = L.cym[slot ? j : 1], cyp = L.cyp[slot ? j : 1];
+        const double czm = L.czm[slot ? k : 1], czp = L.czp[slot ? k : 1];
 #pragma unroll
         for (int c = 0; c < 2; ++c) {      // first colour: i + j + k odd (src/rbgs_poisson_matrix.f90:242)
             const int i = 2 * t + 1 + ((j + k + c) & 1);
             has[c] = slot && i <= nx;
             p[c] = has[c] ? i + sy * j + sz * k : 1 + sy + sz;
-            cxm[c] = has[c] ? L.cxm[i] : 0.0;
-            cxp[c] = has[c] ? L.cxp[i] : 0.0;
+            cxm[c] = L.cxm[has[c] ? i : 1];
+            cxp[c] = L.cxp[has[c] ? i : 1];
             c0[c] = cs[3][p[c]];
             y[c] = cs[4][p[c]];
             b[c] = cs[1][p[c]];
@@ -318,9 +322,9 @@ __device__ int coarse_rbgs_chip(const LevelK<double> &L, double (*cs)[kChipCoars
                 s = __dadd_rn(s, __dmul_rn(czp, nb[q + sz]));
                 const double d = __dsub_rn(b[c], s);
                 if (omega1)
-                    v = add_zero_times_f64(quot_f64(d, c0[c], y[c]), own[q]);
+                    v = add_zero_times_f64(quot64_dp(d, c0[c], y[c]), own[q]);
                 else
-                    v = __dadd_rn(quot_f64(__dmul_rn(omega, d), c0[c], y[c]), __dmul_rn(omw, own[q]));
+                    v = __dadd_rn(quot64_dp(__dmul_rn(omega, d), c0[c], y[c]), __dmul_rn(omw, own[q]));
             } else {
                 const double tx = fma(cxp[c], nb[q + 1], __dmul_rn(cxm[c], nb[q - 1]));
                 const double ty = fma(cyp, nb[q + sy], __dmul_rn(cym, nb[q - sy]));
@@ -345,24 +349,34 @@ __device__ int coarse_rbgs_chip(const LevelK<double> &L, double (*cs)[kChipCoars
     } else if (tid < nthr) {
         // ---- norms ----
         const int rt = tid - ro.P, lane = tid & 31, warp = rt >> 5, nw = ro.R >> 5;
+        const int i0 = rt % nx + 1, j0 = rt / nx % ny + 1, k0 = rt / nx / ny + 1;
         auto squares = [&](const double *x) {
             double acc = 0.0;
             for (int u = 0; u < ro.NN; ++u) {
                 const int q = rt + u * ro.R;
                 if (q >= n) break;
-                const int i = q % nx + 1, r2 = q / nx, j = r2 % ny + 1, k = r2 / ny + 1;
+                int i = i0, j = j0, k = k0;
+                if (u > 0) {
+                    const int r2 = q / nx;
+                    i = q - r2 * nx + 1;
+                    j = r2 % ny + 1;
+                    k = r2 / ny + 1;
+                }
                 const int c = i + sy * j + sz * k;
                 double r;
                 if (REF) {
-                    r = __dmul_rn(cs[3][c], x[c]);
-                    r = __dadd_rn(r, __dmul_rn(L.cxm[i], x[c - 1]));
-                    r = __dadd_rn(r, __dmul_rn(L.cxp[i], x[c + 1]));
-                    r = __dadd_rn(r, __dmul_rn(L.cym[j], x[c - sy]));
-                    r = __dadd_rn(r, __dmul_rn(L.cyp[j], x[c + sy]));
-                    r = __dadd_rn(r, __dmul_rn(L.czm[k], x[c - sz]));
-                    r = __dadd_rn(r, __dmul_rn(L.czp[k], x[c + sz]));
+                    auto term = [](double f, double v) {
+                        return INT_NORM ? mul64(mul64_factor(f), v) : __dmul_rn(f, v);
+                    };
+                    r = term(cs[3][c], x[c]);
+                    r = __dadd_rn(r, term(L.cxm[i], x[c - 1]));
+                    r = __dadd_rn(r, term(L.cxp[i], x[c + 1]));
+                    r = __dadd_rn(r, term(L.cym[j], x[c - sy]));
+                    r = __dadd_rn(r, term(L.cyp[j], x[c + sy]));
+                    r = __dadd_rn(r, term(L.czm[k], x[c - sz]));
+                    r = __dadd_rn(r, term(L.czp[k], x[c + sz]));
                     r = __dsub_rn(cs[1][c], r);
-                    acc = __dadd_rn(acc, __dmul_rn(r, r));
+                    acc = fma(r, r, acc);
                 } else {
                     const double tx = fma(L.cxp[i], x[c + 1], __dmul_rn(L.cxm[i], x[c - 1]));
                     const double ty = fma(L.cyp[j], x[c + sy], __dmul_rn(L.cym[j], x[c - sy]));

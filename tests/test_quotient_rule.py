@@ -1,4 +1,4 @@
-"""The FP64 path's division by the diagonal (quot_f64 in pmg_common.cuh: a product with the
+"""The FP64 path's division by the diagonal (quot64 in pmg_mul64.cuh: a product with the
 rounded reciprocal and two FMAs) against the correctly rounded quotient, in exact rational
 arithmetic: random operands, and operands whose quotient lies as close to a rounding boundary
 as a quotient can, including divisors whose reciprocal does (which the kernel's table rejects).
