@@ -779,7 +779,15 @@ int Ctx::build_mixed()
                       rb32_fused_layout_ok(f, m->e[1][l], m->b[l]);
         m->rows[l] = rows;
         m->planes[l] = planes;
-        if (m->fused[l] && use_tma) PMG_TRY_M(rb32_tma_setup(&m->tma[l], f, base, rows, planes));
+        // the TMA-fed kernels divide by a diagonal in the normal range (div_normal)
+        bool normal = true;
+        const double *coef[6] = {k.cxm, k.cxp, k.cym, k.cyp, k.czm, k.czp};
+        for (int a = 0; a < 6; ++a)
+            for (int i = 1; i <= lv[l].n[a / 2]; ++i) {
+                const float v = m->tables_host[(size_t)(coef[a] - d_tables) + i];
+                normal = normal && v > 0x1p-100f && v < 0x1p100f;
+            }
+        if (m->fused[l] && use_tma && normal) PMG_TRY_M(rb32_tma_setup(&m->tma[l], f, base, rows, planes));
     }
     for (int l = 0; l < nl; ++l) {
         const XferK<double> &x = X[l];

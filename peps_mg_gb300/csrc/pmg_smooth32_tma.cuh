@@ -36,6 +36,8 @@
 
 namespace pmg {
 
+extern __shared__ unsigned char rbt_smem_raw[];   // the TMA-fed kernels' dynamic shared memory
+
 constexpr int RBT_TX = 60;       // tile columns (same as the register-window kernel)
 constexpr int RBT_W = 64;        // stage row width in floats
 constexpr int RBT_NS = 8;        // stages
@@ -72,18 +74,18 @@ __device__ __forceinline__ void mbar_init(unsigned long long *bar, unsigned coun
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count) : "memory");
 }
 
-__device__ __forceinline__ void mbar_expect_tx(unsigned long long *bar, unsigned bytes)
+__device__ __forceinline__ void mbar_expect_tx(unsigned bar, unsigned bytes)
 {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes)
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
                  : "memory");
 }
 
-__device__ __forceinline__ void mbar_arrive(unsigned long long *bar)
+__device__ __forceinline__ void mbar_arrive(unsigned bar)
 {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
-__device__ __forceinline__ bool mbar_try_wait(unsigned long long *bar, unsigned parity)
+__device__ __forceinline__ bool mbar_try_wait(unsigned bar, unsigned parity)
 {
     unsigned ok;
     asm volatile(
@@ -91,9 +93,14 @@ __device__ __forceinline__ bool mbar_try_wait(unsigned long long *bar, unsigned 
         "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(ok)
-        : "r"(smem_addr(bar)), "r"(parity)
+        : "r"(bar), "r"(parity)
         : "memory");
     return ok != 0;
+}
+
+__device__ __forceinline__ bool mbar_try_wait(unsigned long long *bar, unsigned parity)
+{
+    return mbar_try_wait(smem_addr(bar), parity);
 }
 
 // Waits for the given phase parity; gives up after about one second of clock cycles.
@@ -116,32 +123,43 @@ constexpr long long kStallWaitCycles = 1LL << 13;
 // failure.  The limit is a template constant: a limit read at run time costs the
 // production kernels' sweep loop registers (spills) around this call.
 template <long long LIMIT>
-static __device__ __noinline__ bool mbar_wait_slow(unsigned long long *bar, unsigned parity, volatile int *abort_flag)
+static __device__ __noinline__ bool mbar_wait_slow(unsigned bar, unsigned parity, unsigned abort_flag)
 {
     const long long t0 = clock64();
     while (!mbar_try_wait(bar, parity)) {
-        if (*abort_flag) return false;
+        int raised;
+        asm volatile("ld.volatile.shared.s32 %0, [%1];" : "=r"(raised) : "r"(abort_flag) : "memory");
+        if (raised) return false;
         if (clock64() - t0 > LIMIT) {
-            *abort_flag = 1;
+            asm volatile("st.volatile.shared.s32 [%0], %1;" ::"r"(abort_flag), "r"(1) : "memory");
             return false;
         }
     }
     return true;
 }
 
-__device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, unsigned long long *bar, int x, int y,
-                                            int z)
+__device__ __forceinline__ void tma_load_3d(unsigned dst, const CUtensorMap *map, unsigned bar, int x, int y, int z)
 {
     asm volatile(
         "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], "
-        "[%5];" ::"r"(smem_addr(dst)),
-        "l"(reinterpret_cast<unsigned long long>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_addr(bar))
+        "[%5];" ::"r"(dst),
+        "l"(reinterpret_cast<unsigned long long>(map)), "r"(x), "r"(y), "r"(z), "r"(bar)
         : "memory");
 }
 
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 __device__ __forceinline__ void fence_mbar_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
+
+// a / d as __fdividef forms it (a times the approximate reciprocal), without its scaling for
+// a d outside the normal range (the host keeps such levels off these kernels): 512^3, 14-row
+// tiles, 313 -> 306 us per iteration, the same bits.
+__device__ __forceinline__ float div_normal(float a, float d)
+{
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+    return __fmul_rn(a, r);
+}
 
 template <int Q>
 __device__ __forceinline__ float cq(const float2 &v) { return Q ? v.y : v.x; }
@@ -217,22 +235,22 @@ struct RbtProducer {
         load_item(src);
     }
     // issue every slot up to and including `limit`
-    __device__ __forceinline__ void issue_upto(int limit, const Src &src, unsigned char *smem, unsigned long long *bars)
+    __device__ __forceinline__ void issue_upto(int limit, const Src &src, unsigned sb)
     {
         using S = RbtShape<TY>;
         if (src.stall()) return;   // self-test: nothing is issued, every wait runs out
         while (slot <= limit && src.valid(it)) {
             const int s = slot % RBT_NS;
-            unsigned char *st = smem + s * S::STAGE;
+            const unsigned st = sb + s * S::STAGE, bar = sb + RBT_NS * S::STAGE + 8 * s;
             const bool with_b = q >= k0 - 1 && q <= k1 + 1;
             const unsigned bytes = (ZERO_IN ? 0u : (unsigned)S::EBYTES) + (with_b ? (unsigned)S::BBYTES : 0u);
             const int x = RBT_DATA_OFF + RBT_TX * bx - 1;      // column of cell i0 - 2
             if (bytes) {
-                rbtdetail::mbar_expect_tx(&bars[s], bytes);
-                if (!ZERO_IN) rbtdetail::tma_load_3d(st, me, &bars[s], x, TY * by, q + 1);
-                if (with_b) rbtdetail::tma_load_3d(st + S::EBYTES, mb, &bars[s], x, TY * by + 1, q + 1);
+                rbtdetail::mbar_expect_tx(bar, bytes);
+                if (!ZERO_IN) rbtdetail::tma_load_3d(st, me, bar, x, TY * by, q + 1);
+                if (with_b) rbtdetail::tma_load_3d(st + S::EBYTES, mb, bar, x, TY * by + 1, q + 1);
             } else {
-                rbtdetail::mbar_arrive(&bars[s]);
+                rbtdetail::mbar_arrive(bar);
             }
             ++slot;
             if (++q > k1 + 2) {
@@ -246,22 +264,32 @@ struct RbtProducer {
 template <int TY, bool ZERO_IN, bool OMEGA1>
 struct RbtItem {
     using S = RbtShape<TY>;
+    // FREE: every lane forms its updates and drops the ones its cells do not take, instead of
+    // branching around them.  Measured per iteration at 512^3: 10-row tiles 371 -> 343 us, 6-row
+    // ones 375 -> 345 (and the 128-box batch 44.7 -> 42.9 ms); at 80 registers a thread (14 and
+    // 22 rows) the wider live ranges cost more than the branches: 306 -> 340, 314 -> 332 us.
+    static constexpr bool FREE = TY <= 10;
     static_assert((RBT_NS & (RBT_NS - 1)) == 0, "stage count must be a power of two");
-    unsigned char *smem;
-    unsigned long long *bars;
-    volatile int *abort_flag;
+    // shared addresses are 32-bit and relative to one base: the stages, then the mbarriers,
+    // then the abort flag; b's pair lies OB bytes behind e's in a stage.  (The sweep loop is
+    // short of registers: every pointer pair it does not hold is a spill less.)
+    static constexpr unsigned BARS = RBT_NS * S::STAGE, ABORT = BARS + 8 * RBT_NS, OB = S::EBYTES - RBT_W * 4;
+    unsigned sb;                       // shared base
     const float *czm_t, *czp_t;
-    int nz, k0, k1, cbase;
-    int oe, ob;                        // byte offsets in a stage of row a's own e pair and b pair
-    bool nA[2], nB[2];                 // rows a / b: cell 0 / 1 of the pair takes a first-colour update
-    bool stA, stB, st_full;            // rows a / b are stored; the pair is stored whole
-    float *pwA;                        // e_out at row a, plane 0 (row b at + sy)
+    int nz, k0, k1;
+    int slot0;                         // slot of plane t less t
+    unsigned oe;                       // offset in shared memory, in stage 0, of row a's own e pair
+    // one register for the lane's conditions: bits 0 / 1 row a's cell 0 / 1 takes a first-colour
+    // update, 2 / 3 row b's; 4 / 5 row a / b is stored, 6 the pair is stored whole
+    unsigned flags;
+    float *pw;                         // e_out at row a of the plane the next step stores (row b at + sy)
     int sy;
     long long sz;
     float omega, omw;
     float cxm[2], cxp[2];
     float dA[2], dB[2];                // x-part + y-part of -c0, rows a and b
     float cymA, cypA, cymB, cypB;
+    __device__ __forceinline__ bool flag(int n) const { return flags & (1u << n); }
     float2 EA[4], EB[4], BA[2], BB[2];
     float czm_n, czp_n;                // z coefficients of the next plane (prefetched)
     bool fail;
@@ -273,25 +301,26 @@ struct RbtItem {
     template <bool STALL>
     __device__ __forceinline__ void wait(int slot)
     {
-        unsigned long long *bar = &bars[slot & (RBT_NS - 1)];
+        const unsigned bar = sb + BARS + 8u * (unsigned)(slot & (RBT_NS - 1));
         const unsigned par = (unsigned)(slot / RBT_NS) & 1u;
         constexpr long long lim = STALL ? rbtdetail::kStallWaitCycles : rbtdetail::kWaitCycles;
-        if (!rbtdetail::mbar_try_wait(bar, par) && !rbtdetail::mbar_wait_slow<lim>(bar, par, abort_flag)) fail = true;
+        if (!rbtdetail::mbar_try_wait(bar, par) && !rbtdetail::mbar_wait_slow<lim>(bar, par, sb + ABORT)) fail = true;
     }
-    __device__ __forceinline__ float2 lds2(unsigned off) const
+    // a: offset in the CTA's dynamic shared memory
+    __device__ __forceinline__ static float2 lds2(unsigned a)
     {
-        return *reinterpret_cast<const float2 *>(smem + off);
+        return *reinterpret_cast<const float2 *>(rbt_smem_raw + a);
     }
-    __device__ __forceinline__ float lds(unsigned off) const { return *reinterpret_cast<const float *>(smem + off); }
-    __device__ __forceinline__ void sts2(unsigned off, float2 v) const
+    __device__ __forceinline__ static float lds(unsigned a) { return *reinterpret_cast<const float *>(rbt_smem_raw + a); }
+    __device__ __forceinline__ static void sts2(unsigned a, float2 v)
     {
-        *reinterpret_cast<float2 *>(smem + off) = v;
+        *reinterpret_cast<float2 *>(rbt_smem_raw + a) = v;
     }
     // first- or second-colour update of one cell: s = off-diagonal sum, d = -c0
     __device__ __forceinline__ float upd(float old, float bb, float s, float d) const
     {
-        if (OMEGA1) return __fdividef(s - bb, d);
-        return fmaf(omw, old, __fdividef(omega * (s - bb), d));
+        if (OMEGA1) return rbtdetail::div_normal(s - bb, d);
+        return fmaf(omw, old, rbtdetail::div_normal(omega * (s - bb), d));
     }
     template <bool CHECKED>
     __device__ __forceinline__ void load_cz(int k)
@@ -313,15 +342,15 @@ struct RbtItem {
         constexpr int im2 = P % 4, im1 = (P + 1) % 4, i00 = (P + 2) % 4, ip1 = (P + 3) % 4;
         constexpr int bm1 = P % 2, b00 = (P + 1) % 2;
         constexpr int QB = 1 - Q;
-        const int cs = cbase + (t - k0 + 2);      // slot of plane t
-        const unsigned s0 = stage_off(cs), sp = stage_off(cs + 1), sm = stage_off(cs - 1);
+        const int cs = slot0 + t;      // slot of plane t
+        const unsigned s0 = oe + stage_off(cs), sp = oe + stage_off(cs + 1), sm = oe + stage_off(cs - 1);
         wait<Src::kStall>(cs + 1);
         if (!ZERO_IN) {
-            EA[ip1] = lds2(sp + oe);
-            EB[ip1] = lds2(sp + oe + RBT_W * 4);
+            EA[ip1] = lds2(sp);
+            EB[ip1] = lds2(sp + RBT_W * 4);
         }
-        BA[b00] = lds2(s0 + ob);
-        BB[b00] = lds2(s0 + ob + RBT_W * 4);
+        BA[b00] = lds2(s0 + OB);
+        BB[b00] = lds2(s0 + OB + RBT_W * 4);
         // z coefficients (czm, czp, czm + czp) of plane t-1 in cz[0..2], of plane t in
         // cz[3..5]; plane t+1 is prefetched
         cz[0] = cz[3];
@@ -334,49 +363,70 @@ struct RbtItem {
         const bool plane_in = !CHECKED || (t >= 1 && t <= nz);
         if (ZERO_IN) {
             // every neighbour of a first-colour cell still holds the zero input
-            const float vA = nA[Q] && plane_in ? upd(0.f, cq<Q>(BA[b00]), 0.f, dA[Q] + cz[5]) : 0.f;
-            const float vB = nB[QB] && plane_in ? upd(0.f, cq<QB>(BB[b00]), 0.f, dB[QB] + cz[5]) : 0.f;
+            const float vA = flag(Q) && plane_in ? upd(0.f, cq<Q>(BA[b00]), 0.f, dA[Q] + cz[5]) : 0.f;
+            const float vB = flag(2 + QB) && plane_in ? upd(0.f, cq<QB>(BB[b00]), 0.f, dB[QB] + cz[5]) : 0.f;
             EA[i00] = Q ? make_float2(0.f, vA) : make_float2(vA, 0.f);
             EB[i00] = QB ? make_float2(0.f, vB) : make_float2(vB, 0.f);
-            sts2(s0 + oe, EA[i00]);
-            sts2(s0 + oe + RBT_W * 4, EB[i00]);
+            sts2(s0, EA[i00]);
+            sts2(s0 + RBT_W * 4, EB[i00]);
         } else {
             const float upA = __shfl_up_sync(0xffffffffu, EA[i00].y, 1);
             const float dnA = __shfl_down_sync(0xffffffffu, EA[i00].x, 1);
             const float upB = __shfl_up_sync(0xffffffffu, EB[i00].y, 1);
             const float dnB = __shfl_down_sync(0xffffffffu, EB[i00].x, 1);
             // row a, cell Q: y-neighbours = the stage row below and row b (old values)
-            const float yA = ZERO_IN ? 0.f : lds(s0 + oe - RBT_W * 4 + 4 * Q);
-            const float yB = ZERO_IN ? 0.f : lds(s0 + oe + 2 * RBT_W * 4 + 4 * QB);
-            float vA = 0.f, vB = 0.f;
-            if (nA[Q] && plane_in) {
-                float s = cxm[Q] * (Q ? EA[i00].x : upA);
-                s = fmaf(cxp[Q], Q ? dnA : EA[i00].y, s);
-                s = fmaf(cymA, yA, s);
-                s = fmaf(cypA, cq<Q>(EB[i00]), s);
-                s = fmaf(cz[3], cq<Q>(EA[im1]), s);
-                s = fmaf(cz[4], cq<Q>(EA[ip1]), s);
-                vA = upd(cq<Q>(EA[i00]), cq<Q>(BA[b00]), s, dA[Q] + cz[5]);
+            const float yA = ZERO_IN ? 0.f : lds(s0 - RBT_W * 4 + 4 * Q);
+            const float yB = ZERO_IN ? 0.f : lds(s0 + 2 * RBT_W * 4 + 4 * QB);
+            // every lane forms its update and the lanes whose cell takes none drop it (their
+            // coefficients are zero): branches around the updates cost more than they skip
+            if (FREE) {
+                float t = cxm[Q] * (Q ? EA[i00].x : upA);
+                t = fmaf(cxp[Q], Q ? dnA : EA[i00].y, t);
+                t = fmaf(cymA, yA, t);
+                t = fmaf(cypA, cq<Q>(EB[i00]), t);
+                t = fmaf(cz[3], cq<Q>(EA[im1]), t);
+                t = fmaf(cz[4], cq<Q>(EA[ip1]), t);
+                const float vA = upd(cq<Q>(EA[i00]), cq<Q>(BA[b00]), t, dA[Q] + cz[5]);
+                t = cxm[QB] * (QB ? EB[i00].x : upB);
+                t = fmaf(cxp[QB], QB ? dnB : EB[i00].y, t);
+                t = fmaf(cymB, cq<QB>(EA[i00]), t);
+                t = fmaf(cypB, yB, t);
+                t = fmaf(cz[3], cq<QB>(EB[im1]), t);
+                t = fmaf(cz[4], cq<QB>(EB[ip1]), t);
+                const float vB = upd(cq<QB>(EB[i00]), cq<QB>(BB[b00]), t, dB[QB] + cz[5]);
+                sq<Q>(EA[i00], flag(Q) && plane_in ? vA : cq<Q>(EA[i00]));
+                sq<QB>(EB[i00], flag(2 + QB) && plane_in ? vB : cq<QB>(EB[i00]));
+            } else {
+                float vA = 0.f, vB = 0.f;
+                if (flag(Q) && plane_in) {
+                    float s = cxm[Q] * (Q ? EA[i00].x : upA);
+                    s = fmaf(cxp[Q], Q ? dnA : EA[i00].y, s);
+                    s = fmaf(cymA, yA, s);
+                    s = fmaf(cypA, cq<Q>(EB[i00]), s);
+                    s = fmaf(cz[3], cq<Q>(EA[im1]), s);
+                    s = fmaf(cz[4], cq<Q>(EA[ip1]), s);
+                    vA = upd(cq<Q>(EA[i00]), cq<Q>(BA[b00]), s, dA[Q] + cz[5]);
+                }
+                if (flag(2 + QB) && plane_in) {
+                    float s = cxm[QB] * (QB ? EB[i00].x : upB);
+                    s = fmaf(cxp[QB], QB ? dnB : EB[i00].y, s);
+                    s = fmaf(cymB, cq<QB>(EA[i00]), s);
+                    s = fmaf(cypB, yB, s);
+                    s = fmaf(cz[3], cq<QB>(EB[im1]), s);
+                    s = fmaf(cz[4], cq<QB>(EB[ip1]), s);
+                    vB = upd(cq<QB>(EB[i00]), cq<QB>(BB[b00]), s, dB[QB] + cz[5]);
+                }
+                if (flag(Q) && plane_in) sq<Q>(EA[i00], vA);
+                if (flag(2 + QB) && plane_in) sq<QB>(EB[i00], vB);
             }
-            if (nB[QB] && plane_in) {
-                float s = cxm[QB] * (QB ? EB[i00].x : upB);
-                s = fmaf(cxp[QB], QB ? dnB : EB[i00].y, s);
-                s = fmaf(cymB, cq<QB>(EA[i00]), s);
-                s = fmaf(cypB, yB, s);
-                s = fmaf(cz[3], cq<QB>(EB[im1]), s);
-                s = fmaf(cz[4], cq<QB>(EB[ip1]), s);
-                vB = upd(cq<QB>(EB[i00]), cq<QB>(BB[b00]), s, dB[QB] + cz[5]);
-            }
-            if (nA[Q] && plane_in) sq<Q>(EA[i00], vA);
-            if (nB[QB] && plane_in) sq<QB>(EB[i00], vB);
             // whole pairs: with e_in = 0 the stage holds no copied plane, and cells that are
             // not updated (ghosts, cells beyond the grid) must read as zero there
-            sts2(s0 + oe, EA[i00]);
-            sts2(s0 + oe + RBT_W * 4, EB[i00]);
+            sts2(s0, EA[i00]);
+            sts2(s0 + RBT_W * 4, EB[i00]);
         }
         fence_proxy_async();
         __syncthreads();
-        if (threadIdx.x == 0) prod->issue_upto(cs - 2 + RBT_NS, src, smem, bars);
+        if (threadIdx.x == 0) prod->issue_upto(cs - 2 + RBT_NS, src, sb);
         if (!CHECKED || (t - 1 >= k0 && t - 1 <= k1)) {
             const float upA = __shfl_up_sync(0xffffffffu, EA[im1].y, 1);
             const float dnA = __shfl_down_sync(0xffffffffu, EA[im1].x, 1);
@@ -384,42 +434,63 @@ struct RbtItem {
             const float dnB = __shfl_down_sync(0xffffffffu, EB[im1].x, 1);
             // row a, cell Q: y-neighbours = the stage row below (first colour, plane t-1)
             // and row b's updated first-colour cell; row b, cell 1-Q: row a and the row above
-            const float yA = lds(sm + oe - RBT_W * 4 + 4 * Q);
-            const float yB = lds(sm + oe + 2 * RBT_W * 4 + 4 * QB);
-            float *gA = pwA + sz * (t - 1);
-            if (stA && (Q == 0 || st_full)) {
-                float s = cxm[Q] * (Q ? EA[im1].x : upA);
-                s = fmaf(cxp[Q], Q ? dnA : EA[im1].y, s);
-                s = fmaf(cymA, yA, s);
-                s = fmaf(cypA, cq<Q>(EB[im1]), s);
-                s = fmaf(cz[0], cq<Q>(EA[im2]), s);
-                s = fmaf(cz[1], cq<Q>(EA[i00]), s);
-                const float v = upd(cq<Q>(EA[im1]), cq<Q>(BA[bm1]), s, dA[Q] + cz[2]);
-                sq<Q>(EA[im1], v);
+            const float yA = lds(sm - RBT_W * 4 + 4 * Q);
+            const float yB = lds(sm + 2 * RBT_W * 4 + 4 * QB);
+            float *gA = pw;
+            if (FREE) {
+                float t = cxm[Q] * (Q ? EA[im1].x : upA);
+                t = fmaf(cxp[Q], Q ? dnA : EA[im1].y, t);
+                t = fmaf(cymA, yA, t);
+                t = fmaf(cypA, cq<Q>(EB[im1]), t);
+                t = fmaf(cz[0], cq<Q>(EA[im2]), t);
+                t = fmaf(cz[1], cq<Q>(EA[i00]), t);
+                const float vA = upd(cq<Q>(EA[im1]), cq<Q>(BA[bm1]), t, dA[Q] + cz[2]);
+                t = cxm[QB] * (QB ? EB[im1].x : upB);
+                t = fmaf(cxp[QB], QB ? dnB : EB[im1].y, t);
+                t = fmaf(cymB, cq<QB>(EA[im1]), t);
+                t = fmaf(cypB, yB, t);
+                t = fmaf(cz[0], cq<QB>(EB[im2]), t);
+                t = fmaf(cz[1], cq<QB>(EB[i00]), t);
+                const float vB = upd(cq<QB>(EB[im1]), cq<QB>(BB[bm1]), t, dB[QB] + cz[2]);
+                // (read again by nothing but the stores below)
+                sq<Q>(EA[im1], vA);
+                sq<QB>(EB[im1], vB);
+            } else {
+                if (flag(4) && (Q == 0 || flag(6))) {
+                    float s = cxm[Q] * (Q ? EA[im1].x : upA);
+                    s = fmaf(cxp[Q], Q ? dnA : EA[im1].y, s);
+                    s = fmaf(cymA, yA, s);
+                    s = fmaf(cypA, cq<Q>(EB[im1]), s);
+                    s = fmaf(cz[0], cq<Q>(EA[im2]), s);
+                    s = fmaf(cz[1], cq<Q>(EA[i00]), s);
+                    const float v = upd(cq<Q>(EA[im1]), cq<Q>(BA[bm1]), s, dA[Q] + cz[2]);
+                    sq<Q>(EA[im1], v);
+                }
+                if (flag(5) && (QB == 0 || flag(6))) {
+                    float s = cxm[QB] * (QB ? EB[im1].x : upB);
+                    s = fmaf(cxp[QB], QB ? dnB : EB[im1].y, s);
+                    s = fmaf(cymB, cq<QB>(EA[im1]), s);
+                    s = fmaf(cypB, yB, s);
+                    s = fmaf(cz[0], cq<QB>(EB[im2]), s);
+                    s = fmaf(cz[1], cq<QB>(EB[i00]), s);
+                    const float v = upd(cq<QB>(EB[im1]), cq<QB>(BB[bm1]), s, dB[QB] + cz[2]);
+                    sq<QB>(EB[im1], v);
+                }
             }
-            if (stB && (QB == 0 || st_full)) {
-                float s = cxm[QB] * (QB ? EB[im1].x : upB);
-                s = fmaf(cxp[QB], QB ? dnB : EB[im1].y, s);
-                s = fmaf(cymB, cq<QB>(EA[im1]), s);
-                s = fmaf(cypB, yB, s);
-                s = fmaf(cz[0], cq<QB>(EB[im2]), s);
-                s = fmaf(cz[1], cq<QB>(EB[i00]), s);
-                const float v = upd(cq<QB>(EB[im1]), cq<QB>(BB[bm1]), s, dB[QB] + cz[2]);
-                sq<QB>(EB[im1], v);
-            }
-            if (stA) {
-                if (st_full)
+            if (flag(4)) {
+                if (flag(6))
                     *reinterpret_cast<float2 *>(gA) = EA[im1];
                 else
                     gA[0] = EA[im1].x;
             }
-            if (stB) {
-                if (st_full)
+            if (flag(5)) {
+                if (flag(6))
                     *reinterpret_cast<float2 *>(gA + sy) = EB[im1];
                 else
                     gA[sy] = EB[im1].x;
             }
         }
+        pw += sz;
     }
 
     // Steps t = k0-1 .. k1+1: two checked steps, unchecked steps k0+1 .. k1 unrolled by
@@ -449,8 +520,7 @@ struct RbtItem {
 // One work item.  cbase = slot of plane k0 - 2.  Returns false (uniformly across the
 // CTA) when a wait gave up.
 template <int TY, bool ZERO_IN, bool OMEGA1, class Src>
-__device__ __forceinline__ bool rbt_item(unsigned char *smem, unsigned long long *bars, volatile int *abort_flag,
-                                         const LevelK<float> &L, float *__restrict__ eout, float omega, float omw,
+__device__ __forceinline__ bool rbt_item(unsigned sb, const LevelK<float> &L, float *__restrict__ eout, float omega, float omw,
                                          int bx, int by, int k0, int k1, int cbase, RbtProducer<TY, ZERO_IN, Src> *prod,
                                          const Src &src)
 {
@@ -460,17 +530,14 @@ __device__ __forceinline__ bool rbt_item(unsigned char *smem, unsigned long long
     const int nx = L.nx, ny = L.ny;
     const int a = i0 - 2 + 2 * lane;
     const int ja = j0 - 1 + 2 * w, jb = ja + 1;
-    I.smem = smem;
-    I.bars = bars;
-    I.abort_flag = abort_flag;
+    I.sb = sb;
     I.czm_t = L.czm;
     I.czp_t = L.czp;
     I.nz = L.nz;
     I.k0 = k0;
     I.k1 = k1;
-    I.cbase = cbase;
-    I.oe = ((2 * w + 1) * RBT_W + 2 * lane) * 4;
-    I.ob = S_EB<TY>() + ((2 * w) * RBT_W + 2 * lane) * 4;
+    I.slot0 = cbase + 2 - k0;
+    I.oe = sb - rbtdetail::smem_addr(rbt_smem_raw) + ((2 * w + 1) * RBT_W + 2 * lane) * 4;
     I.sy = L.sy;
     I.sz = L.sz;
     I.omega = omega;
@@ -482,15 +549,12 @@ __device__ __forceinline__ bool rbt_item(unsigned char *smem, unsigned long long
     // a lane updates the first-colour cell of its pair when it is interior and in the tile
     // or the ring cell beside it (lane 0: its second cell, lane 31: its first cell)
     const bool c0ok = in0 && (mid || lane == 31), c1ok = in1 && (mid || lane == 0);
-    I.nA[0] = inA && c0ok;
-    I.nA[1] = inA && c1ok;
-    I.nB[0] = inB && c0ok;
-    I.nB[1] = inB && c1ok;
     const bool col_store = mid && a <= nx;
-    I.stA = col_store && inA && w >= 1;                          // row a of warp 0 is the ring row
-    I.stB = col_store && inB && w <= RbtShape<TY>::WARPS - 2;               // row b of the last warp is the ring row
-    I.st_full = a + 1 <= nx;
-    I.pwA = eout + (long long)a + (long long)L.sy * ja;
+    const bool stA = col_store && inA && w >= 1;                             // row a of warp 0 is the ring row
+    const bool stB = col_store && inB && w <= RbtShape<TY>::WARPS - 2;       // row b of the last warp is the ring row
+    I.flags = (inA && c0ok ? 1u : 0u) | (inA && c1ok ? 2u : 0u) | (inB && c0ok ? 4u : 0u) | (inB && c1ok ? 8u : 0u) |
+              (stA ? 16u : 0u) | (stB ? 32u : 0u) | (a + 1 <= nx ? 64u : 0u);
+    I.pw = eout + (long long)a + (long long)L.sy * ja + L.sz * (k0 - 2);
     I.cymA = inA ? L.cym[ja] : 0.f;
     I.cypA = inA ? L.cyp[ja] : 0.f;
     I.cymB = inB ? L.cym[jb] : 0.f;
@@ -514,11 +578,11 @@ __device__ __forceinline__ bool rbt_item(unsigned char *smem, unsigned long long
     if (ZERO_IN) {
         I.EA[1] = I.EB[1] = I.EA[2] = I.EB[2] = make_float2(0.f, 0.f);
     } else {
-        const unsigned s1 = I.stage_off(cbase), s2 = I.stage_off(cbase + 1);
-        I.EA[1] = I.lds2(s1 + I.oe);
-        I.EB[1] = I.lds2(s1 + I.oe + RBT_W * 4);
-        I.EA[2] = I.lds2(s2 + I.oe);
-        I.EB[2] = I.lds2(s2 + I.oe + RBT_W * 4);
+        const unsigned s1 = I.oe + I.stage_off(cbase), s2 = I.oe + I.stage_off(cbase + 1);
+        I.EA[1] = I.lds2(s1);
+        I.EB[1] = I.lds2(s1 + RBT_W * 4);
+        I.EA[2] = I.lds2(s2);
+        I.EB[2] = I.lds2(s2 + RBT_W * 4);
     }
     I.BA[0] = I.BB[0] = make_float2(0.f, 0.f);
     // the pair's first cell a is odd, so on row a it carries the first colour on plane k
@@ -538,12 +602,12 @@ template <int TY, bool ZERO_IN, bool OMEGA1, class Src, class Per>
 __device__ __forceinline__ void rbt_cta(const Src &src, Per per, float omega, float omw, int *err)
 {
     using S = RbtShape<TY>;
-    extern __shared__ unsigned char rbt_smem_raw[];
     // 128-byte aligned stages (TMA destinations), then the mbarriers, the abort flag and
     // the producer state
     unsigned char *smem = rbt_smem_raw + ((128u - (rbtdetail::smem_addr(rbt_smem_raw) & 127u)) & 127u);
     unsigned long long *bars = reinterpret_cast<unsigned long long *>(smem + RBT_NS * S::STAGE);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(bars + RBT_NS);
+    const unsigned sb = rbtdetail::smem_addr(smem);
     using Prod = RbtProducer<TY, ZERO_IN, Src>;
     static_assert(sizeof(Prod) <= 48, "producer state exceeds its shared-memory slot");
     Prod *prod = reinterpret_cast<Prod *>(bars + RBT_NS + 2);
@@ -555,7 +619,7 @@ __device__ __forceinline__ void rbt_cta(const Src &src, Per per, float omega, fl
     __syncthreads();
     if (threadIdx.x == 0) {
         prod->start(src);
-        prod->issue_upto(RBT_NS - 1, src, smem, bars);
+        prod->issue_upto(RBT_NS - 1, src, sb);
     }
     int cbase = 0;
     for (int it = src.first(); src.valid(it); it = src.next(it)) {
@@ -564,8 +628,7 @@ __device__ __forceinline__ void rbt_cta(const Src &src, Per per, float omega, fl
         const LevelK<float> *L;
         float *eout;
         per(it, L, eout);
-        if (!rbt_item<TY, ZERO_IN, OMEGA1>(smem, bars, abort_flag, *L, eout, omega, omw, bx, by, k0, k1, cbase, prod,
-                                            src)) {
+        if (!rbt_item<TY, ZERO_IN, OMEGA1>(sb, *L, eout, omega, omw, bx, by, k0, k1, cbase, prod, src)) {
             if (threadIdx.x == 0) {
                 atomicOr(err, 1);
                 for (int q = max(0, prod->slot - RBT_NS); q < prod->slot; ++q)
