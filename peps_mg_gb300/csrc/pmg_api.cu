@@ -746,8 +746,9 @@ int Ctx::build(const pmg_config_t *c, cudaStream_t s)
     }
     npart_cap = max_part;
     PMG_CUDA(dev_malloc(&d_partials, npart_cap * sizeof(double)), "scratch allocation");
-    PMG_CUDA(dev_malloc(&d_scal, 16 * sizeof(double)), "scratch allocation");
-    PMG_CUDA(dev_malloc(&d_iscal, 16 * sizeof(int)), "scratch allocation");
+    // scalars and counters in one block, so that one copy fetches a cycle's results
+    PMG_CUDA(dev_malloc(&d_scal, 16 * sizeof(double) + 16 * sizeof(int)), "scratch allocation");
+    d_iscal = reinterpret_cast<int *>(d_scal + 16);
     PMG_CUDA(dev_malloc(&d_cg, sizeof(CgState)), "scratch allocation");
     PMG_CUDA(cudaMemset(d_cg, 0, sizeof(CgState)), "scratch init");
     if (!light) {
@@ -787,7 +788,121 @@ int Ctx::build(const pmg_config_t *c, cudaStream_t s)
         }
         // complete before any other stream (a decomposed solve's) reads the tables
         PMG_CUDA(cudaStreamSynchronize(stream), "diagonal table");
+        PMG_TRY(setup_coop64());
     }
+    return PMG_OK;
+}
+
+// The levels of a plain FP64 cycle that run in one cooperative launch (pmg_coop64.cu): from
+// the first one of at most kCoop64Cells cells on, if every one of them fits mul64's range and
+// the coarsest is solved on chip.
+int Ctx::setup_coop64()
+{
+    const char *env = std::getenv("PEPS_MG_COOP");   // PEPS_MG_COOP=0: the grid kernels on every level
+    if (precision != PMG_FP64 || light || (env && std::strcmp(env, "0") == 0)) return PMG_OK;
+    int dev = 0;
+    PMG_CUDA(cudaGetDevice(&dev), "device");
+    PMG_TRY(coop64_grid(dev, &coop_grid));
+    if (coop_grid == 0) return PMG_OK;
+    PMG_CUDA(dev_malloc(&d_bar, 2 * sizeof(unsigned)), "barrier");
+    PMG_CUDA(cudaMemset(d_bar, 0, 2 * sizeof(unsigned)), "barrier");
+    if (coarse_solver != PMG_COARSE_RBGS || (size_t)coop_grid > npart_cap) return PMG_OK;
+    if (chip_threads(lv[nl].n[0], lv[nl].n[1], lv[nl].n[2]) == 0) return PMG_OK;
+    int l0 = nl + 1;
+    for (int l = nl; l >= 0; --l) {
+        if (!coop64_level_ok(l, kCoop64Cells) || (l < nl && !X[l].mul64)) break;
+        l0 = l;
+    }
+    if (l0 > nl) return PMG_OK;
+    Coop64Desc D;
+    std::memset(&D, 0, sizeof(D));
+    D.l0 = l0;
+    D.nl = nl;
+    // on one CTA: the last levels of at most kCoop64TailCells cells that shared memory holds
+    int lt = nl;
+    long long doubles = 0;
+    auto need = [&](int first) {
+        long long o = 0, largest = 0;
+        for (int l = first; l <= nl; ++l) {
+            const long long t = (long long)lv[l].total;
+            D.sm_x[l] = (int)o;
+            D.sm_b[l] = (int)(o + t);
+            o += 2 * t;
+            if (l < nl) {
+                D.sm_c0[l] = (int)o;
+                D.sm_rc[l] = (int)(o + t);
+                o += 2 * t;
+                largest = std::max(largest, t);
+            }
+        }
+        D.sm_r = (int)o;
+        return o + largest;
+    };
+    while (lt > l0 && (long long)lv[lt - 1].n[0] * lv[lt - 1].n[1] * lv[lt - 1].n[2] <= kCoop64TailCells &&
+           need(lt - 1) * (long long)sizeof(double) <= kCoop64SmemBytes && lt - 1 > 0)
+        --lt;
+    if (lt == 0) return PMG_OK;
+    doubles = need(lt);
+    D.lt = lt;
+    D.sm_doubles = (int)doubles;
+    coop_smem = (int)(doubles * (long long)sizeof(double));
+    if (coop_smem > kCoop64SmemBytes) return PMG_OK;
+    D.coarse_maxit = 1000;   // src/multigrid.f90:1948
+    D.iters_out = d_iscal + 1;
+    D.err = d_iscal + 8;
+    D.partials = d_partials;
+    D.abort = abort_dev;
+    PMG_CUDA(dev_malloc(&d_coop, sizeof(Coop64Desc)), "small levels' descriptor");
+    D.bar = d_bar;
+    for (int l = l0; l <= nl; ++l) D.lv[l] = coop64_level(l);
+    coop_host = new (std::nothrow) Coop64Desc(D);
+    if (!coop_host) return PMG_ENOMEM;
+    coop_l0 = l0;
+    return PMG_OK;
+}
+
+bool Ctx::coop64_level_ok(int l, long long cells) const
+{
+    const int *n = lv[l].n;
+    return (long long)n[0] * n[1] * n[2] <= cells && std::max(n[0], std::max(n[1], n[2])) <= 4096 && K[l].mul64;
+}
+
+Coop64Level Ctx::coop64_level(int l) const
+{
+    Coop64Level V;
+    std::memset(&V, 0, sizeof(V));
+    V.L = K[l];
+    if (l < nl) V.X = X[l];
+    V.x = lv[l].x;
+    V.b = lv[l].b;
+    V.r = lv[l].r;
+    V.c0t = c0t[l];
+    V.dhx = fastdiv_factor((unsigned)(lv[l].n[0] + 1) / 2);
+    V.dnx = fastdiv_factor((unsigned)lv[l].n[0]);
+    V.dny = fastdiv_factor((unsigned)lv[l].n[1]);
+    return V;
+}
+
+// A barrier wait of a cooperative launch that ran out (the caller has synchronised).
+int Ctx::check_coop64()
+{
+    int e = 0;
+    PMG_CUDA(cudaMemcpyAsync(&e, d_iscal + 8, sizeof(int), cudaMemcpyDeviceToHost, stream), "barrier status");
+    PMG_CUDA(cudaStreamSynchronize(stream), "barrier status");
+    if (e == 0) return PMG_OK;
+    cudaMemsetAsync(d_iscal + 8, 0, sizeof(int), stream);
+    set_error("a grid barrier of the small levels' launch gave up");
+    return PMG_ETIMEOUT;
+}
+
+int Ctx::upload_coop64(int maxit, double omega, double tol)
+{
+    Coop64Desc &D = *coop_host;
+    D.maxit = maxit;
+    D.omega = omega;
+    D.omw = 1.0 - omega;
+    D.tol = tol;
+    PMG_CUDA(cudaMemcpyAsync(d_coop, &D, sizeof(D), cudaMemcpyHostToDevice, stream), "small levels' descriptor");
     return PMG_OK;
 }
 
@@ -856,9 +971,11 @@ Ctx::~Ctx()
     for (auto p : c0t) dev_free(p);
     dev_free(d_partials);
     dev_free(d_scal);
-    dev_free(d_iscal);
     dev_free(d_cg);
     if (abort_host) cudaFreeHost(abort_host);
+    dev_free(d_bar);
+    dev_free(d_coop);
+    delete coop_host;
     dev_free(d_fast);
     for (auto p : fast_wdiag_alloc) dev_free(p);
     dev_free(d_cp);
@@ -905,6 +1022,23 @@ int Ctx::solve_residual_norm(double *r, const double *x, const double *b, int sl
     int np = 0;
     PMG_TRY(fast_residual(K[0], fastK[0], launch[0], r, x, b, d_partials, &np, stream));
     return f64_reduce(d_partials, np, d_scal + slot, stream);
+}
+
+// The residual norm, the coarsest solver's iterations and the barrier flag of a cycle.
+int Ctx::fetch_cycle(double *rsd_val, int *coarse_iters)
+{
+    struct {
+        double d[16];
+        int i[16];
+    } h;
+    PMG_CUDA(cudaMemcpyAsync(&h, d_scal, sizeof(h), cudaMemcpyDeviceToHost, stream), "scalar read");
+    PMG_CUDA(cudaStreamSynchronize(stream), "stream sync");
+    *rsd_val = h.d[1];
+    if (coarse_iters) *coarse_iters = h.i[1];
+    if (h.i[8] == 0) return PMG_OK;
+    cudaMemsetAsync(d_iscal + 8, 0, sizeof(int), stream);
+    set_error("a grid barrier of the small levels' launch gave up");
+    return PMG_ETIMEOUT;
 }
 
 int Ctx::fetch_scalars(double *h, int n)
@@ -972,7 +1106,14 @@ int Ctx::vcycle_f64(double *sol, double *rsd, const double *rhs, int maxit, doub
 {
     NvtxRange cycle_range(fast64 ? "fp64-fast V-cycle" : "fp64 V-cycle");
     const double N = (double)K[0].nx * K[0].ny * K[0].nz;
-    const int grid_end = std::min(tail_l0, nl);
+    const bool coop = coop_l0 <= nl;
+    if (coop && coop_l0 == 0) {
+        const int pi = prof.begin(stream);
+        PMG_TRY(coop64_cycle(d_coop, coop_grid, coop_smem, sol, rhs, rsd, d_scal + 1, stream));
+        prof.end(pi, PC_TAIL64, 1, 0.0, stream);
+        return PMG_OK;
+    }
+    const int grid_end = coop ? coop_l0 : std::min(tail_l0, nl);
     // the grid levels' operations: bitwise kernels, or those of the FP64 performance mode
     // (which stores omega/c0: 4 more bytes per updated cell and half-sweep)
     const bool fast = fast64;
@@ -1031,16 +1172,15 @@ int Ctx::vcycle_f64(double *sol, double *rsd, const double *rhs, int maxit, doub
         PMG_TRY(restr(l, L.r, lv[l + 1].b));
     }
     if (coarse_launches > 0) prof.end(pc, PC_COARSE64, coarse_launches, coarse_bytes(true) / coarse_launches, stream);
-    if (tail_l0 <= nl) {
+    const bool tail = coop || tail_l0 <= nl;
+    if (tail) {
         pi = prof.begin(stream);
-        PMG_TRY(f64_tail(d_tail, tail_threads, stream));
+        if (coop)
+            PMG_TRY(coop64_cycle(d_coop, coop_l0 == coop_host->lt ? 1 : coop_grid, coop_smem, nullptr, nullptr,
+                                 nullptr, nullptr, stream));
+        else
+            PMG_TRY(f64_tail(d_tail, tail_threads, stream));
         prof.end(pi, PC_TAIL64, 1, 0.0, stream);
-        if (coarse_iters) {
-            int h = 0;
-            PMG_CUDA(cudaMemcpyAsync(&h, d_iscal + 1, sizeof(int), cudaMemcpyDeviceToHost, stream), "iters");
-            PMG_CUDA(cudaStreamSynchronize(stream), "sync");
-            *coarse_iters = h;
-        }
     } else {
         PMG_TRY(coarse_solve_grid(tol, omega, coarse_iters));
     }
@@ -1097,7 +1237,11 @@ int Ctx::solve_f64(double *sol, double *rsd, const double *rhs, int maxit, doubl
         }
         return PMG_OK;
     }
-    if (tail_l0 <= nl) PMG_TRY(upload_tail(tail_l0, maxit, omega, tol));
+    const bool coop = coop_l0 <= nl;
+    if (coop)
+        PMG_TRY(upload_coop64(maxit, omega, tol));
+    else if (tail_l0 <= nl)
+        PMG_TRY(upload_tail(tail_l0, maxit, omega, tol));
     int cycles = 0, converged = 0;
     double ratio = 0.0;
     for (int cyc = 1; cyc <= n_vcycles; ++cyc) {
@@ -1114,10 +1258,11 @@ int Ctx::solve_f64(double *sol, double *rsd, const double *rhs, int maxit, doubl
         int ci = 0;
         PMG_TRY(vcycle_f64(sol, rsd, rhs, maxit, omega, tol, rep && rep->coarse_iterations ? &ci : nullptr));
         int pr = prof.begin(stream);
-        PMG_TRY(solve_residual_norm(rsd, sol, rhs, 1));  // :1970-1971
+        if (!(coop && coop_l0 == 0)) PMG_TRY(solve_residual_norm(rsd, sol, rhs, 1));  // :1970-1971
         prof.end(pr, PC_RES64, 1, (!fast64 && diag(0) ? 32.0 : 24.0) * (double)K[0].nx * K[0].ny * K[0].nz, stream);
-        PMG_TRY(fetch_scalars(h, 2));
-        const double rsd_val = h[1];
+        double rsd_val = 0.0;
+        const bool tail = coop || tail_l0 <= nl;     // else the cycle has set ci
+        PMG_TRY(fetch_cycle(&rsd_val, tail ? &ci : nullptr));
         ratio = std::sqrt(rsd_val / res0tol);
         cycles = cyc;
         if (rep) {
@@ -1593,6 +1738,10 @@ int pmg_rbgs_iterator(pmg_ctx *ctx, int level, double *x, const double *b, int m
 {
     PMG_TRY(check_ctx_level(ctx, level));
     Ctx &c = ctx->impl;
+    // several half-sweeps of a small level in one launch
+    if (c.coop_grid > 0 && maxiteration >= 2 && c.coop64_level_ok(level, pmg::kCoop64SweepCells))
+        return pmg::coop64_sweeps(c.coop64_level(level), c.coop_grid, x, b, maxiteration, omega, c.d_bar,
+                                  c.d_iscal + 8, c.stream);
     return pmg::f64_rbgs_sweeps(c.K[level], c.launch[level], x, b, maxiteration, omega, c.stream, c.diag(level));
 }
 
@@ -1801,7 +1950,8 @@ int pmg_selftest_wait_timeout(pmg_ctx *ctx, int level)
 int pmg_sync(pmg_ctx *ctx)
 {
     if (!ctx) return PMG_EINVAL;
-    return pmg::cuda_status(cudaStreamSynchronize(ctx->impl.stream), "sync");
+    const int rc = pmg::cuda_status(cudaStreamSynchronize(ctx->impl.stream), "sync");
+    return rc == PMG_OK && ctx->impl.coop_grid > 0 ? ctx->impl.check_coop64() : rc;
 }
 
 const char *pmg_last_error(void) { return pmg::g_last_error.c_str(); }

@@ -623,10 +623,6 @@ struct Tail32Level {
     unsigned dhx, dnx, dny;      // fastdiv's factors of (nx+1)/2, nx and ny
 };
 
-// q / d for q < 2^18 and d <= 2^12, m = fastdiv_factor(d): 2^32/d rounded up, and 0 for d = 1
-__device__ __forceinline__ unsigned fastdiv_factor(unsigned d) { return d > 1 ? 0xffffffffu / d + 1u : 0u; }
-__device__ __forceinline__ int fastdiv(int q, unsigned m) { return m ? (int)__umulhi((unsigned)q, m) : q; }
-
 // f(i, j, k, p) for every interior cell of the level
 template <typename F>
 __device__ __forceinline__ void tail32_cells(const Tail32Level &T, F f)

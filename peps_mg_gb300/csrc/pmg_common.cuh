@@ -53,6 +53,11 @@ __host__ __device__ inline long long lin(int i, int j, int k, int sy, long long 
     return (long long)i + (long long)sy * j + sz * k;
 }
 
+// q / d by a multiplication, for q < 2^18 and d <= 2^12: m = fastdiv_factor(d), 2^32 / d
+// rounded up (0 stands for d = 1)
+__host__ __device__ __forceinline__ unsigned fastdiv_factor(unsigned d) { return d > 1 ? 0xffffffffu / d + 1u : 0u; }
+__device__ __forceinline__ int fastdiv(int q, unsigned m) { return m ? (int)__umulhi((unsigned)q, m) : q; }
+
 // Largest coarsest level (stored values, ghosts included) that the on-chip coarsest-level
 // solvers hold in shared memory (pmg_tail64.cuh).
 constexpr int kChipCoarseMax = 1000;
@@ -222,6 +227,23 @@ __device__ __forceinline__ double restrict_cell_f64(const XferK<double> &X, cons
     s = __dadd_rn(s, __dmul_rn(v122, vf[lin(ip, jz, kz, sy, sz)]));
     s = __dadd_rn(s, __dmul_rn(v222, vf[lin(iz, jz, kz, sy, sz)]));
     return __ddiv_rn(s, vol);
+}
+
+// Coarse index, neighbour and the own and the neighbour's 1-D weight of fine index f along
+// one axis (stride 2: odd f is the low child, even f the high one; stride 1: the high child,
+// src/multigrid.f90:1594-1649).
+__device__ __forceinline__ void side64(int st, int f, const double *pp, const double *pn, int &c, int &nb, double &wa,
+                                       double &wb)
+{
+    if (st == 2) {
+        c = (f + 1) >> 1;
+        nb = (f & 1) ? c - 1 : c + 1;
+        wa = (f & 1) ? pp[f] : pn[f];
+        wb = (f & 1) ? pp[f + 1] : pn[f - 1];
+    } else {
+        c = nb = f;
+        wa = wb = pn[f];
+    }
 }
 
 // One child of a coarse cell in the prolongation (src/multigrid.f90:1676-1754).  The

@@ -1,0 +1,435 @@
+// pmg_coop64.cu -- the small levels of a plain FP64 V-cycle in one cooperative launch.
+//
+// Levels of at most 2^15 cells are bound by latency, not by the FP64 unit: dependent launches
+// start about 6 us apart however little they do, and a V-cycle has eleven per level.  Here one
+// CTA per SM runs the whole part of the V-cycle below the first such level (or all of it, with
+// the residual norm that ends the cycle, where the finest level is that small): the levels of
+// more than 512 cells a phase at a time over all CTAs with a grid barrier between phases (3 us
+// a phase: a cell's chain of instructions behind L2 loads, and the barrier), the rest (where a
+// half-sweep is a microsecond or two on one SM) on the first CTA in shared memory.  Same
+// operations and order per cell as the grid kernels of pmg_f64.cu, so the same bits.  Larger
+// levels keep those: at 64^3 cells a phase here took 8 us, a launch 6.
+// Measured: 64^3 FP64 solve (levels 32^3 to 4^3 here) 4.5 -> 3.15 ms.
+//
+// Data written during the launch is read past L1 (__ldcg): another SM may have written it
+// since.  Barrier waits are bounded (about a second); one that runs out sets the error flag
+// and every CTA leaves.
+//
+// Compiled with --fmad=false.
+#include <cuda_runtime.h>
+
+#include "../../include/peps_mg.h"
+#include "pmg_internal.h"
+#include "pmg_mul64.cuh"
+#include "pmg_tail64.cuh"
+
+namespace pmg {
+
+namespace {
+
+constexpr int kThreads = kTail64Threads;
+constexpr int kManyCells = 8192;   // prolongation by integer products above this many cells
+
+// Where a level's arrays live: global memory written by other SMs during the launch, or this
+// CTA's shared memory.
+struct Far {
+    __device__ __forceinline__ static double ld(const double *p) { return __ldcg(p); }
+};
+struct Near {
+    __device__ __forceinline__ static double ld(const double *p) { return *p; }
+};
+
+// A product and a division of the bitwise arithmetic: on the integer pipe where many warps
+// share the FP64 unit and a cell has many products (the prolongation), else on that unit: with
+// a few warps per SM a phase is one cell's chain of instructions, and the integer products'
+// are the longer one.
+template <bool INT>
+__device__ __forceinline__ double prod(double c, double x)
+{
+    return INT ? mul64(mul64_factor(c), x) : __dmul_rn(c, x);
+}
+template <bool INT>
+__device__ __forceinline__ double quot(double d, double c, double y)
+{
+    return INT ? quot64(d, c, y) : quot64_dp(d, c, y);
+}
+
+// c1 x(i-1) + ... + c6 x(k+1) onto t0 (the residual's c0 x), or from the first product
+template <class M, bool INT, bool DIAG>
+__device__ __forceinline__ double nbsum(const LevelK<double> &L, const double *x, int p, int i, int j, int k,
+                                        double c0)
+{
+    const int sy = L.sy, sz = (int)L.sz;
+    double t;
+    if (DIAG) {
+        t = prod<INT>(c0, M::ld(x + p));
+        t = __dadd_rn(t, prod<INT>(L.cxm[i], M::ld(x + p - 1)));
+    } else {
+        t = prod<INT>(L.cxm[i], M::ld(x + p - 1));
+    }
+    t = __dadd_rn(t, prod<INT>(L.cxp[i], M::ld(x + p + 1)));
+    t = __dadd_rn(t, prod<INT>(L.cym[j], M::ld(x + p - sy)));
+    t = __dadd_rn(t, prod<INT>(L.cyp[j], M::ld(x + p + sy)));
+    t = __dadd_rn(t, prod<INT>(L.czm[k], M::ld(x + p - sz)));
+    t = __dadd_rn(t, prod<INT>(L.czp[k], M::ld(x + p + sz)));
+    return t;
+}
+
+// f(i, j, k, p) for the cells q0, q0 + step, ... of a level
+template <typename F>
+__device__ __forceinline__ void cells(const Coop64Level &V, int q0, int step, F f)
+{
+    const int nx = V.L.nx, ny = V.L.ny, n = nx * ny * V.L.nz, sy = V.L.sy, sz = (int)V.L.sz;
+    for (int q = q0; q < n; q += step) {
+        const int rr = fastdiv(q, V.dnx), kk = fastdiv(rr, V.dny);
+        const int i = q - rr * nx + 1, j = rr - kk * ny + 1, k = kk + 1;
+        f(i, j, k, i + sy * j + sz * k);
+    }
+}
+
+// Half-sweep h of a smoothing step on x: the cells of colour h & 1 (src/rbgs_poisson_matrix.f90
+// :242).  first: x enters as zero and is not read; the other colour's cells are set to it.
+template <class M, bool INT>
+__device__ __forceinline__ void half_sweep(const Coop64Level &V, double *x, const double *b, const double *c0t,
+                                           const double *rc, int h, bool first, double omega, double omw, int q0,
+                                           int step)
+{
+    const LevelK<double> &L = V.L;
+    const bool omega1 = omega == 1.0;
+    auto update = [&](int p, double s, double old) {
+        const double d = __dsub_rn(M::ld(b + p), s);
+        const double c0 = c0t[p], y = rc[p];
+        x[p] = omega1 ? add_zero_times_f64(quot<INT>(d, c0, y), old)
+                      : __dadd_rn(quot<INT>(__dmul_rn(omega, d), c0, y), __dmul_rn(omw, old));
+    };
+    if (first) {
+        cells(V, q0, step, [&](int i, int j, int k, int p) {
+            if ((i + j + k) & 1)
+                update(p, 0.0, 0.0);
+            else
+                x[p] = 0.0;
+        });
+        return;
+    }
+    const int nx = L.nx, ny = L.ny, hx = (nx + 1) / 2, nq = hx * ny * L.nz, sy = L.sy, sz = (int)L.sz;
+    for (int q = q0; q < nq; q += step) {
+        const int rr = fastdiv(q, V.dhx), kk = fastdiv(rr, V.dny);
+        const int j = rr - kk * ny + 1, k = kk + 1;
+        const int i = 2 * (q - rr * hx) + 1 + ((j + k + h) & 1);
+        if (i > nx) continue;
+        const int p = i + sy * j + sz * k;
+        update(p, nbsum<M, INT, false>(L, x, p, i, j, k, 0.0), M::ld(x + p));
+    }
+}
+
+// r = b - A x; the sum of the squares of this thread's cells
+template <class M, bool INT>
+__device__ __forceinline__ double residual(const Coop64Level &V, double *r, const double *x, const double *b,
+                                           const double *c0t, int q0, int step)
+{
+    double acc = 0.0;
+    cells(V, q0, step, [&](int i, int j, int k, int p) {
+        const double v = __dsub_rn(M::ld(b + p), nbsum<M, INT, true>(V.L, x, p, i, j, k, c0t[p]));
+        r[p] = v;
+        acc = __fma_rn(v, v, acc);
+    });
+    return acc;
+}
+
+// restrict_cell_f64 (pmg_common.cuh) on the coarse level C
+template <class M, bool INT>
+__device__ __forceinline__ void restriction(const Coop64Level &C, const XferK<double> &X, const double *r, double *bc,
+                                            int q0, int step)
+{
+    cells(C, q0, step, [&](int i, int j, int k, int p) {
+        const int ip = i * X.stx, iz = ip - (X.stx - 1);
+        const int jp = j * X.sty, jz = jp - (X.sty - 1);
+        const int kp = k * X.stz, kz = kp - (X.stz - 1);
+        const double xz = X.wx[iz], xp = X.wx[ip], yz = X.wy[jz], yp = X.wy[jp], zz = X.wz[kz], zp = X.wz[kp];
+        const double xy[4] = {__dmul_rn(xz, yz), __dmul_rn(xp, yz), __dmul_rn(xz, yp), __dmul_rn(xp, yp)};
+        double vol = 0.0, s = 0.0;
+#pragma unroll 1
+        for (int c = 0; c < 8; ++c) {
+            const double w = __dmul_rn(c & 2 ? (c & 1 ? xy[3] : xy[2]) : (c & 1 ? xy[1] : xy[0]), c < 4 ? zz : zp);
+            const int f = ((c & 1) ? iz : ip) + X.fsy * ((c & 2) ? jz : jp) + (int)X.fsz * ((c & 4) ? kz : kp);
+            const double t = prod<INT>(w, M::ld(r + f));
+            vol = c == 0 ? w : __dadd_rn(vol, w);
+            s = c == 0 ? t : __dadd_rn(s, t);
+        }
+        bc[p] = __ddiv_rn(s, vol);
+    });
+}
+
+// x += P xc (prolong_child_f64) on the fine level F
+template <class M, bool INT>
+__device__ __forceinline__ void prolong_add(const Coop64Level &F, const double *xc, double *x, int q0, int step)
+{
+    const XferK<double> &X = F.X;
+    cells(F, q0, step, [&](int fi, int jf, int kf, int p) {
+        int i, in, j, jn, k, kn;
+        double ax, bx, ay, by, az, bz;
+        side64(X.stx, fi, X.pxp, X.pxn, i, in, ax, bx);
+        side64(X.sty, jf, X.pyp, X.pyn, j, jn, ay, by);
+        side64(X.stz, kf, X.pzp, X.pzn, k, kn, az, bz);
+        const int csy = X.csy, csz = (int)X.csz;
+        // x neighbour, y neighbour, z neighbour as bits 0 .. 2, in the reference's order of terms
+        constexpr int order[8] = {0, 1, 2, 4, 3, 5, 6, 7};
+        double t = 0.0;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int c = order[u];
+            const double w = prod<INT>(__dmul_rn(c & 1 ? bx : ax, c & 2 ? by : ay), c & 4 ? bz : az);
+            const double v = prod<INT>(
+                w, M::ld(xc + (c & 1 ? in : i) + csy * (c & 2 ? jn : j) + csz * (c & 4 ? kn : k)));
+            t = u == 0 ? v : __dadd_rn(t, v);
+        }
+        const double den = prod<INT>(__dmul_rn(X.sx[fi], X.sy[jf]), X.szz[kf]);
+        const double y0 = __dmul_rn(__dmul_rn(X.rx[fi], X.ry[jf]), X.rz[kf]);
+        const double y = __fma_rn(y0, __fma_rn(-den, y0, 1.0), y0);
+        x[p] = __dadd_rn(M::ld(x + p), quot64_near(t, den, y));
+    });
+}
+
+// This thread's first cell: consecutive warps' worth of cells go to consecutive SMs, so that a
+// level of few warps has one on each rather than sixteen on a few.
+__device__ __forceinline__ int spread_start()
+{
+    return (int)(((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32 + (threadIdx.x & 31));
+}
+
+// The grid barrier: an arrival count that thread 0 of each CTA waits on.
+struct GridBarrier {
+    unsigned *ctr;
+    unsigned goal;
+    int *s_fail;
+    __device__ __forceinline__ bool sync()
+    {
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            goal += gridDim.x;
+            __threadfence();
+            atomicAdd(ctr, 1u);
+            const long long t0 = clock64();
+            int spins = 0;
+            unsigned v;
+            do {
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(ctr) : "memory");
+                if (v >= goal) break;
+                if (++spins > 256) __nanosleep(64);
+                if (clock64() - t0 > (1LL << 31)) *s_fail = 1;
+            } while (!*s_fail);
+        }
+        __syncthreads();
+        return !*s_fail;
+    }
+    // the last CTA to leave clears the counters for the next launch
+    __device__ __forceinline__ void leave(int *err)
+    {
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            if (*s_fail) atomicOr(err, 1);
+            __threadfence();
+            if (atomicAdd(ctr + 1, 1u) == gridDim.x - 1) {
+                ctr[0] = 0;
+                ctr[1] = 0;
+                __threadfence();
+            }
+        }
+    }
+};
+
+// Levels lt .. nl on one CTA, in shared memory: b of level lt comes in from global memory, x
+// of it goes back.
+__device__ __noinline__ void chip_sweeps(const Coop64Level &V, double *x, const double *b, const double *c0t,
+                                         const double *rc, int iters, bool zero_start, double omega, double omw)
+{
+    for (int h = 0; h < 2 * iters; ++h) {
+        half_sweep<Near, false>(V, x, b, c0t, rc, h, zero_start && h == 0, omega, omw, threadIdx.x, blockDim.x);
+        __syncthreads();
+    }
+}
+
+__device__ void chip_tail(const Coop64Desc &D, double *sm)
+{
+    __shared__ double cs[5][kChipCoarseMax];
+    const int lt = D.lt, nl = D.nl, t0 = threadIdx.x, st = blockDim.x;
+    for (int q = t0; q < D.sm_doubles; q += st) sm[q] = 0.0;
+    __syncthreads();
+    cells(D.lv[lt], t0, st, [&](int, int, int, int p) { sm[D.sm_b[lt] + p] = __ldcg(D.lv[lt].b + p); });
+    for (int l = lt; l < nl; ++l) {
+        const Coop64Level &V = D.lv[l];
+        const long long total = V.L.sz * (V.L.nz + 2);
+        cells(V, t0, st, [&](int, int, int, int p) {
+            sm[D.sm_c0[l] + p] = V.c0t[p];
+            sm[D.sm_rc[l] + p] = V.c0t[p + total];
+        });
+    }
+    __syncthreads();
+    double *r = sm + D.sm_r;
+    for (int l = lt; l < nl; ++l) {
+        const Coop64Level &V = D.lv[l];
+        double *x = sm + D.sm_x[l], *b = sm + D.sm_b[l], *bc = sm + D.sm_b[l + 1];
+        const double *c0 = sm + D.sm_c0[l], *rc = sm + D.sm_rc[l];
+        chip_sweeps(V, x, b, c0, rc, D.maxit, true, D.omega, D.omw);
+        residual<Near, false>(V, r, x, b, c0, t0, st);
+        __syncthreads();
+        restriction<Near, false>(D.lv[l + 1], V.X, r, bc, t0, st);
+        __syncthreads();
+    }
+    {
+        const LevelK<double> &C = D.lv[nl].L;
+        const double *b = sm + D.sm_b[nl];
+        double *x = sm + D.sm_x[nl];
+        const int total = (int)(C.sz * (C.nz + 2));
+        for (int q = t0; q < total; q += st) cs[1][q] = b[q];
+        __syncthreads();
+        int xs;
+        const int iters =
+            C.nx * C.ny * C.nz > 128
+                ? coarse_rbgs_chip<true, true>(C, cs, D.coarse_maxit, D.tol, D.omega, D.omw, D.abort, &xs)
+                : coarse_rbgs_chip<true, false>(C, cs, D.coarse_maxit, D.tol, D.omega, D.omw, D.abort, &xs);
+        if (t0 == 0) *D.iters_out = iters;
+        for (int q = t0; q < total; q += st) x[q] = cs[xs][q];
+        __syncthreads();
+    }
+    for (int l = nl - 1; l >= lt; --l) {
+        const Coop64Level &V = D.lv[l];
+        double *x = sm + D.sm_x[l], *b = sm + D.sm_b[l];
+        const double *c0 = sm + D.sm_c0[l], *rc = sm + D.sm_rc[l], *xc = sm + D.sm_x[l + 1];
+        if (V.L.nx * V.L.ny * V.L.nz > 128)
+            prolong_add<Near, true>(V, xc, x, t0, st);
+        else
+            prolong_add<Near, false>(V, xc, x, t0, st);
+        __syncthreads();
+        chip_sweeps(V, x, b, c0, rc, D.maxit, false, D.omega, D.omw);
+    }
+    cells(D.lv[lt], t0, st, [&](int, int, int, int p) { D.lv[lt].x[p] = sm[D.sm_x[lt] + p]; });
+}
+
+// Levels l0 .. nl of one V-cycle; x0, b0, r0: the arrays of level 0 where l0 is 0, and then
+// the cycle's residual norm goes to *norm_out.
+__global__ void __launch_bounds__(kThreads, 1)
+    k_coop_f64(const Coop64Desc *__restrict__ Dp, double *x0, const double *b0, double *r0, double *norm_out)
+{
+    extern __shared__ double coop_sm[];
+    __shared__ int s_fail;
+    __shared__ double sw[kThreads / 32];
+    const Coop64Desc &D = *Dp;
+    if (threadIdx.x == 0) s_fail = 0;
+    __syncthreads();
+    GridBarrier bar{D.bar, 0u, &s_fail};
+    const int q0 = spread_start(), step = gridDim.x * blockDim.x;
+    auto X = [&](int l) { return l == 0 ? x0 : D.lv[l].x; };
+    auto B = [&](int l) { return l == 0 ? b0 : (const double *)D.lv[l].b; };
+    auto R = [&](int l) { return l == 0 ? r0 : D.lv[l].r; };
+    auto smooth = [&](int l, bool zero_start) {
+        const Coop64Level &V = D.lv[l];
+        const long long total = V.L.sz * (V.L.nz + 2);
+        if (zero_start && D.maxit == 0) {
+            cells(V, q0, step, [&](int, int, int, int p) { X(l)[p] = 0.0; });
+            return bar.sync();
+        }
+        for (int h = 0; h < 2 * D.maxit; ++h) {
+            half_sweep<Far, false>(V, X(l), B(l), V.c0t, V.c0t + total, h, zero_start && h == 0, D.omega, D.omw, q0,
+                                  step);
+            if (!bar.sync()) return false;
+        }
+        return true;
+    };
+    bool ok = true;
+    for (int l = D.l0; ok && l < D.lt; ++l) {
+        const Coop64Level &V = D.lv[l];
+        ok = smooth(l, l > 0);
+        if (!ok) break;
+        residual<Far, false>(V, R(l), X(l), B(l), V.c0t, q0, step);
+        ok = bar.sync();
+        if (!ok) break;
+        restriction<Far, false>(D.lv[l + 1], V.X, R(l), D.lv[l + 1].b, q0, step);
+        ok = bar.sync();
+    }
+    if (ok) {
+        if (blockIdx.x == 0) chip_tail(D, coop_sm);
+        if (gridDim.x > 1) ok = bar.sync();
+    }
+    for (int l = D.lt - 1; ok && l >= D.l0; --l) {
+        const LevelK<double> &L = D.lv[l].L;
+        if (L.nx * L.ny * L.nz > kManyCells)
+            prolong_add<Far, true>(D.lv[l], D.lv[l + 1].x, X(l), q0, step);
+        else
+            prolong_add<Far, false>(D.lv[l], D.lv[l + 1].x, X(l), q0, step);
+        ok = bar.sync() && smooth(l, false);
+    }
+    if (ok && norm_out) {
+        const double acc = residual<Far, false>(D.lv[0], r0, x0, b0, D.lv[0].c0t, q0, step);
+        const double s = block_sum(acc, sw);
+        if (threadIdx.x == 0) D.partials[blockIdx.x] = s;
+        ok = bar.sync();
+        if (ok && blockIdx.x == 0) {
+            double t = 0.0;
+            for (int q = threadIdx.x; q < (int)gridDim.x; q += blockDim.x) t = __dadd_rn(t, __ldcg(D.partials + q));
+            t = block_sum(t, sw);
+            if (threadIdx.x == 0) *norm_out = t;
+        }
+    }
+    bar.leave(D.err);
+}
+
+// The half-sweeps of a smoother call on one small level: two iterations take 12.4 us up to 32^3
+// cells and 18.5 at 48^3, and 24.6 as four launches (which start 6.1 us apart however small).
+__global__ void __launch_bounds__(kThreads, 1)
+    k_coop_sweeps(Coop64Level V, double *x, const double *b, int iters, double omega, double omw, unsigned *ctr,
+                  int *err)
+{
+    __shared__ int s_fail;
+    if (threadIdx.x == 0) s_fail = 0;
+    __syncthreads();
+    GridBarrier bar{ctr, 0u, &s_fail};
+    const int q0 = spread_start(), step = gridDim.x * blockDim.x;
+    const long long total = V.L.sz * (V.L.nz + 2);
+    for (int h = 0; h < 2 * iters; ++h) {
+        half_sweep<Far, false>(V, x, b, V.c0t, V.c0t + total, h, false, omega, omw, q0, step);
+        if (h + 1 < 2 * iters && !bar.sync()) break;
+    }
+    bar.leave(err);
+}
+
+}  // namespace
+
+int coop64_grid(int device, int *grid)
+{
+    int coop = 0, sms = 0, per = 0;
+    *grid = 0;
+    cudaError_t e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_coop_f64, cudaFuncAttributeMaxDynamicSharedMemorySize, kCoop64SmemBytes);
+    if (e == cudaSuccess)
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_coop_f64, kThreads, kCoop64SmemBytes);
+    if (e == cudaSuccess && coop && per > 0) *grid = sms;
+    return cuda_status(e, "cooperative launch set-up");
+}
+
+int coop64_cycle(const Coop64Desc *dev, int grid, int smem, double *x0, const double *b0, double *r0, double *norm_out,
+                 cudaStream_t s)
+{
+    void *args[] = {(void *)&dev, (void *)&x0, (void *)&b0, (void *)&r0, (void *)&norm_out};
+    const cudaError_t e =
+        cudaLaunchCooperativeKernel((const void *)k_coop_f64, dim3(grid), dim3(kThreads), args, (size_t)smem, s);
+    count_launches(1);
+    return cuda_status(e, "small levels");
+}
+
+int coop64_sweeps(const Coop64Level &V, int grid, double *x, const double *b, int iters, double omega, unsigned *bar,
+                  int *err, cudaStream_t s)
+{
+    Coop64Level v = V;
+    double omw = 1.0 - omega;
+    void *args[] = {(void *)&v, (void *)&x, (void *)&b, (void *)&iters, (void *)&omega, (void *)&omw, (void *)&bar,
+                    (void *)&err};
+    const cudaError_t e =
+        cudaLaunchCooperativeKernel((const void *)k_coop_sweeps, dim3(grid), dim3(kThreads), args, 0, s);
+    count_launches(1);
+    return cuda_status(e, "small level's sweeps");
+}
+
+}  // namespace pmg

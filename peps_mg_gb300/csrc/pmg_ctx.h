@@ -72,6 +72,16 @@ struct Ctx {
     bool deep_tail = true;     // mixed cycle: move small levels into the tail (batch members keep tail_l0)
     TailDesc<double> tail_host;
     TailDesc<double> *d_tail = nullptr;
+    // small levels of the plain FP64 cycle in one cooperative launch (coop_l0 <= nl: in use)
+    int coop_l0 = 1 << 30, coop_grid = 0, coop_smem = 0;
+    Coop64Desc *coop_host = nullptr, *d_coop = nullptr;
+    unsigned *d_bar = nullptr;
+    int setup_coop64();
+    int upload_coop64(int maxit, double omega, double tol);
+    int check_coop64();
+    bool coop64_level_ok(int l, long long cells) const;
+    Coop64Level coop64_level(int l) const;
+    int fetch_cycle(double *rsd_val, int *coarse_iters);
     double *d_partials = nullptr;
     size_t npart_cap = 0;
     double *d_scal = nullptr;

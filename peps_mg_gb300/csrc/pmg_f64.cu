@@ -250,23 +250,6 @@ __global__ void __launch_bounds__(kBX *kBY) k_restrict_f64(XferK<double> X, cons
         }
 }
 
-// Coarse index, neighbour and the own and the neighbour's 1-D weight of fine index f along
-// one axis (stride 2: odd f is the low child, even f the high one; stride 1: the high child,
-// src/multigrid.f90:1594-1649).
-__device__ __forceinline__ void side64(int st, int f, const double *pp, const double *pn, int &c, int &nb, double &wa,
-                                       double &wb)
-{
-    if (st == 2) {
-        c = (f + 1) >> 1;
-        nb = (f & 1) ? c - 1 : c + 1;
-        wa = (f & 1) ? pp[f] : pn[f];
-        wb = (f & 1) ? pp[f + 1] : pn[f - 1];
-    } else {
-        c = nb = f;
-        wa = wb = pn[f];
-    }
-}
-
 // Prolongation on the integer pipe: a thread takes the fine cells of one column over a chunk
 // of fine planes (coalesced, where a thread per coarse cell writes every second cell).  The
 // x-y products of the weights are formed once per column; the eight weights, the denominator
@@ -679,14 +662,15 @@ void grid_for_cells(const LevelK<double> &L, const Launch &ln, dim3 *grid, dim3 
 
 // The grid of the column kernels (each_cell and its kin): the tiles of the (i, j) plane and
 // chunks of planes, of at most 8 so that a thread's column set-up is shared, as long as the
-// grid fills every SM a few times over.
-static dim3 grid_columns(int nx_threads, int ny, int nz, const Launch &ln)
+// grid fills every SM a few times over.  kc_min: planes per chunk that pay for the set-up even
+// where they leave SMs with fewer CTAs (the prolongation's weights: 64^3, 4 planes).
+static dim3 grid_columns(int nx_threads, int ny, int nz, const Launch &ln, int kc_min = 1)
 {
     dim3 g = grid3(nx_threads, ny, nz, ln);
     if (ln.collapse[2]) return g;
     const long long want = 152 * 16;
     const long long ctas = (long long)g.x * g.y * nz;
-    const int kc = (int)(ctas / want < 1 ? 1 : ctas / want > 8 ? 8 : ctas / want);
+    const int kc = (int)(ctas / want < kc_min ? kc_min : ctas / want > 8 ? 8 : ctas / want);
     const int gz = (nz + kc - 1) / kc;
     g.z = (unsigned)(gz < kMaxGridZ ? gz : kMaxGridZ);
     return g;
@@ -807,7 +791,7 @@ int f64_prolong(const XferK<double> &X, const Launch &ln, const double *vc, doub
 {
     const dim3 bl(kBX, kBY, 1);
     if (X.mul64) {
-        const dim3 g = grid_columns(X.ncx * X.stx, X.ncy * X.sty, X.ncz * X.stz, ln);
+        const dim3 g = grid_columns(X.ncx * X.stx, X.ncy * X.sty, X.ncz * X.stz, ln, 4);
         if (add)
             k_prolong_m64<true><<<g, bl, 0, s>>>(X, vc, vf);
         else

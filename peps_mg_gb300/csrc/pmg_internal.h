@@ -56,6 +56,35 @@ struct TailDesc {
     const volatile int *abort;
 };
 
+// The small levels of a plain FP64 V-cycle in one cooperative launch (pmg_coop64.cu): levels
+// l0 .. lt-1 over the whole grid, lt .. nl on one CTA in shared memory (offsets in doubles).
+struct Coop64Level {
+    LevelK<double> L;
+    XferK<double> X;              // to the next coarser level
+    double *x, *b, *r;
+    const double *c0t;            // diagonal table and reciprocals (f64_diag_table)
+    unsigned dhx, dnx, dny;       // fastdiv's factors of (nx+1)/2, nx and ny
+};
+struct Coop64Desc {
+    int l0, lt, nl, maxit, coarse_maxit;
+    double omega, omw, tol;
+    Coop64Level lv[kMaxLevels];
+    int sm_x[kMaxLevels], sm_b[kMaxLevels], sm_c0[kMaxLevels], sm_rc[kMaxLevels], sm_r, sm_doubles;
+    int *iters_out, *err;
+    unsigned *bar;                // two counters, zero between launches
+    double *partials;
+    const volatile int *abort;
+};
+constexpr int kCoop64SmemBytes = 96 * 1024;   // dynamic shared memory of the on-chip levels at most
+constexpr int kCoop64Cells = 1 << 15;         // levels of at most this many cells
+constexpr int kCoop64TailCells = 512;         // levels of at most this many run on one CTA
+constexpr int kCoop64SweepCells = 1 << 17;    // a smoother call's half-sweeps in one launch: levels of at most this
+int coop64_grid(int device, int *grid);       // CTAs of a launch; 0 = not available
+int coop64_cycle(const Coop64Desc *dev, int grid, int smem, double *x0, const double *b0, double *r0, double *norm_out,
+                 cudaStream_t s);
+int coop64_sweeps(const Coop64Level &V, int grid, double *x, const double *b, int iters, double omega, unsigned *bar,
+                  int *err, cudaStream_t s);
+
 // Layout of a hierarchy built on the device (pmg_f64.cu): level sizes and, per level and
 // axis, the offsets (in doubles) of the mesh (dm, dg, xg, n+2 values each, consecutive) in
 // the mesh blob and of the coefficient tables / transfer weights in the table blob.
