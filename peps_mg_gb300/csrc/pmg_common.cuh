@@ -321,6 +321,14 @@ __device__ __forceinline__ void prolong_cell_f64(const XferK<double> &X, const d
     }
 }
 
+// The planes k0 .. k1 of this CTA: consecutive chunks of the nz planes.
+__device__ __forceinline__ void plane_chunk(int nz, int &k0, int &k1)
+{
+    const int kc = (nz + gridDim.z - 1) / gridDim.z;
+    k0 = 1 + kc * blockIdx.z;
+    k1 = min(nz, k0 + kc - 1);
+}
+
 // Deterministic block-wide sum (fixed shuffle tree, then warps in order).  All
 // threads of the block must call it; returns the sum in every thread.
 template <typename T>

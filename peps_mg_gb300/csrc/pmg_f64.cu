@@ -7,6 +7,7 @@
 // column (the CGPSA per-axis step-down), without changing any cell's arithmetic.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <type_traits>
 
 #include "../../include/peps_mg.h"
@@ -75,14 +76,6 @@ __device__ __forceinline__ double ax_cell(const LevelK<double> &L, const double 
     t = __dadd_rn(t, prod<MODE>(L.czm[k], x[p - L.sz]));
     t = __dadd_rn(t, prod<MODE>(L.czp[k], x[p + L.sz]));
     return t;
-}
-
-// The planes k0 .. k1 of this CTA: consecutive chunks of the nz planes.
-__device__ __forceinline__ void plane_chunk(int nz, int &k0, int &k1)
-{
-    const int kc = (nz + gridDim.z - 1) / gridDim.z;
-    k0 = 1 + kc * blockIdx.z;
-    k1 = min(nz, k0 + kc - 1);
 }
 
 // f(i, j, k, p) on the cells of this thread.
@@ -283,6 +276,8 @@ __global__ void __launch_bounds__(kBX *kBY) k_prolong_m64(XferK<double> X, const
                 int k, kn;
                 double a, b;
                 side64(X.stz, kf, X.pzp, X.pzn, k, kn, a, b);
+                const long long q = X.fsz * kf;
+                const double old = ADD ? out[q] : 0.0;
                 if (kf == k0 || __double_as_longlong(a) != __double_as_longlong(az) ||
                     __double_as_longlong(b) != __double_as_longlong(bz)) {
                     az = a;
@@ -306,8 +301,7 @@ __global__ void __launch_bounds__(kBX *kBY) k_prolong_m64(XferK<double> X, const
 #pragma unroll
                 for (int u = 1; u < 8; ++u) t[0] = __dadd_rn(t[0], t[u]);
                 const double v = quot64_near(t[0], den, y);
-                const long long q = X.fsz * kf;
-                out[q] = ADD ? __dadd_rn(out[q], v) : v;
+                out[q] = ADD ? __dadd_rn(old, v) : v;
             }
         }
 }
@@ -426,7 +420,7 @@ __global__ void __launch_bounds__(kBX *kBY) k_cg_init(LevelK<double> L, double *
 
 // Ap = A p (src/poisson_matrix_operator.f90:146-159), temp2 = Ap.p (:112), alpha (:114)
 template <int MODE>
-__global__ void __launch_bounds__(kBX *kBY) k_cg_apdot(LevelK<double> L, const double *__restrict__ p,
+__global__ void __launch_bounds__(kBX *kBY, MODE == kInt ? 6 : 1) k_cg_apdot(LevelK<double> L, const double *__restrict__ p,
                                                        double *__restrict__ ap, double *partials, CgState *st,
                                                        const double *__restrict__ c0t)
 {
@@ -458,10 +452,13 @@ __global__ void __launch_bounds__(kBX *kBY) k_cg_update(LevelK<double> L, double
 {
     if (st->done) return;
     const double alpha = st->alpha;
+    const Mul64 fa = mul64_factor(alpha);
+    const bool in = mul64_factor_ok(alpha);     // the same for every thread
     double acc = 0.0;
     each_cell(L, [&](int, int, int, long long q) {
-        x[q] = __dadd_rn(x[q], mul64_vv(alpha, p[q]));
-        const double v = __dsub_rn(r[q], mul64_vv(alpha, ap[q]));
+        const double xq = x[q], pq = p[q], rq = r[q], aq = ap[q];
+        x[q] = __dadd_rn(xq, in ? mul64(fa, pq) : mul64_slow_vv(alpha, pq));
+        const double v = __dsub_rn(rq, in ? mul64(fa, aq) : mul64_slow_vv(alpha, aq));
         r[q] = v;
         acc = add_prod(acc, v, v);
     });
@@ -489,7 +486,11 @@ __global__ void __launch_bounds__(kBX *kBY) k_cg_p(LevelK<double> L, double *__r
 {
     if (st->done) return;
     const double beta = st->beta;
-    each_cell(L, [&](int, int, int, long long q) { p[q] = __dadd_rn(r[q], mul64_vv(beta, p[q])); });
+    const Mul64 fb = mul64_factor(beta);
+    const bool in = mul64_factor_ok(beta);
+    each_cell(L, [&](int, int, int, long long q) {
+        p[q] = __dadd_rn(r[q], in ? mul64(fb, p[q]) : mul64_slow_vv(beta, p[q]));
+    });
 }
 
 // ------------------------------------------------------------------------------------
@@ -663,14 +664,16 @@ void grid_for_cells(const LevelK<double> &L, const Launch &ln, dim3 *grid, dim3 
 // The grid of the column kernels (each_cell and its kin): the tiles of the (i, j) plane and
 // chunks of planes, of at most 8 so that a thread's column set-up is shared, as long as the
 // grid fills every SM a few times over.  kc_min: planes per chunk that pay for the set-up even
-// where they leave SMs with fewer CTAs (the prolongation's weights: 64^3, 4 planes).
-static dim3 grid_columns(int nx_threads, int ny, int nz, const Launch &ln, int kc_min = 1)
+// where they leave SMs with fewer CTAs (the prolongation's weights: 64^3, 4 planes).  sum: the
+// CTAs end with a block sum, 48 warp instructions on the FP64 unit (0.45 us an SM), so they are
+// fewer and longer (a CG update of 224 x 160 x 128: 65 -> 52 us with 1216 CTAs instead of 4864).
+dim3 grid_columns(int nx_threads, int ny, int nz, const Launch &ln, int kc_min, bool sum)
 {
     dim3 g = grid3(nx_threads, ny, nz, ln);
     if (ln.collapse[2]) return g;
-    const long long want = 152 * 16;
+    const long long want = sum ? 152 * 8 : 152 * 16, kc_max = sum ? 64 : 8;
     const long long ctas = (long long)g.x * g.y * nz;
-    const int kc = (int)(ctas / want < kc_min ? kc_min : ctas / want > 8 ? 8 : ctas / want);
+    const int kc = (int)std::min(kc_max, std::max((long long)kc_min, ctas / want));
     const int gz = (nz + kc - 1) / kc;
     g.z = (unsigned)(gz < kMaxGridZ ? gz : kMaxGridZ);
     return g;
@@ -737,7 +740,7 @@ int f64_diag_table(const LevelK<double> &L, double *c0t, cudaStream_t s)
 int f64_residual(const LevelK<double> &L, const Launch &ln, double *r, const double *x, const double *b,
                  double *partials, int *npart, cudaStream_t s, const double *c0t)
 {
-    const dim3 g = grid_columns(L.nx, L.ny, L.nz, ln), bl(kBX, kBY, 1);
+    const dim3 g = grid_columns(L.nx, L.ny, L.nz, ln, 1, partials != nullptr), bl(kBX, kBY, 1);
     with_mode(arith_mode(L, c0t), [&](auto m) {
         if (partials)
             k_residual_f64<true, decltype(m)::value><<<g, bl, 0, s>>>(L, r, x, b, partials, c0t);
@@ -833,19 +836,8 @@ int f64_tail(const TailDesc<double> *dev_desc, int threads, cudaStream_t s)
 }
 
 
-// Grid of the fused CG kernels: the level's CTA tiles in x and y, and enough z planes per
-// CTA that the grid is about four waves of 256-thread CTAs (at most 4864 CTAs, so the
-// last CTA's sum over the partials stays short); collapsed axes keep one CTA column.
-static dim3 cg_grid(const LevelK<double> &L, const Launch &ln)
-{
-    dim3 g = grid3(L.nx, L.ny, L.nz, ln);
-    const unsigned plane = g.x * g.y;
-    const unsigned target = 4864;
-    unsigned gz = plane >= target ? 1u : (target + plane - 1) / plane;
-    if (gz > g.z) gz = g.z;
-    g.z = gz;
-    return g;
-}
+// Grid of the fused CG kernels (every one of them, so that a cell stays with its thread).
+static dim3 cg_grid(const LevelK<double> &L, const Launch &ln) { return grid_columns(L.nx, L.ny, L.nz, ln, 1, true); }
 
 int f64_cg_partials(const LevelK<double> &L, const Launch &ln)
 {

@@ -25,6 +25,7 @@
 #include <algorithm>
 
 #include "pmg_internal.h"
+#include "pmg_mul64.cuh"
 
 namespace pmg {
 
@@ -46,8 +47,10 @@ __global__ void __launch_bounds__(kBX *kBY) k_fast_wdiag(LevelK<double> L, doubl
 }
 
 // One colour of the red-black sweep (colour 0: (i+j+k) odd first, as the bitwise kernel).
+// Bound by the latency of its loads (FP64 unit about half busy), so six CTAs per SM: 320 x 256
+// x 192, finest level, 123 -> 112 us.
 template <bool OMEGA1>
-__global__ void __launch_bounds__(kBX *kBY) k_rbgs_fast(LevelK<double> L, const double *__restrict__ wd,
+__global__ void __launch_bounds__(kBX *kBY, 6) k_rbgs_fast(LevelK<double> L, const double *__restrict__ wd,
                                                         double *__restrict__ x, const double *__restrict__ b,
                                                         double omw, int colour)
 {
@@ -64,12 +67,16 @@ __global__ void __launch_bounds__(kBX *kBY) k_rbgs_fast(LevelK<double> L, const 
                 acc = fma(-cyp, x[p + L.sy], acc);
                 acc = fma(-czm, x[p - L.sz], acc);
                 acc = fma(-czp, x[p + L.sz], acc);
-                x[p] = OMEGA1 ? wd[p] * acc : fma(wd[p], acc, omw * x[p]);
+                // the update's lone product on the integer pipe (pmg_mul64.cuh): 6 FP64
+                // instructions instead of 7
+                x[p] = OMEGA1 ? mul64_vv(wd[p], acc) : fma(wd[p], acc, mul64_vv(omw, x[p]));
             }
         }
 }
 
-// r = b - A x with -c0 = sx(i) + dy(j) + dz(k); with NORM the per-block sums of r^2.
+// r = b - A x with -c0 = sx(i) + dy(j) + dz(k); with NORM the per-block sums of r^2.  A thread
+// takes a column over a chunk of planes: one block sum per chunk instead of one per plane (320 x
+// 256 x 192 with the norm: 480 -> 241 us).
 template <bool NORM>
 __global__ void __launch_bounds__(kBX *kBY) k_residual_fast(LevelK<double> L, const double *__restrict__ dy,
                                                             const double *__restrict__ dz, double *__restrict__ r,
@@ -77,15 +84,23 @@ __global__ void __launch_bounds__(kBX *kBY) k_residual_fast(LevelK<double> L, co
                                                             const double *__restrict__ b, double *partials)
 {
     double acc2 = 0.0;
-    for (int k = blockIdx.z + 1; k <= L.nz; k += gridDim.z)
-        for (int j = blockIdx.y * blockDim.y + threadIdx.y + 1; j <= L.ny; j += gridDim.y * blockDim.y) {
-            const double dyz = dy[j] + dz[k];
-            const double cym = L.cym[j], cyp = L.cyp[j], czm = L.czm[k], czp = L.czp[k];
-            for (int i = blockIdx.x * blockDim.x + threadIdx.x + 1; i <= L.nx; i += gridDim.x * blockDim.x) {
+    int k0, k1;
+    plane_chunk(L.nz, k0, k1);
+    for (int j = blockIdx.y * blockDim.y + threadIdx.y + 1; j <= L.ny; j += gridDim.y * blockDim.y)
+        for (int i = blockIdx.x * blockDim.x + threadIdx.x + 1; i <= L.nx; i += gridDim.x * blockDim.x) {
+            const double cym = L.cym[j], cyp = L.cyp[j], cxm = L.cxm[i], cxp = L.cxp[i], sx = L.sx[i], dyj = dy[j];
+            double dzk = 0.0, d = 0.0;
+            for (int k = k0; k <= k1; ++k) {
                 const long long p = lin(i, j, k, L.sy, L.sz);
-                double acc = fma(L.sx[i] + dyz, x[p], b[p]);
-                acc = fma(-L.cxm[i], x[p - 1], acc);
-                acc = fma(-L.cxp[i], x[p + 1], acc);
+                const double czm = L.czm[k], czp = L.czp[k];
+                // the diagonal changes with the plane only where the z widths do
+                if (k == k0 || __double_as_longlong(dz[k]) != __double_as_longlong(dzk)) {
+                    dzk = dz[k];
+                    d = sx + (dyj + dzk);
+                }
+                double acc = fma(d, x[p], b[p]);
+                acc = fma(-cxm, x[p - 1], acc);
+                acc = fma(-cxp, x[p + 1], acc);
                 acc = fma(-cym, x[p - L.sy], acc);
                 acc = fma(-cyp, x[p + L.sy], acc);
                 acc = fma(-czm, x[p - L.sz], acc);
@@ -127,62 +142,90 @@ __global__ void __launch_bounds__(kBX *kBY) k_restrict_fast(XferK<double> X, Fas
             }
 }
 
-// The eight children of a coarse cell, x_f += P x_c (ADD) or x_f = P x_c: per child a
-// z-interpolation of y-interpolations of x-interpolations of the coarse values, with the
-// weights of the reference's trilinear formula normalised per axis (pa own side, pb the
-// neighbour's).  The x-interpolations of the 3 x 3 coarse lines around the cell are
-// shared by the children.  Coarse ghost values (zero for a correction) enter as in the
-// reference; along a stride-1 axis the neighbour is the cell itself.
-template <bool ADD>
-__global__ void __launch_bounds__(kBX *kBY) k_prolong_fast(XferK<double> X, FastXferK W,
+// x_f += P x_c: per child a z-interpolation of y-interpolations of x-interpolations of the
+// coarse values, with the weights of the reference's trilinear formula normalised per axis
+// (pa own side, pb the neighbour's).  Coarse ghost values (zero for a correction) enter as in
+// the reference; along a stride-1 axis the neighbour is the cell itself.
+//
+// A thread takes a column of coarse cells over a chunk of planes: the x- and y-interpolated
+// values of a coarse plane (four: two children per axis) serve the planes above and below it,
+// and each interpolation's lone product runs on the integer pipe (INT; weights within mul64's
+// range), which leaves 26 FP64 instructions per coarse cell of the 84 of a thread that
+// interpolates its eight children by itself.  Same values: same operations, formed once.
+// Finest level of 320 x 256 x 192: about 370 -> 200 us.
+template <bool INT>
+__global__ void __launch_bounds__(kBX *kBY, 3) k_prolong_fast(XferK<double> X, FastXferK W,
                                                            const double *__restrict__ vc, double *__restrict__ vf)
 {
-    for (int k = blockIdx.z + 1; k <= X.ncz; k += gridDim.z)
-        for (int j = blockIdx.y * blockDim.y + threadIdx.y + 1; j <= X.ncy; j += gridDim.y * blockDim.y)
-            for (int i = blockIdx.x * blockDim.x + threadIdx.x + 1; i <= X.ncx; i += gridDim.x * blockDim.x) {
-                const int ox = X.stx - 1, oy = X.sty - 1, oz = X.stz - 1;
-                const int ip = i * X.stx, iz = ip - ox;
-                const int jp = j * X.sty, jz = jp - oy;
-                const int kp = k * X.stz, kz = kp - oz;
-                // xi[s][b][c]: x-side s (0 low child iz, 1 high child ip) on coarse line
-                // (j + (b-1) oy, k + (c-1) oz)
-                double xi[2][3][3];
-                const double alo = W.pax[iz], blo = W.pbx[iz], ahi = W.pax[ip], bhi = W.pbx[ip];
+    const int ox = X.stx - 1, oy = X.sty - 1, oz = X.stz - 1;
+    int k0, k1;
+    plane_chunk(X.ncz, k0, k1);
+    auto times = [](const Mul64 &f, double w, double v) { return INT ? mul64(f, v) : w * v; };
+    for (int j = blockIdx.y * blockDim.y + threadIdx.y + 1; j <= X.ncy; j += gridDim.y * blockDim.y)
+        for (int i = blockIdx.x * blockDim.x + threadIdx.x + 1; i <= X.ncx; i += gridDim.x * blockDim.x) {
+            const int ip = i * X.stx, iz = ip - ox, jp = j * X.sty, jz = jp - oy;
+            const double alo = W.pax[iz], blo = W.pbx[iz], ahi = W.pax[ip], bhi = W.pbx[ip];
+            const double ay[2] = {W.pay[jz], W.pay[jp]}, by[2] = {W.pby[jz], W.pby[jp]};
+            const Mul64 flo = mul64_factor(blo), fhi = mul64_factor(bhi);
+            const Mul64 fy[2] = {mul64_factor(by[0]), mul64_factor(by[1])};
+            const double *col = vc + lin(i, j, 0, X.csy, X.csz);
+            // the (low, high) x (low, high) children's values on coarse plane k
+            auto plane = [&](int k, double (&Y)[2][2]) {
+                double xi[2][3];
 #pragma unroll
-                for (int c = 0; c < 3; ++c)
+                for (int c = 0; c < 3; ++c) {
+                    const double *q = col + X.csz * k + (c - 1) * oy * X.csy;
+                    xi[0][c] = fma(alo, q[0], times(flo, blo, q[-ox]));
+                    xi[1][c] = fma(ahi, q[0], times(fhi, bhi, q[ox]));
+                }
 #pragma unroll
-                    for (int bb = 0; bb < 3; ++bb) {
-                        const long long p = lin(i, j + (bb - 1) * oy, k + (c - 1) * oz, X.csy, X.csz);
-                        const double v0 = vc[p];
-                        xi[0][bb][c] = fma(alo, v0, blo * vc[p - ox]);
-                        xi[1][bb][c] = fma(ahi, v0, bhi * vc[p + ox]);
-                    }
+                for (int si = 0; si < 2; ++si)
+#pragma unroll
+                    for (int sj = 0; sj < 2; ++sj)
+                        Y[si][sj] = fma(ay[sj], xi[si][1], times(fy[sj], by[sj], xi[si][sj ? 2 : 0]));
+            };
+            double A[2][2], B[2][2], C[2][2];
+            if (oz) plane(k0 - 1, A);
+            plane(k0, B);
+            for (int k = k0; k <= k1; ++k) {
+                if (oz) plane(k + 1, C);
 #pragma unroll
                 for (int sk = 0; sk < 2; ++sk) {
                     if (sk == 0 && oz == 0) continue;
-                    const int kf = sk ? kp : kz, cz = sk ? 2 : 0;
+                    const int kf = sk ? k * X.stz : k * X.stz - oz;
                     const double az = W.paz[kf], bz = W.pbz[kf];
+                    const Mul64 fz = mul64_factor(bz);
+                    // the children's old values, in flight together (a load behind each store
+                    // would wait for memory four times)
+                    double old[2][2];
+#pragma unroll
+                    for (int c = 0; c < 4; ++c)
+                        if (!((c & 1) == 0 && ox == 0) && !((c >> 1) == 0 && oy == 0))
+                            old[c >> 1][c & 1] = vf[lin(c & 1 ? ip : iz, c >> 1 ? jp : jz, kf, X.fsy, X.fsz)];
 #pragma unroll
                     for (int sj = 0; sj < 2; ++sj) {
                         if (sj == 0 && oy == 0) continue;
-                        const int jf = sj ? jp : jz, by = sj ? 2 : 0;
-                        const double ay = W.pay[jf], byw = W.pby[jf];
 #pragma unroll
                         for (int si = 0; si < 2; ++si) {
                             if (si == 0 && ox == 0) continue;
-                            const int ifn = si ? ip : iz;
-                            const double yo = fma(ay, xi[si][1][1], byw * xi[si][by][1]);
-                            const double yn = fma(ay, xi[si][1][cz], byw * xi[si][by][cz]);
-                            const double v = fma(az, yo, bz * yn);
-                            const long long q = lin(ifn, jf, kf, X.fsy, X.fsz);
-                            if (ADD)
-                                vf[q] = vf[q] + v;
-                            else
-                                vf[q] = v;
+                            const double n = oz == 0 ? B[si][sj] : sk ? C[si][sj] : A[si][sj];
+                            const double v = fma(az, B[si][sj], times(fz, bz, n));
+                            const long long q = lin(si ? ip : iz, sj ? jp : jz, kf, X.fsy, X.fsz);
+                            vf[q] = old[sj][si] + v;
                         }
                     }
                 }
+                if (oz) {
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        A[q & 1][q >> 1] = B[q & 1][q >> 1];
+                        B[q & 1][q >> 1] = C[q & 1][q >> 1];
+                    }
+                } else if (k < k1) {
+                    plane(k + 1, B);
+                }
             }
+        }
 }
 
 // Per-axis tables of a level and of its transfer to the next (device side, from the
@@ -274,7 +317,7 @@ int fast_rbgs_sweeps(const LevelK<double> &L, const FastLevelK &F, const Launch 
 int fast_residual(const LevelK<double> &L, const FastLevelK &F, const Launch &ln, double *r, const double *x,
                   const double *b, double *partials, int *npart, cudaStream_t s)
 {
-    const dim3 g = grid3f(L.nx, L.ny, L.nz, ln), bl(kBX, kBY, 1);
+    const dim3 g = grid_columns(L.nx, L.ny, L.nz, ln, 1, partials != nullptr), bl(kBX, kBY, 1);
     if (partials) {
         k_residual_fast<true><<<g, bl, 0, s>>>(L, F.dy, F.dz, r, x, b, partials);
         *npart = (int)(g.x * g.y * g.z);
@@ -296,7 +339,11 @@ int fast_restrict(const XferK<double> &X, const FastXferK &W, const Launch &ln, 
 int fast_prolong(const XferK<double> &X, const FastXferK &W, const Launch &ln, const double *vc, double *vf,
                  cudaStream_t s)
 {
-    k_prolong_fast<true><<<grid3f(X.ncx, X.ncy, X.ncz, ln), dim3(kBX, kBY, 1), 0, s>>>(X, W, vc, vf);
+    const dim3 g = grid_columns(X.ncx, X.ncy, X.ncz, ln, 4), bl(kBX, kBY, 1);
+    if (X.mul64)
+        k_prolong_fast<true><<<g, bl, 0, s>>>(X, W, vc, vf);
+    else
+        k_prolong_fast<false><<<g, bl, 0, s>>>(X, W, vc, vf);
     count_launches(1);
     return cuda_status(cudaGetLastError(), "fast prolongation");
 }

@@ -101,6 +101,9 @@ struct HierDesc {
     long long ps[kMaxLevels][3], pr[kMaxLevels][3];
 };
 
+// Grid of the FP64 column kernels (32 x 8 threads, plane_chunk), pmg_f64.cu.
+dim3 grid_columns(int nx_threads, int ny, int nz, const Launch &ln, int kc_min = 1, bool sum = false);
+
 // ---- FP64 (bitwise) launchers, pmg_f64.cu -------------------------------------
 // Builds the coarse meshes (unless given) and every level's tables on the device.
 int hierarchy_setup(const HierDesc *dev_desc, double *meshes, double *tables, cudaStream_t s);

@@ -52,6 +52,13 @@ __device__ __forceinline__ bool mul64_in_range(unsigned xh)
     return xh + xh - (523u << 21) < (1001u << 21);
 }
 
+// Whether f can be a factor of mul64: exponent field in [623, 1423].
+__device__ __forceinline__ bool mul64_factor_ok(double f)
+{
+    const unsigned fh = (unsigned)__double2hiint(f);
+    return fh + fh - (623u << 21) < (801u << 21);
+}
+
 __device__ __forceinline__ bool is_zero64(unsigned xh, unsigned xl) { return ((xh << 1) | xl) == 0u; }
 
 // f x for x in range.
