@@ -29,6 +29,7 @@
 #include <vector>
 
 #include "pmg_ctx.h"
+#include "pmg_mul64.cuh"
 
 namespace pmg {
 
@@ -42,36 +43,60 @@ namespace {
 
 constexpr int kBX = 32, kBY = 8;
 
-// out = w / vol on the interior, 0 on the ghosts (mode 0); out = vol * w on the interior
-// (mode 1).  vol = dxm(i) dym(j) dzm(k).
+// out = in / vol on the interior (DIV) or vol * in, vol = dxm(i) dym(j) dzm(k).  A thread takes a
+// column over a chunk of planes and forms vol and its reciprocal where the plane's width
+// changes; INT (widths within mul64's range) then leaves 2 FP64 instructions of a division's 11
+// and none of a product's, with the same bits (quot64, pmg_mul64.cuh).  256^3: 201 -> 111 us
+// (a division), 201 -> 70 (a product).
+template <bool DIV, bool INT>
 __global__ void __launch_bounds__(kBX *kBY) k_volume_scale(int nx, int ny, int nz, int sy, long long sz,
                                                            const double *__restrict__ dxm,
                                                            const double *__restrict__ dym,
                                                            const double *__restrict__ dzm,
-                                                           const double *__restrict__ in, double *__restrict__ out,
-                                                           int mode)
+                                                           const double *__restrict__ in, double *__restrict__ out)
 {
-    for (int k = blockIdx.z + 1; k <= nz; k += gridDim.z)
-        for (int j = blockIdx.y * blockDim.y + threadIdx.y + 1; j <= ny; j += gridDim.y * blockDim.y)
-            for (int i = blockIdx.x * blockDim.x + threadIdx.x + 1; i <= nx; i += gridDim.x * blockDim.x) {
+    int k0, k1;
+    plane_chunk(nz, k0, k1);
+    for (int j = blockIdx.y * blockDim.y + threadIdx.y + 1; j <= ny; j += gridDim.y * blockDim.y)
+        for (int i = blockIdx.x * blockDim.x + threadIdx.x + 1; i <= nx; i += gridDim.x * blockDim.x) {
+            const double area = __dmul_rn(dxm[i], dym[j]);
+            double dz = 0.0, vol = 1.0, y = 1.0;
+            Mul64 f = mul64_factor(1.0);
+            for (int k = k0; k <= k1; ++k) {
                 const long long p = lin(i, j, k, sy, sz);
-                const double vol = __dmul_rn(__dmul_rn(dxm[i], dym[j]), dzm[k]);
-                out[p] = mode == 0 ? __ddiv_rn(in[p], vol) : __dmul_rn(vol, in[p]);
+                const double v = in[p];
+                if (k == k0 || __double_as_longlong(dzm[k]) != __double_as_longlong(dz)) {
+                    dz = dzm[k];
+                    vol = __dmul_rn(area, dz);
+                    if (INT && DIV) y = recip_f64(vol);
+                    if (INT) f = mul64_factor(vol);
+                }
+                if (DIV)
+                    out[p] = INT ? quot64(v, vol, y) : __ddiv_rn(v, vol);
+                else
+                    out[p] = INT ? mul64(f, v) : __dmul_rn(vol, v);
             }
+        }
 }
 
-// dL/dg for the six faces: block f sums -c_f * lambda over face f (x-, x+, y-, y+, z-, z+)
-// in a fixed order.
-__global__ void __launch_bounds__(1024) k_face_gradients(LevelK<double> L, const double *__restrict__ lam,
-                                                         double *__restrict__ out)
+// dL/dg for the six faces: the kFaceCtas CTAs of face f = blockIdx.y sum -c_f * lambda over
+// their share of face f (x-, x+, y-, y+, z-, z+) in a fixed order and the last of the face to
+// arrive adds their sums in order.  (One CTA per face was bound by the latency of its strided
+// loads: 256^3, 59 -> 14 us.)
+constexpr int kFaceCtas = 24;
+__global__ void __launch_bounds__(256) k_face_gradients(LevelK<double> L, const double *__restrict__ lam,
+                                                        double *__restrict__ partials, unsigned *__restrict__ arrive,
+                                                        double *__restrict__ out)
 {
-    __shared__ double sw[32];
-    const int f = blockIdx.x;
+    __shared__ double sw[8];
+    __shared__ bool s_last;
+    const int f = blockIdx.y;
     const int axis = f >> 1, hi = f & 1;
     const int n1 = axis == 0 ? L.ny : L.nx;
     const int n2 = axis == 2 ? L.ny : L.nz;
     double acc = 0.0;
-    for (long long q = threadIdx.x; q < (long long)n1 * n2; q += blockDim.x) {
+    for (long long q = blockIdx.x * blockDim.x + threadIdx.x; q < (long long)n1 * n2;
+         q += (long long)gridDim.x * blockDim.x) {
         const int a = (int)(q % n1) + 1, c = (int)(q / n1) + 1;
         int i, j, k;
         double coef;
@@ -85,10 +110,21 @@ __global__ void __launch_bounds__(1024) k_face_gradients(LevelK<double> L, const
             i = a; j = c; k = hi ? L.nz : 1;
             coef = hi ? L.czp[k] : L.czm[k];
         }
-        acc = __dadd_rn(acc, __dmul_rn(coef, lam[lin(i, j, k, L.sy, L.sz)]));
+        acc = __fma_rn(coef, lam[lin(i, j, k, L.sy, L.sz)], acc);
     }
     const double s = block_sum(acc, sw);
-    if (threadIdx.x == 0) out[f] = -s;
+    if (threadIdx.x == 0) {
+        partials[f * kFaceCtas + blockIdx.x] = s;
+        __threadfence();
+        s_last = atomicAdd(arrive + f, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (s_last && threadIdx.x == 0) {
+        double t = 0.0;
+        for (int q = 0; q < (int)gridDim.x; ++q) t = __dadd_rn(t, __ldcg(partials + f * kFaceCtas + q));
+        out[f] = -t;
+        arrive[f] = 0;
+    }
 }
 
 }  // namespace
@@ -104,7 +140,7 @@ int Ctx::adjoint(const double *dLdu, double *dLdb, double *dLdg, int maxit, doub
         // later call starts again instead of finding a partial set
         double *a[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
         const size_t sz[5] = {bytes, bytes, bytes, (S.n[0] + S.n[1] + S.n[2] + 6) * sizeof(double),
-                              6 * sizeof(double)};
+                              (6 + 6 * kFaceCtas) * sizeof(double) + 6 * sizeof(unsigned)};
         int st = PMG_OK;
         for (int q = 0; q < 5 && st == PMG_OK; ++q) st = cuda_status(dev_malloc(&a[q], sz[q]), "adjoint allocation");
         if (st == PMG_OK) {
@@ -112,6 +148,7 @@ int Ctx::adjoint(const double *dLdu, double *dLdb, double *dLdg, int maxit, doub
             for (int d = 0; d < 3; ++d) h.insert(h.end(), S.dm[d].begin(), S.dm[d].end());
             st = cuda_status(cudaMemcpy(a[3], h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice),
                              "adjoint tables");
+            if (st == PMG_OK) st = cuda_status(cudaMemset(a[4], 0, sz[4]), "adjoint counters");
         }
         if (st != PMG_OK) {
             for (auto p : a) dev_free(p);
@@ -124,18 +161,32 @@ int Ctx::adjoint(const double *dLdu, double *dLdb, double *dLdg, int maxit, doub
         adj_faces = a[4];
     }
     const double *dxm = adj_vol, *dym = adj_vol + S.n[0] + 2, *dzm = dym + S.n[1] + 2;
-    const dim3 g((S.n[0] + kBX - 1) / kBX, (S.n[1] + kBY - 1) / kBY, std::min(S.n[2], 65535)), bl(kBX, kBY, 1);
+    const dim3 g = grid_columns(S.n[0], S.n[1], S.n[2], Launch{{false, false, false}}, 4), bl(kBX, kBY, 1);
+    bool in_range = true;     // the widths' products fit mul64's factors
+    for (int d = 0; d < 3; ++d) in_range = in_range && exponents_within(S.dm[d].data() + 1, S.n[d], 120);
     PMG_TRY_A(cuda_status(cudaMemsetAsync(adj_rhs, 0, bytes, stream), "adjoint init"));
     PMG_TRY_A(cuda_status(cudaMemsetAsync(adj_sol, 0, bytes, stream), "adjoint init"));
-    k_volume_scale<<<g, bl, 0, stream>>>(S.n[0], S.n[1], S.n[2], S.sy, S.sz, dxm, dym, dzm, dLdu, adj_rhs, 0);
+    if (in_range)
+        k_volume_scale<true, true>
+            <<<g, bl, 0, stream>>>(S.n[0], S.n[1], S.n[2], S.sy, S.sz, dxm, dym, dzm, dLdu, adj_rhs);
+    else
+        k_volume_scale<true, false>
+            <<<g, bl, 0, stream>>>(S.n[0], S.n[1], S.n[2], S.sy, S.sz, dxm, dym, dzm, dLdu, adj_rhs);
     count_launches(1);
     PMG_TRY_A(cuda_status(cudaGetLastError(), "adjoint rhs"));
     const int rc = precision == PMG_MIXED ? solve_mixed(adj_sol, adj_rsd, adj_rhs, maxit, tol, omega, rep)
                                           : solve_f64(adj_sol, adj_rsd, adj_rhs, maxit, tol, omega, rep);
     if (rc != PMG_OK) return rc;
     PMG_TRY_A(cuda_status(cudaMemsetAsync(dLdb, 0, bytes, stream), "adjoint output"));
-    k_volume_scale<<<g, bl, 0, stream>>>(S.n[0], S.n[1], S.n[2], S.sy, S.sz, dxm, dym, dzm, adj_sol, dLdb, 1);
-    k_face_gradients<<<6, 1024, 0, stream>>>(K[0], dLdb, adj_faces);
+    if (in_range)
+        k_volume_scale<false, true>
+            <<<g, bl, 0, stream>>>(S.n[0], S.n[1], S.n[2], S.sy, S.sz, dxm, dym, dzm, adj_sol, dLdb);
+    else
+        k_volume_scale<false, false>
+            <<<g, bl, 0, stream>>>(S.n[0], S.n[1], S.n[2], S.sy, S.sz, dxm, dym, dzm, adj_sol, dLdb);
+    double *face_part = adj_faces + 6;
+    k_face_gradients<<<dim3(kFaceCtas, 6), 256, 0, stream>>>(
+        K[0], dLdb, face_part, reinterpret_cast<unsigned *>(face_part + 6 * kFaceCtas), adj_faces);
     count_launches(2);
     PMG_TRY_A(cuda_status(cudaGetLastError(), "adjoint gradients"));
     if (dLdg) {

@@ -439,7 +439,7 @@ bool host_setup()
 // an even length (16-byte alignment).
 // Every v[0..n) positive, finite and within 2^+-e: what the integer-pipe products of the FP64
 // kernels (pmg_mul64.cuh) ask of a level's tables.
-static bool exponents_within(const double *v, int n, int e)
+bool exponents_within(const double *v, int n, int e)
 {
     for (int i = 0; i < n; ++i)
         if (!(v[i] > 0.0) || !std::isfinite(v[i]) || std::abs(std::ilogb(v[i])) > e) return false;

@@ -44,7 +44,7 @@ __device__ __forceinline__ int block_lin()
 // instruction and SM), so kInt takes the products off it: an RBGS update keeps 8 of 21 FP64
 // instructions (15 with the reciprocal alone), a residual 7 of 14, A p with its dot product 7
 // of 16.  Measured: a half-sweep at 384^3 1.15 -> 0.53 ms, a residual at 324 x 258 x 194 0.474
-// -> 0.252 ms, A p at 224 x 160 x 128 159 -> 103 us; the FP64 unit is 80% busy in the sweep.
+// -> 0.246 ms, A p at 224 x 160 x 128 159 -> 103 us; the FP64 unit is 80% busy in the sweep.
 enum ArithMode { kPlain = 0, kTab = 1, kInt = 2 };
 
 template <int MODE>
@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(kBX *kBY) k_diag_f64(LevelK<double> L, double 
 
 // r = b - A x on the interior (src/multigrid.f90:1795-1805); optional per-block sum of r^2.
 template <bool NORM, int MODE>
-__global__ void __launch_bounds__(kBX *kBY) k_residual_f64(LevelK<double> L, double *__restrict__ r,
+__global__ void __launch_bounds__(kBX *kBY, 6) k_residual_f64(LevelK<double> L, double *__restrict__ r,
                                                            const double *__restrict__ x,
                                                            const double *__restrict__ b, double *partials,
                                                            const double *__restrict__ c0t)
@@ -194,9 +194,10 @@ __global__ void __launch_bounds__(1024) k_reduce_f64(const double *__restrict__ 
 // A thread takes the coarse cells of one column (i, j) over a chunk of planes, so the weights'
 // x-y products are formed once, and the full weights, their sum and its reciprocal only where
 // the plane's weights change: on a uniform z axis a coarse cell keeps 9 of 43 FP64
-// instructions (324 x 258 x 194, stretched: 192 -> 122 us).
+// instructions (324 x 258 x 194, stretched: 192 -> 99 us; at 64 registers, four CTAs an SM, and
+// 106 at the 108 it would take).
 template <bool M64>
-__global__ void __launch_bounds__(kBX *kBY) k_restrict_f64(XferK<double> X, const double *__restrict__ vf,
+__global__ void __launch_bounds__(kBX *kBY, 4) k_restrict_f64(XferK<double> X, const double *__restrict__ vf,
                                                            double *__restrict__ vc)
 {
     int k0, k1;
@@ -249,9 +250,10 @@ __global__ void __launch_bounds__(kBX *kBY) k_restrict_f64(XferK<double> X, cons
 // and its reciprocal only where the plane's weights change, which on a uniform z axis is at
 // the chunk's first plane and at the boundaries.  A fine cell then keeps 10 (14 where the
 // weights change) of about 40 FP64 instructions; where they change the integer products (19)
-// bound it.  324 x 258 x 194, stretched: 1.43 -> 0.60 ms.  Terms and order: prolong_child_f64.
+// bound it.  324 x 258 x 194, stretched: 1.43 -> 0.51 ms (0.58 at 128 registers: more warps
+// overlap the two pipes better).  Terms and order: prolong_child_f64.
 template <bool ADD>
-__global__ void __launch_bounds__(kBX *kBY) k_prolong_m64(XferK<double> X, const double *__restrict__ vc,
+__global__ void __launch_bounds__(kBX *kBY, 4) k_prolong_m64(XferK<double> X, const double *__restrict__ vc,
                                                           double *__restrict__ vf)
 {
     const int nfx = X.ncx * X.stx, nfy = X.ncy * X.sty, nfz = X.ncz * X.stz;

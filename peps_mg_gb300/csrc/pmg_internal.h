@@ -101,6 +101,7 @@ struct HierDesc {
     long long ps[kMaxLevels][3], pr[kMaxLevels][3];
 };
 
+bool exponents_within(const double *v, int n, int e);   // pmg_api.cu
 // Grid of the FP64 column kernels (32 x 8 threads, plane_chunk), pmg_f64.cu.
 dim3 grid_columns(int nx_threads, int ny, int nz, const Launch &ln, int kc_min = 1, bool sum = false);
 
