@@ -83,3 +83,21 @@ def test_level_operations(n, mesh, value):
         got = to_dev(x)
         mg.prolong_add(0, got, to_dev(xc))
         assert same(from_dev(got)[inner], want)
+
+
+@pytest.mark.parametrize("nz", [4, 5, 180, 182])
+def test_diagonal_of_a_column(nz):
+    """The tables of the diagonal where a z axis changes its spacing now and then, within one
+    chunk of planes and across two, against the oracle's sweep."""
+    n = (96, 80, nz)
+    rng = np.random.Generator(np.random.PCG64(nz))
+    w = np.repeat(rng.uniform(0.5, 1.5, nz), rng.integers(1, 6, nz))[:nz] / nz
+    axes = [G.uniform_axis(n[0], 0.0, 1.0), G.mesh_from_widths(rng.uniform(0.5, 1.5, n[1]) / n[1]),
+            G.mesh_from_widths(w)]
+    x, b = (np.asfortranarray(rng.uniform(-1.0, 1.0, tuple(m + 2 for m in n))) for _ in range(2))
+    want = x.copy(order="F")
+    O.rbgs_iterator(O.matrix_create(axes), want, b, 1, 1.0)
+    with pmg.Multigrid(axes, 2, 1) as mg:
+        got = to_dev(x)
+        mg.rbgs_iterator(0, got, to_dev(b), 1, 1.0)
+    assert same(from_dev(got), want)
