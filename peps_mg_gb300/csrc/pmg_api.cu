@@ -867,6 +867,20 @@ bool Ctx::coop64_level_ok(int l, long long cells) const
     return (long long)n[0] * n[1] * n[2] <= cells && std::max(n[0], std::max(n[1], n[2])) <= 4096 && K[l].mul64;
 }
 
+// The barrier counters belong to the context, so its cooperative launches may not overlap: not
+// where a graph of them could be replayed beside another, and not on the handle that names
+// another stream in every thread.
+bool Ctx::launches_in_order() const
+{
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (stream == cudaStreamPerThread) return false;
+    if (cudaStreamIsCapturing(stream, &st) != cudaSuccess) {
+        cudaGetLastError();   // the legacy stream beside a capture; the launches report it
+        return false;
+    }
+    return st == cudaStreamCaptureStatusNone;
+}
+
 Coop64Level Ctx::coop64_level(int l) const
 {
     Coop64Level V;
@@ -1739,7 +1753,8 @@ int pmg_rbgs_iterator(pmg_ctx *ctx, int level, double *x, const double *b, int m
     PMG_TRY(check_ctx_level(ctx, level));
     Ctx &c = ctx->impl;
     // several half-sweeps of a small level in one launch
-    if (c.coop_grid > 0 && maxiteration >= 2 && c.coop64_level_ok(level, pmg::kCoop64SweepCells))
+    if (c.coop_grid > 0 && maxiteration >= 2 && c.coop64_level_ok(level, pmg::kCoop64SweepCells) &&
+        c.launches_in_order())
         return pmg::coop64_sweeps(c.coop64_level(level), c.coop_grid, x, b, maxiteration, omega, c.d_bar,
                                   c.d_iscal + 8, c.stream);
     return pmg::f64_rbgs_sweeps(c.K[level], c.launch[level], x, b, maxiteration, omega, c.stream, c.diag(level));

@@ -80,6 +80,7 @@ struct Ctx {
     int upload_coop64(int maxit, double omega, double tol);
     int check_coop64();
     bool coop64_level_ok(int l, long long cells) const;
+    bool launches_in_order() const;
     Coop64Level coop64_level(int l) const;
     int fetch_cycle(double *rsd_val, int *coarse_iters);
     double *d_partials = nullptr;

@@ -1,7 +1,7 @@
 """The cooperative launch of the small FP64 levels (pmg_coop64.cu) against the oracle, bit for
 bit: whole solves whose finest level is inside it (the norm too), on its limit or above, with
 one to three sweeps, stride-1 transfers, stretched meshes and Dirichlet faces; and smoother
-calls on boxes beside the limit of the one-launch sweeps."""
+calls on boxes beside the limit of the one-launch sweeps, also captured in graphs."""
 import numpy as np
 import pytest
 
@@ -55,3 +55,30 @@ def test_sweeps(n, iters, omega):
         mg.rbgs_iterator(0, x, to_dev(rhs), iters, omega)
         mg.sync()
     assert np.array_equal(from_dev(x), want)
+
+
+def test_sweeps_captured():
+    """Two graphs of a context's sweeps, replayed at once on two streams."""
+    n = (32, 24, 16)
+    mesh, rhs, sol0 = box(n, 5)
+    coeff = O.matrix_create(mesh)
+    streams = [torch.cuda.Stream() for _ in range(3)]
+    b, xs, wants, graphs = to_dev(rhs), [], [], []
+    with pmg.Multigrid(mesh, 2, 1, stream=streams[0].cuda_stream) as mg:
+        for iters in (2, 5):
+            x, g = to_dev(sol0), torch.cuda.CUDAGraph()
+            torch.cuda.synchronize()
+            with torch.cuda.graph(g, stream=streams[0]):
+                mg.rbgs_iterator(0, x, b, iters, 1.0)
+            want = sol0.copy(order="F")
+            O.rbgs_iterator(coeff, want, rhs, 3 * iters, 1.0)
+            xs, wants, graphs = xs + [x], wants + [want], graphs + [g]
+        torch.cuda.synchronize()
+        for _ in range(3):
+            for g, s in zip(graphs, streams[1:]):
+                with torch.cuda.stream(s):
+                    g.replay()
+        torch.cuda.synchronize()
+        mg.sync()
+    for x, want in zip(xs, wants):
+        assert np.array_equal(from_dev(x), want)
