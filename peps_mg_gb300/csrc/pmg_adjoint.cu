@@ -45,9 +45,9 @@ constexpr int kBX = 32, kBY = 8;
 
 // out = in / vol on the interior (DIV) or vol * in, vol = dxm(i) dym(j) dzm(k).  A thread takes a
 // column over a chunk of planes and forms vol and its reciprocal where the plane's width
-// changes; INT (widths within mul64's range) then leaves 2 FP64 instructions of a division's 11
-// and none of a product's, with the same bits (quot64, pmg_mul64.cuh).  256^3: 201 -> 111 us
-// (a division), 201 -> 70 (a product).
+// changes; INT (widths within mul64's range) then leaves no FP64 instruction of a division or a
+// product, with the same bits (quot64, mul64, pmg_mul64.cuh).  256^3: 201 -> 91 us (a
+// division), 201 -> 70 (a product).
 template <bool DIV, bool INT>
 __global__ void __launch_bounds__(kBX *kBY) k_volume_scale(int nx, int ny, int nz, int sy, long long sz,
                                                            const double *__restrict__ dxm,
@@ -60,7 +60,8 @@ __global__ void __launch_bounds__(kBX *kBY) k_volume_scale(int nx, int ny, int n
     for (int j = blockIdx.y * blockDim.y + threadIdx.y + 1; j <= ny; j += gridDim.y * blockDim.y)
         for (int i = blockIdx.x * blockDim.x + threadIdx.x + 1; i <= nx; i += gridDim.x * blockDim.x) {
             const double area = __dmul_rn(dxm[i], dym[j]);
-            double dz = 0.0, vol = 1.0, y = 1.0;
+            double dz = 0.0, vol = 1.0;
+            unsigned long long y = 0;
             Mul64 f = mul64_factor(1.0);
             for (int k = k0; k <= k1; ++k) {
                 const long long p = lin(i, j, k, sy, sz);
@@ -68,7 +69,7 @@ __global__ void __launch_bounds__(kBX *kBY) k_volume_scale(int nx, int ny, int n
                 if (k == k0 || __double_as_longlong(dzm[k]) != __double_as_longlong(dz)) {
                     dz = dzm[k];
                     vol = __dmul_rn(area, dz);
-                    if (INT && DIV) y = recip_f64(vol);
+                    if (INT && DIV) y = recip64(vol);
                     if (INT) f = mul64_factor(vol);
                 }
                 if (DIV)

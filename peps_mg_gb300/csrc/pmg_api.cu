@@ -779,7 +779,7 @@ int Ctx::build(const pmg_config_t *c, cudaStream_t s)
     if (precision == PMG_FP64) {
         // per-cell diagonal tables of the plain FP64 path and of its reciprocal (the grid
         // kernels read c0 instead of summing five 1-D table entries per cell, the values are
-        // diag_f64's bits, and divide by it with two FMAs)
+        // diag_f64's bits, and divide by it on the integer pipe)
         c0t.assign((size_t)nl + 1, nullptr);
         for (int l = 0; l <= nl; ++l) {
             PMG_CUDA(dev_malloc(&c0t[l], 2 * lv[l].total * sizeof(double)), "diagonal table");

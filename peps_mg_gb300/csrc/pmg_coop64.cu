@@ -48,11 +48,6 @@ __device__ __forceinline__ double prod(double c, double x)
 {
     return INT ? mul64(mul64_factor(c), x) : __dmul_rn(c, x);
 }
-template <bool INT>
-__device__ __forceinline__ double quot(double d, double c, double y)
-{
-    return INT ? quot64(d, c, y) : quot64_dp(d, c, y);
-}
 
 // c1 x(i-1) + ... + c6 x(k+1) onto t0 (the residual's c0 x), or from the first product
 template <class M, bool INT, bool DIAG>
@@ -98,9 +93,10 @@ __device__ __forceinline__ void half_sweep(const Coop64Level &V, double *x, cons
     const bool omega1 = omega == 1.0;
     auto update = [&](int p, double s, double old) {
         const double d = __dsub_rn(M::ld(b + p), s);
-        const double c0 = c0t[p], y = rc[p];
-        x[p] = omega1 ? add_zero_times_f64(quot<INT>(d, c0, y), old)
-                      : __dadd_rn(quot<INT>(__dmul_rn(omega, d), c0, y), __dmul_rn(omw, old));
+        const double c0 = c0t[p];
+        const unsigned long long y = (unsigned long long)__double_as_longlong(rc[p]);
+        x[p] = omega1 ? add_zero_times_f64(quot64(d, c0, y), old)
+                      : __dadd_rn(quot64(__dmul_rn(omega, d), c0, y), __dmul_rn(omw, old));
     };
     if (first) {
         cells(V, q0, step, [&](int i, int j, int k, int p) {

@@ -41,10 +41,11 @@ __device__ __forceinline__ int block_lin()
 //          reciprocal: levels whose coefficients fit mul64's range, which all but meshes with
 //          spacings beyond 2^+-190 do.
 // The bits are the same.  These kernels are bound by the FP64 unit (19 clocks per warp
-// instruction and SM), so kInt takes the products off it: an RBGS update keeps 8 of 21 FP64
-// instructions (15 with the reciprocal alone), a residual 7 of 14, A p with its dot product 7
-// of 16.  Measured: a half-sweep at 384^3 1.15 -> 0.53 ms, a residual at 324 x 258 x 194 0.474
-// -> 0.246 ms, A p at 224 x 160 x 128 159 -> 103 us; the FP64 unit is 80% busy in the sweep.
+// instruction and SM), so kInt takes the products and the quotient off it: an RBGS update keeps
+// 6 of 21 FP64 instructions, a residual 7 of 14, A p with its dot product 7 of 16.  Measured: a
+// half-sweep at 384^3 1.15 -> 0.44 ms (0.53 with two FMAs of the quotient left on it), a
+// residual at 324 x 258 x 194 0.474 -> 0.247 ms, A p at 224 x 160 x 128 159 -> 103 us; the
+// sweep keeps the FP64 unit 73% busy.
 enum ArithMode { kPlain = 0, kTab = 1, kInt = 2 };
 
 template <int MODE>
@@ -52,6 +53,11 @@ __device__ __forceinline__ double diag_at(const LevelK<double> &L, const double 
                                           int k)
 {
     return MODE != kPlain ? c0t[p] : diag_f64(L, i, j, k);
+}
+
+__device__ __forceinline__ unsigned long long recip_at(const double *t, long long p)
+{
+    return (unsigned long long)__double_as_longlong(t[p]);
 }
 
 template <int MODE>
@@ -92,8 +98,9 @@ __device__ __forceinline__ void each_cell(const LevelK<double> &L, F f)
 // One colour of the red-black sweep.  colour 0 is the reference's first half-sweep:
 // ista = 1 + mod(j+k, 2) (src/rbgs_poisson_matrix.f90:242); colour 1 the second
 // (:260).  Thread t of a row updates i = 2t + ista.
+// 7 CTAs per SM where the products are integer ones: 440 us at 384^3, 445 with 6, 468 with 5.
 template <int MODE, bool OMEGA1>
-__global__ void __launch_bounds__(kBX *kBY) k_rbgs_f64(LevelK<double> L, double *__restrict__ x,
+__global__ void __launch_bounds__(kBX *kBY, MODE == kInt ? 7 : 6) k_rbgs_f64(LevelK<double> L, double *__restrict__ x,
                                                        const double *__restrict__ b, double omega, double omw,
                                                        int colour, const double *__restrict__ c0t)
 {
@@ -115,9 +122,9 @@ __global__ void __launch_bounds__(kBX *kBY) k_rbgs_f64(LevelK<double> L, double 
                     s = __dadd_rn(s, prod<MODE>(L.czp[k], x[p + L.sz]));
                     const double d = __dsub_rn(b[p], s);
                     if (OMEGA1)
-                        x[p] = add_zero_times_f64(quot64(d, c0t[p], c0t[p + total]), x[p]);
+                        x[p] = add_zero_times_f64(quot64(d, c0t[p], recip_at(c0t, p + total)), x[p]);
                     else
-                        x[p] = __dadd_rn(quot64(mul64_vv(omega, d), c0t[p], c0t[p + total]), mul64_vv(omw, x[p]));
+                        x[p] = __dadd_rn(quot64(mul64_vv(omega, d), c0t[p], recip_at(c0t, p + total)), mul64_vv(omw, x[p]));
                 } else {
                     x[p] = rbgs_cell_c0_f64<OMEGA1>(L, x, b, i, j, k, omega, omw, diag_at<MODE>(L, c0t, p, i, j, k));
                 }
@@ -125,9 +132,10 @@ __global__ void __launch_bounds__(kBX *kBY) k_rbgs_f64(LevelK<double> L, double 
 }
 
 // c0t = the diagonal of every interior cell (diag_f64), then as many values again its
-// reciprocals (recip_f64); the ghosts are left as they are.  A thread marches its column of
+// reciprocals (recip64); the ghosts are left as they are.  A thread marches its column of
 // planes and forms the two values anew only where the plane's z coefficients differ from
-// those of the plane before: on a uniform z axis once a chunk.  A context of 384^3 is then created in 2.48 ms, 2.39 without the reciprocals.
+// those of the plane before: on a uniform z axis once a chunk.  A context of 384^3 is then
+// created in 2.48 ms, 2.39 without the reciprocals.
 __global__ void __launch_bounds__(kBX *kBY) k_diag_f64(LevelK<double> L, double *__restrict__ c0t)
 {
     const long long total = L.sz * (L.nz + 2);
@@ -135,12 +143,12 @@ __global__ void __launch_bounds__(kBX *kBY) k_diag_f64(LevelK<double> L, double 
     plane_chunk(L.nz, k0, k1);
     for (int j = blockIdx.y * blockDim.y + threadIdx.y + 1; j <= L.ny; j += gridDim.y * blockDim.y)
         for (int i = blockIdx.x * blockDim.x + threadIdx.x + 1; i <= L.nx; i += gridDim.x * blockDim.x) {
-            double c0 = 0.0, y = 0.0;
+            double c0 = 0.0, y = 0.0;   // y: the bits of recip64
             for (int k = k0; k <= k1; ++k) {
                 if (k == k0 || __double_as_longlong(L.czm[k]) != __double_as_longlong(L.czm[k - 1]) ||
                     __double_as_longlong(L.czp[k]) != __double_as_longlong(L.czp[k - 1])) {
                     c0 = diag_f64(L, i, j, k);
-                    y = recip_f64(c0);
+                    y = __longlong_as_double((long long)recip64(c0));
                 }
                 const long long p = lin(i, j, k, L.sy, L.sz);
                 c0t[p] = c0;
@@ -225,7 +233,8 @@ __global__ void __launch_bounds__(kBX *kBY, 4) k_restrict_f64(XferK<double> X, c
             // child c of a plane: (ip|iz, jp|jz) in the reference's order (restrict_cell_f64)
             const long long o[4] = {lin(ip, jp, 0, X.fsy, X.fsz), lin(iz, jp, 0, X.fsy, X.fsz),
                                     lin(ip, jz, 0, X.fsy, X.fsz), lin(iz, jz, 0, X.fsy, X.fsz)};
-            double wz0 = 0.0, wz1 = 0.0, vol = 1.0, y = 1.0;
+            double wz0 = 0.0, wz1 = 0.0, vol = 1.0;
+            unsigned long long y = 0;
             Mul64 w[8];
             for (int k = k0; k <= k1; ++k) {
                 const int kp = k * X.stz, kz = kp - (X.stz - 1);
@@ -240,7 +249,7 @@ __global__ void __launch_bounds__(kBX *kBY, 4) k_restrict_f64(XferK<double> X, c
                         vol = c == 0 ? v : __dadd_rn(vol, v);
                         w[c] = mul64_factor(v);
                     }
-                    y = recip_f64(vol);
+                    y = recip64(vol);
                 }
                 // v11* meets the plane kp's children first (src/multigrid.f90:1483-1490)
                 double v[8], s[8];

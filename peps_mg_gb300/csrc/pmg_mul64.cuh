@@ -7,7 +7,8 @@
 // place, a round-up by the carry of the first dropped bit): 13 to 17 clocks per SM that
 // overlap with the FP64 unit's (measured: 7 products and 8 additions per cell 167 clocks
 // instead of 300).  So the kernels below form their products here and leave the FP64 unit
-// the additions and the two FMAs of a division.
+// the additions.  A quotient is such a product too, with 64 bits of the divisor's reciprocal
+// (quot64).
 //
 // mul64(f, x) returns RN(f x) for every double x, f a factor decoded once by mul64_factor:
 //  * x normal with an exponent within 2^+-500, f's exponent within 2^+-400 (the callers
@@ -61,12 +62,13 @@ __device__ __forceinline__ bool mul64_factor_ok(double f)
 
 __device__ __forceinline__ bool is_zero64(unsigned xh, unsigned xl) { return ((xh << 1) | xl) == 0u; }
 
-// f x for x in range.
-__device__ __forceinline__ double mul64_core(const Mul64 &f, unsigned xh, unsigned xl)
+// The product of f's 64-bit significand and x's 53-bit one: its leading 53 bits in (h1, h0),
+// the next 32 in m1; top, the place in h1 that tells whether it reached bit 116.
+__device__ __forceinline__ void mul64_words(const Mul64 &f, unsigned xh, unsigned xl, unsigned &m1, unsigned &h0,
+                                            unsigned &h1, unsigned &top)
 {
     const unsigned mh = (xh & 0xfffffu) | 0x100000u;
-    // words 1, 2 and 3 of the 128-bit product (m1, h0, h1); word 0 only settles ties
-    unsigned m1, h0, h1;
+    // words 1, 2 and 3 of the 128-bit product (m1, h0, h1)
     {
         const unsigned p0h = __umulhi(xl, f.l), p1l = xl * f.h, p1h = __umulhi(xl, f.h);
         const unsigned p2l = mh * f.l, p2h = __umulhi(mh, f.l), p3l = mh * f.h, p3h = __umulhi(mh, f.h);
@@ -80,23 +82,36 @@ __device__ __forceinline__ double mul64_core(const Mul64 &f, unsigned xh, unsign
             : "r"(p0h), "r"(p1l), "r"(p1h), "r"(p3l), "r"(p3h), "r"(p2l), "r"(p2h));
     }
     // the significand is bits 52 .. 0 of (h1, h0) when bit 52 is set, else one place lower
-    const unsigned top = h1 & 0x100000u;
+    top = h1 & 0x100000u;
     if (!top) {
         h1 = __funnelshift_l(h0, h1, 1);
         h0 = __funnelshift_l(m1, h0, 1);
         m1 <<= 1;
     }
-    // the first dropped bit rounds up, except on a tie (word 0 zero too) with an even
-    // significand; factors of few bits, such as those of uniform meshes, tie often
-    if (m1 == 0x80000000u && (h0 & 1u) == 0u && xl * f.l == 0u) m1 = 0u;
+}
+
+// The double of significand (h1, h0), rounded up where m1 >= 2^31, and sign and exponent e.
+__device__ __forceinline__ double mul64_round(unsigned m1, unsigned h0, unsigned h1, unsigned e)
+{
     unsigned rl, rh;
     asm("{\n\t.reg .u32 t;\n\t"
         "add.cc.u32 t, %2, 0x80000000;\n\t"
         "addc.cc.u32 %0, %3, 0;\n\t"
         "addc.u32 %1, %4, %5;\n\t}"
         : "=&r"(rl), "=r"(rh)
-        : "r"(m1), "r"(h0), "r"(h1), "r"((xh & 0xfff00000u) + f.e + top));
+        : "r"(m1), "r"(h0), "r"(h1), "r"(e));
     return __hiloint2double((int)rh, (int)rl);
+}
+
+// f x for x in range.
+__device__ __forceinline__ double mul64_core(const Mul64 &f, unsigned xh, unsigned xl)
+{
+    unsigned m1, h0, h1, top;
+    mul64_words(f, xh, xl, m1, h0, h1, top);
+    // the first dropped bit rounds up, except on a tie (word 0 zero too) with an even
+    // significand; factors of few bits, such as those of uniform meshes, tie often
+    if (m1 == 0x80000000u && (h0 & 1u) == 0u && xl * f.l == 0u) m1 = 0u;
+    return mul64_round(m1, h0, h1, (xh & 0xfff00000u) + f.e + top);
 }
 
 __device__ __forceinline__ double mul64(const Mul64 &f, double x)
@@ -155,24 +170,53 @@ __device__ __forceinline__ double mul64_vv(double a, double b)
     return r;
 }
 
-// d / c with y = recip_f64(c) (pmg_common.cuh: why the bits are the division's).
-__device__ __forceinline__ double quot64(double d, double c, double y)
+// Y = floor(2^116 / C), C the 53-bit significand of c: the leading 64 bits of c's reciprocal,
+// for quot64; 0 if c's exponent lies beyond 2^+-400, and 2^64 - 1 for 2^64 (c a power of two).
+__device__ __forceinline__ unsigned long long recip64(double c)
+{
+    const unsigned long long one = 1ULL << 52;
+    const unsigned long long C = ((unsigned long long)__double_as_longlong(c) & (one - 1)) | one;
+    const unsigned e = ((unsigned)__double2hiint(c) >> 20) & 0x7ffu;
+    // RN(1/c) is within 2^10 of it, so 2^116 - Y0 C fits 64 bits
+    const double y = __drcp_rn(c);
+    const unsigned long long Y0 = (((unsigned long long)__double_as_longlong(y) & (one - 1)) | one) << 11;
+    const long long r = -(long long)(Y0 * C);
+    long long t = (long long)__float2int_rd(__fmul_rn(__ll2float_rn(r), __frcp_rn(__ull2float_rn(C))));
+    const long long rest = r - t * (long long)C;
+    t += rest < 0 ? -1 : rest >= (long long)C ? 1 : 0;
+    if (e - 623u > 800u) return 0ULL;
+    return C == one ? ~0ULL : Y0 + (unsigned long long)t;
+}
+
+// d / c with Y = recip64(c).  With D the significand of d, D Y lies below the quotient's 117 bits
+// D 2^116 / C by at most D < 2^53, so its leading 53 bits round as the quotient's do unless the
+// bits that follow lie just below a half: 2^54 of 2^64 places, which take the IEEE division as
+// operands out of range do.  A quotient is never half way itself, and D Y is below it, so a
+// half rounds up.  A product with RN(1/c) and two FMAs (quot64_dp) took the FP64 unit 38 clocks
+// a warp.
+__device__ __forceinline__ double quot64(double d, double c, unsigned long long Y)
 {
     const unsigned dh = (unsigned)__double2hiint(d), dl = (unsigned)__double2loint(d);
-    const double q0 = mul64_core(mul64_factor(y), dh, dl);
-    const double r = __fma_rn(-c, q0, d);
-    double q = __fma_rn(r, y, q0);
-    if (!mul64_in_range(dh) || ((unsigned)__double2hiint(y) & 0x7ff00000u) == 0x7ff00000u) {
-        if (is_zero64(dh, dl) && ((unsigned)__double2hiint(y) & 0x7ff00000u) != 0x7ff00000u)
-            q = __hiloint2double((int)((dh ^ (unsigned)__double2hiint(c)) & 0x80000000u), 0);
+    const unsigned ch = (unsigned)__double2hiint(c);
+    Mul64 f;
+    f.h = (unsigned)(Y >> 32);
+    f.l = (unsigned)Y;
+    f.e = (1021u << 20) - (ch & 0xfff00000u);
+    unsigned m1, h0, h1, top;
+    mul64_words(f, dh, dl, m1, h0, h1, top);
+    double q = mul64_round(m1, h0, h1, (dh & 0xfff00000u) + f.e + top);
+    if (!mul64_in_range(dh) || (int)f.h >= 0 || 0x7fffffffu - m1 < 0x400002u) {
+        if (is_zero64(dh, dl) && (int)f.h < 0)
+            q = __hiloint2double((int)((dh ^ ch) & 0x80000000u), 0);
         else
             q = div64_slow(d, c);
     }
     return q;
 }
 
-// The same on the FP64 unit: three instructions instead of about forty, where a warp runs
-// alone and its instructions have to be fetched.
+// d / c on the FP64 unit with y = recip_f64(c) (pmg_common.cuh: why the bits are the
+// division's): three instructions instead of about forty, where a warp runs alone and its
+// instructions have to be fetched.
 __device__ __forceinline__ double quot64_dp(double d, double c, double y)
 {
     const unsigned dh = (unsigned)__double2hiint(d);

@@ -81,3 +81,44 @@ def test_quotient_is_correctly_rounded(kind):
 def test_reciprocal_table_rejects_the_exceptional_divisor():
     """The divisor with all mantissa bits set: its reciprocal lies next to a midpoint."""
     assert recip(Fraction(2 ** 53 - 1, 2 ** 52)) is None
+
+
+def quot_by_bits(D, C):
+    """quot64 on 53-bit significands: the quotient's significand (53 bits) and its exponent
+    less 52, or None where the kernel takes the IEEE division."""
+    Y = min(2 ** 116 // C, 2 ** 64 - 1)
+    y0 = int(rn(Fraction(2 ** 116, C)))          # the kernel's start: 2^10 away at most
+    assert C == 2 ** 52 or abs(2 ** 116 - y0 * C) < 2 ** 63
+    P, e = D * Y, 0
+    if P < 2 ** 116:
+        P, e = 2 * P, -1
+    q, m1 = P >> 64, P >> 32 & 0xffffffff
+    if e:
+        m1 &= 0xfffffffe                         # the shift brings no bit of word 0 in
+    if 0x7fffffff - 0x400002 < m1 <= 0x7fffffff:
+        return None
+    return (q + (m1 >> 31)) * Fraction(2) ** (e - 52)
+
+
+@pytest.mark.parametrize("kind", ["random", "boundary", "extreme", "short"])
+def test_quotient_by_integers(kind):
+    rng = np.random.Generator(np.random.PCG64(13))
+    one = 2 ** 52
+    if kind == "random":
+        pairs = [(int(a), int(b)) for a, b in rng.integers(one, 2 * one, size=(4000, 2))]
+    elif kind == "boundary":
+        pairs = [(int(d * one), int(c * one)) for d, c in near_boundary(rng, 4000)]
+    elif kind == "extreme":
+        ends = [one + k for k in range(12)] + [2 * one - 1 - k for k in range(12)]
+        ends += [3 * one // 2 + k for k in range(-3, 4)]
+        pairs = [(a, b) for a in ends for b in ends]
+    else:                                        # few bits: exact quotients and periodic ones
+        few = [int(v) << (53 - int(v).bit_length()) for v in range(1, 80)]
+        pairs = [(a, b) for a in few for b in few]
+    left = 0
+    for D, C in pairs:
+        q = quot_by_bits(D, C)
+        left += q is None
+        assert q is None or q == rn(Fraction(D, C)), (D, C)
+    if kind in ("random", "short"):
+        assert left <= len(pairs) // 100         # about one in a thousand takes the division
