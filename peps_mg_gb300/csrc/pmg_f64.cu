@@ -43,7 +43,7 @@ __device__ __forceinline__ int block_lin()
 // The bits are the same.  These kernels are bound by the FP64 unit (19 clocks per warp
 // instruction and SM), so kInt takes the products and the quotient off it: an RBGS update keeps
 // 6 of 21 FP64 instructions, a residual 7 of 14, A p with its dot product 7 of 16.  Measured: a
-// half-sweep at 384^3 1.15 -> 0.44 ms (0.53 with two FMAs of the quotient left on it), a
+// half-sweep at 384^3 1.15 -> 0.435 ms (0.53 with two FMAs of the quotient left on it), a
 // residual at 324 x 258 x 194 0.474 -> 0.247 ms, A p at 224 x 160 x 128 159 -> 103 us; the
 // sweep keeps the FP64 unit 73% busy.
 enum ArithMode { kPlain = 0, kTab = 1, kInt = 2 };
@@ -676,6 +676,11 @@ dim3 grid3(int nx_threads, int ny, int nz, const Launch &ln)
 
 }  // namespace
 
+// Planes per chunk of a sweep, whose column shares little: 256^3 141.4 us a half-sweep with 8
+// (3.4 rounds of CTAs, the last one a third full), 135.4 with 3, 139.0 with 1; 384^3 438.8,
+// 434.8, 457.0.
+static constexpr int kSweepPlanes = 3;
+
 void grid_for_cells(const LevelK<double> &L, const Launch &ln, dim3 *grid, dim3 *block)
 {
     *grid = grid3(L.nx, L.ny, L.nz, ln);
@@ -683,16 +688,16 @@ void grid_for_cells(const LevelK<double> &L, const Launch &ln, dim3 *grid, dim3 
 }
 
 // The grid of the column kernels (each_cell and its kin): the tiles of the (i, j) plane and
-// chunks of planes, of at most 8 so that a thread's column set-up is shared, as long as the
+// chunks of planes, of at most kc_max so that a thread's column set-up is shared, as long as the
 // grid fills every SM a few times over.  kc_min: planes per chunk that pay for the set-up even
 // where they leave SMs with fewer CTAs (the prolongation's weights: 64^3, 4 planes).  sum: the
 // CTAs end with a block sum, 48 warp instructions on the FP64 unit (0.45 us an SM), so they are
 // fewer and longer (a CG update of 224 x 160 x 128: 65 -> 52 us with 1216 CTAs instead of 4864).
-dim3 grid_columns(int nx_threads, int ny, int nz, const Launch &ln, int kc_min, bool sum)
+dim3 grid_columns(int nx_threads, int ny, int nz, const Launch &ln, int kc_min, bool sum, int kc_most)
 {
     dim3 g = grid3(nx_threads, ny, nz, ln);
     if (ln.collapse[2]) return g;
-    const long long want = sum ? 152 * 8 : 152 * 16, kc_max = sum ? 64 : 8;
+    const long long want = sum ? 152 * 8 : 152 * 16, kc_max = sum ? 64 : kc_most;
     const long long ctas = (long long)g.x * g.y * nz;
     const int kc = (int)std::min(kc_max, std::max((long long)kc_min, ctas / want));
     const int gz = (nz + kc - 1) / kc;
@@ -734,7 +739,7 @@ int f64_rbgs_sweeps(const LevelK<double> &L, const Launch &ln, double *x, const 
                     double omega, cudaStream_t s, const double *c0t)
 {
     const double omw = 1.0 - omega;   // (1.0d0-omega), src/rbgs_poisson_matrix.f90:250
-    const dim3 g = grid_columns((L.nx + 1) / 2, L.ny, L.nz, ln);
+    const dim3 g = grid_columns((L.nx + 1) / 2, L.ny, L.nz, ln, 1, false, kSweepPlanes);
     for (int it = 0; it < iters; ++it)
         for (int c = 0; c < 2; ++c) launch_rbgs_colour(L, g, x, b, omega, omw, c, c0t, s);
     count_launches(2LL * iters);
@@ -744,7 +749,7 @@ int f64_rbgs_sweeps(const LevelK<double> &L, const Launch &ln, double *x, const 
 int f64_rbgs_colour(const LevelK<double> &L, const Launch &ln, double *x, const double *b, double omega, int colour,
                     cudaStream_t s, const double *c0t)
 {
-    const dim3 g = grid_columns((L.nx + 1) / 2, L.ny, L.nz, ln);
+    const dim3 g = grid_columns((L.nx + 1) / 2, L.ny, L.nz, ln, 1, false, kSweepPlanes);
     launch_rbgs_colour(L, g, x, b, omega, 1.0 - omega, colour & 1, c0t, s);
     count_launches(1);
     return cuda_status(cudaGetLastError(), "rbgs half-sweep");

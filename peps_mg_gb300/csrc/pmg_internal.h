@@ -103,7 +103,8 @@ struct HierDesc {
 
 bool exponents_within(const double *v, int n, int e);   // pmg_api.cu
 // Grid of the FP64 column kernels (32 x 8 threads, plane_chunk), pmg_f64.cu.
-dim3 grid_columns(int nx_threads, int ny, int nz, const Launch &ln, int kc_min = 1, bool sum = false);
+dim3 grid_columns(int nx_threads, int ny, int nz, const Launch &ln, int kc_min = 1, bool sum = false,
+                  int kc_max = 8);
 
 // ---- FP64 (bitwise) launchers, pmg_f64.cu -------------------------------------
 // Builds the coarse meshes (unless given) and every level's tables on the device.
