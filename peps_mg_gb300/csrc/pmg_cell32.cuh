@@ -527,11 +527,9 @@ __device__ void t32_sweeps(const LevelK<float> &L, float *x, const float *b, int
 __device__ void tail32_coarsest(const TailDesc<float> &D, const LevelK<float> &L, float *x, const float *b, double *sw)
 {
     const LevelK<double> &C = D.C64;
-    const int chip = chip_threads(C.nx, C.ny, C.nz);
-    const bool fma_form = C.nx * C.ny * C.nz <= 64;
-    if (chip > 0 && (D.coarse_solver != 0 || (chip <= (int)blockDim.x && (fma_form || C.mul64)))) {
-        // small coarsest level: in shared memory; levels of at most 64 cells take the FMA
-        // form of the RBGS solver (the FP32 cycle is not bound to the reference's bits)
+    const int chip = chip32_threads(C.nx, C.ny, C.nz);
+    if (chip > 0 && (D.coarse_solver != 0 || chip <= (int)blockDim.x)) {
+        // small coarsest level: in shared memory
         __shared__ double cs[5][kChipCoarseMax];
         const int total = (int)(C.sz * (C.nz + 2));
         for (int q = threadIdx.x; q < total; q += blockDim.x) cs[1][q] = 0.0;
@@ -544,12 +542,8 @@ __device__ void tail32_coarsest(const TailDesc<float> &D, const LevelK<float> &L
         if (D.coarse_solver != 0) {
             if (threadIdx.x < 32)
                 iters = coarse_cg_warp_f64(C, cs[0], cs[1], cs[2], cs[3], cs[4], D.coarse_maxit, D.tol, D.abort);
-        } else if (fma_form) {
-            iters = coarse_rbgs_chip<false, false>(C, cs, D.coarse_maxit, D.tol, D.omega64, D.omw64, D.abort, &xs64);
-        } else if (C.nx * C.ny * C.nz <= 128) {
-            iters = coarse_rbgs_chip<true, false>(C, cs, D.coarse_maxit, D.tol, D.omega64, D.omw64, D.abort, &xs64);
         } else {
-            iters = coarse_rbgs_chip<true, true>(C, cs, D.coarse_maxit, D.tol, D.omega64, D.omw64, D.abort, &xs64);
+            iters = coarse_rbgs_chip32(C, cs, D.coarse_maxit, D.tol, D.omega64, D.omw64, D.abort, &xs64);
         }
         if (threadIdx.x == 0 && D.iters_out) *D.iters_out = iters;
         __syncthreads();

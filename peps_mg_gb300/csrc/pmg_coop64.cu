@@ -282,8 +282,8 @@ __device__ void chip_tail(const Coop64Desc &D, double *sm)
         int xs;
         const int iters =
             C.nx * C.ny * C.nz > 128
-                ? coarse_rbgs_chip<true, true>(C, cs, D.coarse_maxit, D.tol, D.omega, D.omw, D.abort, &xs)
-                : coarse_rbgs_chip<true, false>(C, cs, D.coarse_maxit, D.tol, D.omega, D.omw, D.abort, &xs);
+                ? coarse_rbgs_chip<true>(C, cs, D.coarse_maxit, D.tol, D.omega, D.omw, D.abort, &xs)
+                : coarse_rbgs_chip<false>(C, cs, D.coarse_maxit, D.tol, D.omega, D.omw, D.abort, &xs);
         if (t0 == 0) *D.iters_out = iters;
         for (int q = t0; q < total; q += st) x[q] = cs[xs][q];
         __syncthreads();

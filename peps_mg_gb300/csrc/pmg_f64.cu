@@ -553,9 +553,9 @@ __global__ void __launch_bounds__(kTailThreads) k_tail_f64(const TailDesc<double
             }
             int xs;
             if (C.nx * C.ny * C.nz > 128)
-                iters = coarse_rbgs_chip<true, true>(C, cs, D.coarse_maxit, D.tol, D.omega64, D.omw64, D.abort, &xs);
+                iters = coarse_rbgs_chip<true>(C, cs, D.coarse_maxit, D.tol, D.omega64, D.omw64, D.abort, &xs);
             else
-                iters = coarse_rbgs_chip<true, false>(C, cs, D.coarse_maxit, D.tol, D.omega64, D.omw64, D.abort, &xs);
+                iters = coarse_rbgs_chip<false>(C, cs, D.coarse_maxit, D.tol, D.omega64, D.omw64, D.abort, &xs);
             for (int q = threadIdx.x; q < total; q += blockDim.x) D.cx64[q] = cs[xs][q];
         } else {
             iters = coarse_solve_f64(C, D.cx64, D.cb64, D.cp64, D.cap64, D.crr64, D.coarse_solver, D.coarse_maxit,

@@ -235,18 +235,15 @@ __device__ __forceinline__ double warp_sum_f64(double v)
 // sqrt(rn / r0) <= tol is decided by integer comparison with tol^2 r0 unless rn lies within
 // 2^-40 of it, where it is evaluated as written.
 //
-// REF: the reference's operation order, bit for bit (the level's mul64 flag must be set).  The
+// The reference's operation order, bit for bit (the level's mul64 flag must be set).  The
 // sweeps multiply on the FP64 unit: a lone warp is bound by fetching its instructions, and the
 // integer products' forty each made an iteration at 4^3 cells 1.9 us instead of 1.4.  INT_NORM
 // (levels of more than 128 cells, where the unit is shared by many warps) takes the norm's
 // products to the integer pipe.
-// Otherwise (the FP32 cycle's coarsest level of at most 64 cells): the neighbour sum as a
-// tree of FMAs and x = (omega/c0)(b - t) + (1-omega) x, for the shorter chain.
 //
-// Measured per iteration (one warp before, or a 64-thread block with both phases in turn and
-// an IEEE division per update): FMA form 2^3 cells 1.0 us and 4^3 1.15 us (4.6 us before);
-// REF 2^3 1.35 us, 4^3 1.4 us, 7 x 5 x 3 1.8 us (about 9 before), 8 x 6 x 4 2.2 us (about 14),
-// 8^3 4.8 us.
+// Measured per iteration (a 64-thread block with both phases in turn and an IEEE division per
+// update before): 2^3 cells 1.35 us, 4^3 1.4 us, 7 x 5 x 3 1.8 us (about 9 before), 8 x 6 x 4
+// 2.2 us (about 14), 8^3 4.8 us.
 // ---------------------------------------------------------------------------------------
 __device__ __forceinline__ void bar_named(int id, int threads)
 {
@@ -256,7 +253,7 @@ __device__ __forceinline__ void bar_named(int id, int threads)
 // cs: five shared arrays of the level's (nx+2)(ny+2)(nz+2) layout; cs[1] holds b (ghosts
 // zero), the others are scratch.  All threads of the block call it (at least chip_threads of
 // them).  Returns the iteration counter; *xsel = the array that holds the solution.
-template <bool REF, bool INT_NORM>
+template <bool INT_NORM>
 __device__ int coarse_rbgs_chip(const LevelK<double> &L, double (*cs)[kChipCoarseMax], int maxit, double tol,
                                 double omega, double omw, const volatile int *abort, int *xsel)
 {
@@ -276,7 +273,7 @@ __device__ int coarse_rbgs_chip(const LevelK<double> &L, double (*cs)[kChipCoars
         const int i = q % nx + 1, r2 = q / nx, j = r2 % ny + 1, k = r2 / ny + 1;
         const double c0 = diag_f64(L, i, j, k);
         cs[3][i + sy * j + sz * k] = c0;
-        cs[4][i + sy * j + sz * k] = REF ? recip_f64(c0) : __ddiv_rn(omega, c0);
+        cs[4][i + sy * j + sz * k] = recip_f64(c0);
     }
     __syncthreads();
     if (n == 1) {
@@ -312,26 +309,17 @@ __device__ int coarse_rbgs_chip(const LevelK<double> &L, double (*cs)[kChipCoars
         const bool omega1 = omega == 1.0;
         auto update = [&](int c, const double *nb, const double *own, double *out) {
             const int q = p[c];
-            double v;
-            if (REF) {
-                double s = __dmul_rn(cxm[c], nb[q - 1]);
-                s = __dadd_rn(s, __dmul_rn(cxp[c], nb[q + 1]));
-                s = __dadd_rn(s, __dmul_rn(cym, nb[q - sy]));
-                s = __dadd_rn(s, __dmul_rn(cyp, nb[q + sy]));
-                s = __dadd_rn(s, __dmul_rn(czm, nb[q - sz]));
-                s = __dadd_rn(s, __dmul_rn(czp, nb[q + sz]));
-                const double d = __dsub_rn(b[c], s);
-                if (omega1)
-                    v = add_zero_times_f64(quot64_dp(d, c0[c], y[c]), own[q]);
-                else
-                    v = __dadd_rn(quot64_dp(__dmul_rn(omega, d), c0[c], y[c]), __dmul_rn(omw, own[q]));
-            } else {
-                const double tx = fma(cxp[c], nb[q + 1], __dmul_rn(cxm[c], nb[q - 1]));
-                const double ty = fma(cyp, nb[q + sy], __dmul_rn(cym, nb[q - sy]));
-                const double tz = fma(czp, nb[q + sz], __dmul_rn(czm, nb[q - sz]));
-                const double s = __dadd_rn(__dadd_rn(tx, ty), tz);
-                v = fma(y[c], __dsub_rn(b[c], s), __dmul_rn(omw, own[q]));
-            }
+            double v, s = __dmul_rn(cxm[c], nb[q - 1]);
+            s = __dadd_rn(s, __dmul_rn(cxp[c], nb[q + 1]));
+            s = __dadd_rn(s, __dmul_rn(cym, nb[q - sy]));
+            s = __dadd_rn(s, __dmul_rn(cyp, nb[q + sy]));
+            s = __dadd_rn(s, __dmul_rn(czm, nb[q - sz]));
+            s = __dadd_rn(s, __dmul_rn(czp, nb[q + sz]));
+            const double d = __dsub_rn(b[c], s);
+            if (omega1)
+                v = add_zero_times_f64(quot64_dp(d, c0[c], y[c]), own[q]);
+            else
+                v = __dadd_rn(quot64_dp(__dmul_rn(omega, d), c0[c], y[c]), __dmul_rn(omw, own[q]));
             if (has[c]) out[q] = v;
         };
         bar_named(1, nthr);                // |r0| is formed beside nothing
@@ -363,27 +351,18 @@ __device__ int coarse_rbgs_chip(const LevelK<double> &L, double (*cs)[kChipCoars
                     k = r2 / ny + 1;
                 }
                 const int c = i + sy * j + sz * k;
-                double r;
-                if (REF) {
-                    auto term = [](double f, double v) {
-                        return INT_NORM ? mul64(mul64_factor(f), v) : __dmul_rn(f, v);
-                    };
-                    r = term(cs[3][c], x[c]);
-                    r = __dadd_rn(r, term(L.cxm[i], x[c - 1]));
-                    r = __dadd_rn(r, term(L.cxp[i], x[c + 1]));
-                    r = __dadd_rn(r, term(L.cym[j], x[c - sy]));
-                    r = __dadd_rn(r, term(L.cyp[j], x[c + sy]));
-                    r = __dadd_rn(r, term(L.czm[k], x[c - sz]));
-                    r = __dadd_rn(r, term(L.czp[k], x[c + sz]));
-                    r = __dsub_rn(cs[1][c], r);
-                    acc = fma(r, r, acc);
-                } else {
-                    const double tx = fma(L.cxp[i], x[c + 1], __dmul_rn(L.cxm[i], x[c - 1]));
-                    const double ty = fma(L.cyp[j], x[c + sy], __dmul_rn(L.cym[j], x[c - sy]));
-                    const double tz = fma(L.czp[k], x[c + sz], __dmul_rn(L.czm[k], x[c - sz]));
-                    r = __dsub_rn(cs[1][c], fma(cs[3][c], x[c], __dadd_rn(__dadd_rn(tx, ty), tz)));
-                    acc = fma(r, r, acc);
-                }
+                auto term = [](double f, double v) {
+                    return INT_NORM ? mul64(mul64_factor(f), v) : __dmul_rn(f, v);
+                };
+                double r = term(cs[3][c], x[c]);
+                r = __dadd_rn(r, term(L.cxm[i], x[c - 1]));
+                r = __dadd_rn(r, term(L.cxp[i], x[c + 1]));
+                r = __dadd_rn(r, term(L.cym[j], x[c - sy]));
+                r = __dadd_rn(r, term(L.cyp[j], x[c + sy]));
+                r = __dadd_rn(r, term(L.czm[k], x[c - sz]));
+                r = __dadd_rn(r, term(L.czp[k], x[c + sz]));
+                r = __dsub_rn(cs[1][c], r);
+                acc = fma(r, r, acc);
             }
             return acc;
         };
@@ -419,6 +398,168 @@ __device__ int coarse_rbgs_chip(const LevelK<double> &L, double (*cs)[kChipCoars
                 if (rt == 0) {
                     const long long v = __double_as_longlong(rn);
                     const bool pass = v <= lo || (v <= hi && sqrt(__ddiv_rn(rn, r0)) <= tol);
+                    // the flag is polled every 16 iterations
+                    const bool stop = !pass && (it & 15) == 0 && abort && *abort;
+                    if (pass || stop || it == maxit) {
+                        s_iters = pass || stop ? it - 1 : maxit;
+                        s_x = cur ? 2 : 0;
+                        s_flag = 1;
+                    }
+                }
+            }
+            bar_named(1, nthr);
+            if (s_flag) break;
+            cur ^= 1;
+        }
+    }
+    __syncthreads();
+    *xsel = s_x;
+    return s_iters;
+}
+
+// The same solve for the FP32 cycle, which is not bound to the reference's bits: same sweeps,
+// same exit test, fewer and shorter chains.
+//  * An update is v = (y b - tx) - (ty + tz) (+ (1 - omega) x) with y = omega / c0 and the
+//    neighbours' coefficients times y in registers: 9 FP64 instructions instead of 11 or 15 (a
+//    warp's take 64 clocks each, dependent or not).
+//  * The norm needs no second evaluation of A x: a cell's residual before its update is
+//    (v - x) / y, so the first colour's of an iterate come out of the next iteration's first
+//    half-sweep, and the second colour's, (1 - omega) times those before its own update, out
+//    of the iterate's last half-sweep (nothing for omega = 1).
+//  * One warp squares and sums them beside the second half-sweep.  The sum over its lanes is
+//    formed in FP32 from the leading 21 bits (a butterfly step of FP64 takes 90 clocks, of FP32
+//    30); within 2^-12 of the threshold, in FP64.
+// Measured per iteration: 7 x 5 x 3 cells 1.12 us (1.78 in coarse_rbgs_chip), 8 x 6 x 4 1.14
+// (2.16), 8^3 2.26 (4.8); 2^3 and 4^3 1.05 (1.02 and 1.15 with two evaluations of A x as FMAs).
+// Threads [0, P) sweep, [P, P + 32) sum; all threads of the block call it.
+__host__ __device__ inline int chip32_threads(int nx, int ny, int nz)
+{
+    if ((long long)(nx + 2) * (ny + 2) * (nz + 2) > kChipCoarseMax) return 0;
+    return chip_roles(nx, ny, nz).P + 32;
+}
+
+// A positive double with its exponent reduced by e0, truncated to FP32; 0 or a huge value where
+// that is out of range (NaN and infinity too).
+__device__ __forceinline__ float scaled_f32(double v, int e0)
+{
+    const int h = __double2hiint(v), e = (h >> 20) - e0;
+    const int bits = ((e + 127) << 23) | ((h & 0xfffff) << 3);
+    return __int_as_float(e < -126 ? 0 : e > 100 ? 0x7d000000 : bits);
+}
+
+__device__ int coarse_rbgs_chip32(const LevelK<double> &L, double (*cs)[kChipCoarseMax], int maxit, double tol,
+                                  double omega, double omw, const volatile int *abort, int *xsel)
+{
+    __shared__ int s_flag, s_iters, s_x;
+    const int nx = L.nx, ny = L.ny, nz = L.nz;
+    const int sy = L.sy, sz = (int)L.sz;
+    const int total = sz * (nz + 2);
+    const int tid = threadIdx.x;
+    for (int q = tid; q < total; q += blockDim.x) cs[0][q] = cs[2][q] = 0.0;
+    if (tid == 0) {
+        s_flag = 0;
+        s_iters = 0;
+        s_x = 0;
+    }
+    __syncthreads();
+    if (nx * ny * nz == 1) {
+        const int c = 1 + sy + sz;
+        if (tid == 0) cs[0][c] = __ddiv_rn(cs[1][c], diag_f64(L, 1, 1, 1));
+        __syncthreads();
+        *xsel = 0;
+        return 0;
+    }
+    const int P = chip_roles(nx, ny, nz).P, nthr = P + 32;
+    const bool omega1 = omega == 1.0;
+    // residuals by slot: the first colour's in cs[3], the second's in cs[4]
+    if (tid < P) {
+        const int hx = (nx + 1) / 2;
+        const int t = tid % hx, r2 = tid / hx, j = r2 % ny + 1, k = r2 / ny + 1;
+        const bool slot = tid < hx * ny * nz;
+        int p[2];
+        bool has[2];
+        double cxm[2], cxp[2], cym[2], cyp[2], czm[2], czp[2], yb[2], ry[2], xo[2];
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {      // first colour: i + j + k odd (src/rbgs_poisson_matrix.f90:242)
+            const int i = 2 * t + 1 + ((j + k + c) & 1);
+            has[c] = slot && i <= nx;
+            const int ii = has[c] ? i : 1, jj = has[c] ? j : 1, kk = has[c] ? k : 1;
+            p[c] = ii + sy * jj + sz * kk;
+            const double c0 = diag_f64(L, ii, jj, kk), y = __ddiv_rn(omega, c0);
+            ry[c] = __ddiv_rn(c0, omega);
+            cxm[c] = y * L.cxm[ii];
+            cxp[c] = y * L.cxp[ii];
+            cym[c] = y * L.cym[jj];
+            cyp[c] = y * L.cyp[jj];
+            czm[c] = y * L.czm[kk];
+            czp[c] = y * L.czp[kk];
+            yb[c] = y * cs[1][p[c]];
+            xo[c] = 0.0;
+        }
+        cs[3][tid] = has[0] ? cs[1][p[0]] : 0.0;     // of x = 0
+        cs[4][tid] = has[1] ? cs[1][p[1]] : 0.0;
+        auto update = [&](int c, const double *nb, double *out) {
+            const int q = p[c];
+            const double tx = fma(cxp[c], nb[q + 1], cxm[c] * nb[q - 1]);
+            const double ty = fma(cyp[c], nb[q + sy], cym[c] * nb[q - sy]);
+            const double tz = fma(czp[c], nb[q + sz], czm[c] * nb[q - sz]);
+            double v = (yb[c] - tx) - (ty + tz);
+            if (!omega1) v = fma(omw, xo[c], v);
+            if (has[c]) {
+                out[q] = v;
+                if (c == 0)
+                    cs[3][tid] = ry[0] * (v - xo[0]);
+                else if (!omega1)
+                    cs[4][tid] = omw * (ry[1] * (v - xo[1]));
+            }
+            xo[c] = v;
+        };
+        bar_named(1, nthr);
+        bar_named(1, nthr);                // the sum of b's squares is formed
+        int cur = 0;
+        for (int it = 0; it <= maxit; ++it) {
+            double *x = cs[cur ? 2 : 0], *xn = cs[cur ? 0 : 2];
+            update(0, x, xn);
+            bar_named(1, nthr);
+            if (it < maxit) update(1, xn, xn);
+            bar_named(1, nthr);
+            if (s_flag) break;
+            cur ^= 1;
+        }
+    } else if (tid < nthr) {
+        const int lane = tid - P;
+        auto squares = [&](const double *rr) {
+            double a = 0.0, a2 = 0.0;
+            for (int q = lane; q < P; q += 64) {
+                const double r = rr[q], r2 = q + 32 < P ? rr[q + 32] : 0.0;
+                a = fma(r, r, a);
+                a2 = fma(r2, r2, a2);
+            }
+            return a + a2;
+        };
+        bar_named(1, nthr);
+        const double r0 = warp_sum_f64(squares(cs[3]) + squares(cs[4]));
+        const double thr = __dmul_rn(__dmul_rn(tol, tol), r0);
+        const bool plain = thr >= 1e-250 && thr <= 1e250;
+        const int e0 = __double2hiint(thr) >> 20;
+        const float tf = scaled_f32(thr, e0), lo = tf * (1.f - 0x1p-12f), hi = tf * (1.f + 0x1p-12f);
+        bar_named(1, nthr);
+        int cur = 0;
+        for (int it = 0; it <= maxit; ++it) {
+            // the second colour's are overwritten beside the second half-sweep
+            const double acc1 = it > 0 && !omega1 ? squares(cs[4]) : 0.0;
+            bar_named(1, nthr);
+            if (it > 0) {
+                const double acc = squares(cs[3]) + acc1;
+                float f = scaled_f32(acc, e0);
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) f += __shfl_xor_sync(0xffffffffu, f, o);
+                bool pass = f < lo;
+                if (!plain || (f >= lo && f <= hi)) {
+                    const double rn = warp_sum_f64(acc);
+                    pass = sqrt(__ddiv_rn(rn, r0)) <= tol;
+                }
+                if (lane == 0) {
                     // the flag is polled every 16 iterations
                     const bool stop = !pass && (it & 15) == 0 && abort && *abort;
                     if (pass || stop || it == maxit) {

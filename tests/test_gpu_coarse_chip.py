@@ -1,6 +1,6 @@
 """The on-chip RBGS coarsest-level solver (coarse_rbgs_chip in pmg_tail64.cuh) at the edges of
 its range: FP64 solves against the oracle, bit for bit, with the oracle's coarsest iteration
-counts; mixed solves (whose coarsest levels of at most 64 cells take the FMA form) within 1e-8,
+counts; mixed solves (whose solver takes the norm from the sweeps) within 1e-8,
 twenty times the 5e-10 that a residual of 1e-10 leaves on these boxes."""
 import numpy as np
 import pytest
