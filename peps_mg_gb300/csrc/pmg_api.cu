@@ -781,9 +781,18 @@ int Ctx::build(const pmg_config_t *c, cudaStream_t s)
         // kernels read c0 instead of summing five 1-D table entries per cell, the values are
         // diag_f64's bits, and divide by it on the integer pipe)
         c0t.assign((size_t)nl + 1, nullptr);
+        const char *env = std::getenv("PEPS_MG_RECIPROCALS");   // =0: the diagonal alone
+        size_t free_bytes = 0, all_bytes = 0;
+        PMG_CUDA(cudaMemGetInfo(&free_bytes, &all_bytes), "free memory");
         for (int l = 0; l <= nl; ++l) {
-            PMG_CUDA(dev_malloc(&c0t[l], 2 * lv[l].total * sizeof(double)), "diagonal table");
-            PMG_CUDA(cudaMemsetAsync(c0t[l], 0, 2 * lv[l].total * sizeof(double), stream), "diagonal table");
+            // The reciprocals' 8 bytes a cell must not be what a box no longer fits for: they
+            // may take an eighth of the free memory (1600^3 cells on an empty 280 GB), else
+            // the level's kernels divide (kTab).
+            const size_t bytes = lv[l].total * sizeof(double);
+            if ((env && std::strcmp(env, "0") == 0) || bytes > free_bytes / 8) K[l].mul64 = 0;
+            const int tables = K[l].mul64 ? 2 : 1;
+            PMG_CUDA(dev_malloc(&c0t[l], tables * bytes), "diagonal table");
+            PMG_CUDA(cudaMemsetAsync(c0t[l], 0, tables * bytes, stream), "diagonal table");
             PMG_TRY(f64_diag_table(K[l], c0t[l], stream));
         }
         // complete before any other stream (a decomposed solve's) reads the tables

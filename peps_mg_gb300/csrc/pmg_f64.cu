@@ -131,8 +131,8 @@ __global__ void __launch_bounds__(kBX *kBY, MODE == kInt ? 7 : 6) k_rbgs_f64(Lev
             }
 }
 
-// c0t = the diagonal of every interior cell (diag_f64), then as many values again its
-// reciprocals (recip64); the ghosts are left as they are.  A thread marches its column of
+// c0t = the diagonal of every interior cell (diag_f64), then, for the integer quotients (mul64),
+// as many values again its reciprocals (recip64); the ghosts are left as they are.  A thread marches its column of
 // planes and forms the two values anew only where the plane's z coefficients differ from
 // those of the plane before: on a uniform z axis once a chunk.  A context of 384^3 is then
 // created in 2.48 ms, 2.39 without the reciprocals.
@@ -148,11 +148,11 @@ __global__ void __launch_bounds__(kBX *kBY) k_diag_f64(LevelK<double> L, double 
                 if (k == k0 || __double_as_longlong(L.czm[k]) != __double_as_longlong(L.czm[k - 1]) ||
                     __double_as_longlong(L.czp[k]) != __double_as_longlong(L.czp[k - 1])) {
                     c0 = diag_f64(L, i, j, k);
-                    y = __longlong_as_double((long long)recip64(c0));
+                    if (L.mul64) y = __longlong_as_double((long long)recip64(c0));
                 }
                 const long long p = lin(i, j, k, L.sy, L.sz);
                 c0t[p] = c0;
-                c0t[p + total] = y;
+                if (L.mul64) c0t[p + total] = y;
             }
         }
 }
@@ -211,8 +211,8 @@ __global__ void __launch_bounds__(1024) k_reduce_f64(const double *__restrict__ 
 // M64: products on the integer pipe; otherwise (weights beyond mul64's range) restrict_cell_f64.
 // A thread takes the coarse cells of one column (i, j) over a chunk of planes, so the weights'
 // x-y products are formed once, and the full weights, their sum and its reciprocal only where
-// the plane's weights change: on a uniform z axis a coarse cell keeps 9 of 43 FP64
-// instructions (324 x 258 x 194, stretched: 192 -> 99 us; at 64 registers, four CTAs an SM, and
+// the plane's weights change: on a uniform z axis a coarse cell keeps 7 of 43 FP64
+// instructions (324 x 258 x 194, stretched: 192 -> 90 us; at 64 registers, four CTAs an SM, and
 // 106 at the 108 it would take).
 template <bool M64>
 __global__ void __launch_bounds__(kBX *kBY, 4) k_restrict_f64(XferK<double> X, const double *__restrict__ vf,

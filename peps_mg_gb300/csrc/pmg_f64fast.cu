@@ -1,19 +1,19 @@
 // pmg_f64fast.cu -- the FP64 performance mode (PMG_FP64_FAST): the plain FP64 V-cycle with
 // fewer FP64 instructions per cell, not bound to the reference's bits.
 //
-// The bitwise kernels (pmg_f64.cu) are FP64-pipe bound on this part (83-86% of the FP64
-// pipe, 2-11% of HBM): an RBGS update costs 28 FP64 instructions there, an IEEE division
-// among them.  This mode changes only the arithmetic of the grid levels, in three ways:
+// The bitwise kernels (pmg_f64.cu) are bound by this part's FP64 pipe, and form their products
+// and quotients on the integer pipe to relieve it.  This mode changes only the arithmetic of
+// the grid levels, in three ways:
 //   * FMA chains: b - sum c_n x_n as six DFMA, b - A x as seven;
 //   * the diagonal enters as a stored per-cell factor omega / c0 (an FP64 array per grid
-//     level, rebuilt when omega changes), so an update needs no division: 7 FP64
-//     instructions for omega = 1, 8 otherwise;
+//     level, rebuilt when omega changes), so an update needs no division: 6 FP64
+//     instructions for omega = 1, 7 otherwise, its last product on the integer pipe;
 //   * restriction and prolongation use per-axis weights normalised once at set-up: the
 //     reference's volume weights are products of per-axis widths and their sums products
 //     of per-axis sums (src/multigrid.f90:1474-1491, :1676-1754), so sum(V r)/sum(V) and
 //     sum(w V)/prod(sum w) factor into three nested 2-term interpolations (14 FP64
-//     instructions per coarse cell for the restriction, about 12 per fine cell for the
-//     prolongation instead of 46 and 40).
+//     instructions per coarse cell for the restriction, 26 for the eight children of the
+//     prolongation).
 // The coarse tail (single CTA) is the bitwise one.  The level sequence, the exit test
 // and the reductions' order are those of the plain path, so the solve converges in the
 // same number of cycles to the same solution within rounding (the tests bound the

@@ -118,7 +118,7 @@ int f64_rbgs_sweeps(const LevelK<double> &L, const Launch &ln, double *x, const 
 int f64_rbgs_colour(const LevelK<double> &L, const Launch &ln, double *x, const double *b, double omega, int colour,
                     cudaStream_t s, const double *c0t = nullptr);
 // c0t = diag_f64 of every interior cell of level L (an array of the level's layout), followed
-// by an array of its reciprocals (recip64).
+// by an array of its reciprocals (recip64) where the level's mul64 flag is set.
 int f64_diag_table(const LevelK<double> &L, double *c0t, cudaStream_t s);
 // r = b - A x (interior); if partials != nullptr also writes per-block sums of r^2
 // and returns the number of partials in *npart.

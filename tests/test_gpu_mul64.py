@@ -101,3 +101,23 @@ def test_diagonal_of_a_column(nz):
         got = to_dev(x)
         mg.rbgs_iterator(0, got, to_dev(b), 1, 1.0)
     assert same(from_dev(got), want)
+
+
+@pytest.mark.parametrize("n", [(20, 12, 8), (64, 48, 40)], ids=str)
+def test_without_reciprocals(n, monkeypatch):
+    """Contexts whose levels are too large for the table of reciprocals: the same bits."""
+    rng = np.random.Generator(np.random.PCG64(3))
+    axes = meshes("random", n, rng)
+    rhs = G.field(*n)
+    rhs[1:-1, 1:-1, 1:-1] = rng.uniform(-1.0, 1.0, n)
+    out = []
+    for value in ("1", "0"):
+        monkeypatch.setenv("PEPS_MG_RECIPROCALS", value)
+        with pmg.Multigrid(axes, 2, 20) as mg:
+            sol, rsd, x = (to_dev(G.field(*n)) for _ in range(3))
+            rep = mg.solve_vcycle(sol, rsd, to_dev(rhs), 2, 1e-9, 1.1)
+            mg.rbgs_iterator(0, x, to_dev(rhs), 2, 1.0)
+        out.append((from_dev(sol), from_dev(rsd), from_dev(x), rep.cycles, list(rep.coarse_iterations)))
+    assert out[0][3:] == out[1][3:]
+    for a, b in zip(out[0][:3], out[1][:3]):
+        assert same(a, b)
