@@ -676,11 +676,6 @@ dim3 grid3(int nx_threads, int ny, int nz, const Launch &ln)
 
 }  // namespace
 
-// Planes per chunk of a sweep, whose column shares little: 256^3 141.4 us a half-sweep with 8
-// (3.4 rounds of CTAs, the last one a third full), 135.4 with 3, 139.0 with 1; 384^3 438.8,
-// 434.8, 457.0.
-static constexpr int kSweepPlanes = 3;
-
 void grid_for_cells(const LevelK<double> &L, const Launch &ln, dim3 *grid, dim3 *block)
 {
     *grid = grid3(L.nx, L.ny, L.nz, ln);

@@ -48,18 +48,21 @@ __global__ void __launch_bounds__(kBX *kBY) k_fast_wdiag(LevelK<double> L, doubl
 
 // One colour of the red-black sweep (colour 0: (i+j+k) odd first, as the bitwise kernel).
 // Bound by the latency of its loads (FP64 unit about half busy), so six CTAs per SM: 320 x 256
-// x 192, finest level, 123 -> 112 us.
+// x 192, finest level, 123 -> 112 us.  Chunks of three planes: a half-sweep of that solve, over
+// all levels, 21.5 -> 19.1 us.
 template <bool OMEGA1>
 __global__ void __launch_bounds__(kBX *kBY, 6) k_rbgs_fast(LevelK<double> L, const double *__restrict__ wd,
                                                         double *__restrict__ x, const double *__restrict__ b,
                                                         double omw, int colour)
 {
-    for (int k = blockIdx.z + 1; k <= L.nz; k += gridDim.z)
-        for (int j = blockIdx.y * blockDim.y + threadIdx.y + 1; j <= L.ny; j += gridDim.y * blockDim.y) {
-            const int ista = 1 + ((j + k + colour) & 1);
-            const double cym = L.cym[j], cyp = L.cyp[j], czm = L.czm[k], czp = L.czp[k];
-            for (int i = ista + 2 * (blockIdx.x * blockDim.x + threadIdx.x); i <= L.nx;
-                 i += 2 * gridDim.x * blockDim.x) {
+    int k0, k1;
+    plane_chunk(L.nz, k0, k1);
+    for (int j = blockIdx.y * blockDim.y + threadIdx.y + 1; j <= L.ny; j += gridDim.y * blockDim.y)
+        for (int t = blockIdx.x * blockDim.x + threadIdx.x; 2 * t < L.nx; t += gridDim.x * blockDim.x)
+            for (int k = k0; k <= k1; ++k) {
+                const int i = 2 * t + 1 + ((j + k + colour) & 1);
+                if (i > L.nx) continue;
+                const double cym = L.cym[j], cyp = L.cyp[j], czm = L.czm[k], czp = L.czp[k];
                 const long long p = lin(i, j, k, L.sy, L.sz);
                 double acc = fma(-L.cxm[i], x[p - 1], b[p]);
                 acc = fma(-L.cxp[i], x[p + 1], acc);
@@ -71,7 +74,6 @@ __global__ void __launch_bounds__(kBX *kBY, 6) k_rbgs_fast(LevelK<double> L, con
                 // instructions instead of 7
                 x[p] = OMEGA1 ? mul64_vv(wd[p], acc) : fma(wd[p], acc, mul64_vv(omw, x[p]));
             }
-        }
 }
 
 // r = b - A x with -c0 = sx(i) + dy(j) + dz(k); with NORM the per-block sums of r^2.  A thread
@@ -302,7 +304,7 @@ int fast_rbgs_sweeps(const LevelK<double> &L, const FastLevelK &F, const Launch 
                      int iters, double omega, cudaStream_t s)
 {
     const double omw = 1.0 - omega;
-    const dim3 g = grid3f((L.nx + 1) / 2, L.ny, L.nz, ln), bl(kBX, kBY, 1);
+    const dim3 g = grid_columns((L.nx + 1) / 2, L.ny, L.nz, ln, 1, false, kSweepPlanes), bl(kBX, kBY, 1);
     for (int it = 0; it < iters; ++it)
         for (int c = 0; c < 2; ++c) {
             if (omega == 1.0)

@@ -102,6 +102,10 @@ struct HierDesc {
 };
 
 bool exponents_within(const double *v, int n, int e);   // pmg_api.cu
+// Planes per chunk of a sweep, whose column shares little: 256^3 141.4 us a half-sweep with 8
+// (3.4 rounds of CTAs, the last one a third full), 135.4 with 3, 139.0 with 1; 384^3 438.8,
+// 434.8, 457.0.
+constexpr int kSweepPlanes = 3;
 // Grid of the FP64 column kernels (32 x 8 threads, plane_chunk), pmg_f64.cu.
 dim3 grid_columns(int nx_threads, int ny, int nz, const Launch &ln, int kc_min = 1, bool sum = false,
                   int kc_max = 8);
