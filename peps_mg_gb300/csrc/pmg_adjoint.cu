@@ -46,7 +46,7 @@ constexpr int kBX = 32, kBY = 8;
 // out = in / vol on the interior (DIV) or vol * in, vol = dxm(i) dym(j) dzm(k).  A thread takes a
 // column over a chunk of planes and forms vol and its reciprocal where the plane's width
 // changes; INT (widths within mul64's range) then leaves no FP64 instruction of a division or a
-// product, with the same bits (quot64, mul64, pmg_mul64.cuh).  256^3: 201 -> 91 us (a
+// product, with the same bits (quot64, mul64, pmg_mul64.cuh).  256^3: 201 -> 87 us (a
 // division), 201 -> 70 (a product).
 template <bool DIV, bool INT>
 __global__ void __launch_bounds__(kBX *kBY) k_volume_scale(int nx, int ny, int nz, int sy, long long sz,

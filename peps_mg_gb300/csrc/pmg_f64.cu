@@ -144,10 +144,11 @@ __global__ void __launch_bounds__(kBX *kBY) k_diag_f64(LevelK<double> L, double 
     for (int j = blockIdx.y * blockDim.y + threadIdx.y + 1; j <= L.ny; j += gridDim.y * blockDim.y)
         for (int i = blockIdx.x * blockDim.x + threadIdx.x + 1; i <= L.nx; i += gridDim.x * blockDim.x) {
             double c0 = 0.0, y = 0.0;   // y: the bits of recip64
+            const double sxy = __dadd_rn(__dadd_rn(L.sx[i], L.cym[j]), L.cyp[j]);
             for (int k = k0; k <= k1; ++k) {
                 if (k == k0 || __double_as_longlong(L.czm[k]) != __double_as_longlong(L.czm[k - 1]) ||
                     __double_as_longlong(L.czp[k]) != __double_as_longlong(L.czp[k - 1])) {
-                    c0 = diag_f64(L, i, j, k);
+                    c0 = -__dadd_rn(__dadd_rn(sxy, L.czm[k]), L.czp[k]);   // diag_f64
                     if (L.mul64) y = __longlong_as_double((long long)recip64(c0));
                 }
                 const long long p = lin(i, j, k, L.sy, L.sz);
@@ -212,7 +213,7 @@ __global__ void __launch_bounds__(1024) k_reduce_f64(const double *__restrict__ 
 // A thread takes the coarse cells of one column (i, j) over a chunk of planes, so the weights'
 // x-y products are formed once, and the full weights, their sum and its reciprocal only where
 // the plane's weights change: on a uniform z axis a coarse cell keeps 7 of 43 FP64
-// instructions (324 x 258 x 194, stretched: 192 -> 90 us; at 64 registers, four CTAs an SM, and
+// instructions (324 x 258 x 194, stretched: 192 -> 87 us; at 64 registers, four CTAs an SM, and
 // 106 at the 108 it would take).
 template <bool M64>
 __global__ void __launch_bounds__(kBX *kBY, 4) k_restrict_f64(XferK<double> X, const double *__restrict__ vf,

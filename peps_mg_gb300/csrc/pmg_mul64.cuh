@@ -172,19 +172,31 @@ __device__ __forceinline__ double mul64_vv(double a, double b)
 
 // Y = floor(2^116 / C), C the 53-bit significand of c: the leading 64 bits of c's reciprocal,
 // for quot64; 0 if c's exponent lies beyond 2^+-400, and 2^64 - 1 for 2^64 (c a power of two).
+// An FP32 reciprocal of the truncated significand (2^-22 off) and one Newton step leave Y0
+// within 2^21 of it; the rest comes from the exact remainder 2^116 - Y0 C, of 74 bits.  Two FP64
+// instructions instead of an IEEE reciprocal's eight or so: a context of 224^3 cells on a
+// non-uniform z axis is created in 0.91 instead of 1.03 ms (0.77 without reciprocals).
 __device__ __forceinline__ unsigned long long recip64(double c)
 {
     const unsigned long long one = 1ULL << 52;
+    const unsigned ch = (unsigned)__double2hiint(c), cl = (unsigned)__double2loint(c);
     const unsigned long long C = ((unsigned long long)__double_as_longlong(c) & (one - 1)) | one;
-    const unsigned e = ((unsigned)__double2hiint(c) >> 20) & 0x7ffu;
-    // RN(1/c) is within 2^10 of it, so 2^116 - Y0 C fits 64 bits
-    const double y = __drcp_rn(c);
-    const unsigned long long Y0 = (((unsigned long long)__double_as_longlong(y) & (one - 1)) | one) << 11;
-    const long long r = -(long long)(Y0 * C);
-    long long t = (long long)__float2int_rd(__fmul_rn(__ll2float_rn(r), __frcp_rn(__ull2float_rn(C))));
-    const long long rest = r - t * (long long)C;
+    const double m = __hiloint2double((int)((ch & 0xfffffu) | 0x3ff00000u), (int)cl);
+    const float r0 = __frcp_rn(__uint_as_float(0x3f800000u | (ch & 0xfffffu) << 3 | cl >> 29));   // (0.5, 1]
+    const unsigned rb = __float_as_uint(r0);
+    const double y0 = __hiloint2double((int)((rb >> 3) + (896u << 20)), (int)(rb << 29));
+    const double y1 = __fma_rn(y0, __fma_rn(-m, y0, 1.0), y0);
+    const int down = 1022 - (__double2hiint(y1) >> 20);       // 1 where y1 < 1/2, -1 where y1 >= 1
+    const unsigned long long M = ((unsigned long long)__double_as_longlong(y1) & (one - 1)) | one;
+    const unsigned long long Y0 = down < 0 ? ~0ULL : (M << 11) >> down;
+    const unsigned long long lo = Y0 * C;
+    const long long rh = (long long)(one - __umul64hi(Y0, C) - (lo != 0ULL));
+    const unsigned long long rl = 0ULL - lo;
+    const float rf = __ll2float_rn((long long)((unsigned long long)rh << 32 | rl >> 32));
+    long long t = __float2ll_rd(__fmul_rn(rf, __frcp_rn(__fmul_rn(__ull2float_rn(C), 0x1p-32f))));
+    const long long rest = (long long)(rl - (unsigned long long)t * C);
     t += rest < 0 ? -1 : rest >= (long long)C ? 1 : 0;
-    if (e - 623u > 800u) return 0ULL;
+    if (((ch >> 20) & 0x7ffu) - 623u > 800u) return 0ULL;
     return C == one ? ~0ULL : Y0 + (unsigned long long)t;
 }
 

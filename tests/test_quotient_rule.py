@@ -87,8 +87,6 @@ def quot_by_bits(D, C):
     """quot64 on 53-bit significands: the quotient's significand (53 bits) and its exponent
     less 52, or None where the kernel takes the IEEE division."""
     Y = min(2 ** 116 // C, 2 ** 64 - 1)
-    y0 = int(rn(Fraction(2 ** 116, C)))          # the kernel's start: 2^10 away at most
-    assert C == 2 ** 52 or abs(2 ** 116 - y0 * C) < 2 ** 63
     P, e = D * Y, 0
     if P < 2 ** 116:
         P, e = 2 * P, -1
@@ -122,3 +120,32 @@ def test_quotient_by_integers(kind):
         assert q is None or q == rn(Fraction(D, C)), (D, C)
     if kind in ("random", "short"):
         assert left <= len(pairs) // 100         # about one in a thousand takes the division
+
+
+def recip_bits(C):
+    """recip64 step by step: FP32 seed, one Newton step, exact remainder."""
+    f32 = np.float32
+    m = Fraction(C, 2 ** 52)
+    r0 = f32(1) / f32(1 + ((C >> 29) & 0x7fffff) / 2 ** 23)
+    y0 = Fraction(float(r0))
+    y1 = rn(y0 * rn(1 - m * y0) + y0)
+    Y0 = 2 ** 64 - 1 if y1 >= 1 else int(y1 * 2 ** 64)
+    rem = 2 ** 116 - Y0 * C
+    assert abs(rem >> 64) < 2 ** 31
+    scale = f32(1) / (f32(C) * f32(2.0 ** -32))
+    t = int(np.floor(f32(rem >> 32) * scale))
+    rest = (rem - t * C) % 2 ** 64
+    rest -= 2 ** 64 if rest >= 2 ** 63 else 0
+    assert rest == rem - t * C
+    t += -1 if rest < 0 else 1 if rest >= C else 0
+    return 2 ** 64 - 1 if C == 2 ** 52 else Y0 + t
+
+
+def test_reciprocal_bits():
+    rng = np.random.Generator(np.random.PCG64(17))
+    one = 2 ** 52
+    few = [int(v) << (53 - int(v).bit_length()) for v in range(1, 400)]
+    ends = [one + k for k in range(300)] + [2 * one - 1 - k for k in range(300)]
+    steps = [one + (k << 29) + d for k in range(0, 2 ** 23, 65521) for d in (0, 1, 2 ** 29 - 1)]
+    for C in few + ends + steps + [int(v) for v in rng.integers(one, 2 * one, size=4000)]:
+        assert recip_bits(C) == min(2 ** 116 // C, 2 ** 64 - 1), C
