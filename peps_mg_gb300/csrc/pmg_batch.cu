@@ -258,6 +258,7 @@ __global__ void __launch_bounds__(NTB) k_batch_nonzero(const double *__restrict_
 // problem's partials in that order.
 constexpr int kOuterWarps = NTB / 32;
 constexpr int kOuterCells = 8192;
+constexpr int kMarchPlanes = 8;
 
 struct OItem {
     int p, j0, j1, k0, k1;
@@ -323,6 +324,12 @@ __global__ void __launch_bounds__(NTB, 4) k_batch_outer_residual(const BOuter *_
 // FP32 copy of r and the warps' partial norms (FP32 sums of the squares scaled by a power
 // of two set by the problem's initial residual; they only decide whether the residual is
 // recomputed).  Problems in mode 1 get the FP64 residual recomputed after this.
+//
+// An item is up to 8 rows, one a warp, of a chunk of kMarchPlanes planes: a lane marches its
+// column with e of three planes in registers and the next plane's loads in flight, as the single
+// grid's k_update_residual_march does.  128 problems, 116.9 M cells: 1.48 -> 1.19 ms (row by row
+// before; chunks of 16 planes 1.20, 32 1.35, 64 1.51, whose items are too few and uneven; three
+// CTAs per SM 1.28).
 __global__ void __launch_bounds__(NTB, 4) k_batch_correct(const BOuter *__restrict__ po,
                                                           const OItem *__restrict__ items, int nitems,
                                                           double *__restrict__ partials,
@@ -355,27 +362,57 @@ __global__ void __launch_bounds__(NTB, 4) k_batch_correct(const BOuter *__restri
         const float nscale = ldexpf(1.0f, -ex);
         const SplitCoef C = O.sc;
         float acc32 = 0.f;
-        for (int t = wid; t < rows; t += kOuterWarps) {
-            const int j = w.j0 + t % nrow, k = w.k0 + t / nrow;
-            const long long row = lin(0, j, k, L.sy, L.sz), row32 = lin(0, j, k, sy32, sz32);
-            const float2 cym = C.cym[j], cyp = C.cyp[j], czm = C.czm[k], czp = C.czp[k];
+        for (int j = w.j0 + wid; j <= w.j1; j += kOuterWarps) {
+            const float2 cym = C.cym[j], cyp = C.cyp[j];
             for (int i = 1 + lane; i <= L.nx; i += 32) {
-                const long long c = row32 + i;
-                const float ec = e[c];
-                float S = 0.f, Sl = 0.f;
-                comp_term(C.cxm[i], e[c - 1], ec, S, Sl);
-                comp_term(C.cxp[i], e[c + 1], ec, S, Sl);
-                comp_term(cym, e[c - sy32], ec, S, Sl);
-                comp_term(cyp, e[c + sy32], ec, S, Sl);
-                comp_term(czm, e[c - sz32], ec, S, Sl);
-                comp_term(czp, e[c + sz32], ec, S, Sl);
-                x[row + i] = x[row + i] + f32_to_f64(ec);
-                const double v = __dsub_rn(__dsub_rn(r[row + i], f32_to_f64_fast(S)), f32_to_f64_fast(Sl));
-                r[row + i] = v;
-                const float v32 = f64_to_f32_rn(v);
-                r32[c] = v32;
-                const float wv = v32 * nscale;
-                acc32 = fmaf(wv, wv, acc32);
+                const float2 cm = C.cxm[i], cp = C.cxp[i];
+                const long long c0 = lin(i, j, 0, sy32, sz32), f0 = lin(i, j, 0, L.sy, L.sz);
+                const float *ec = e + c0;
+                float *rc32 = r32 + c0;
+                double *xc = x + f0, *rc = r + f0;
+                // plane k: e below (em), at (ev), above (ep); its x/y neighbours, x and r
+                float em = ec[sz32 * (w.k0 - 1)], ev = ec[sz32 * w.k0], ep = ec[sz32 * (w.k0 + 1)];
+                float xl = ec[sz32 * w.k0 - 1], xr = ec[sz32 * w.k0 + 1];
+                float yd = ec[sz32 * w.k0 - sy32], yu = ec[sz32 * w.k0 + sy32];
+                double xv = xc[L.sz * w.k0], rv = rc[L.sz * w.k0];
+                for (int k = w.k0; k <= w.k1; ++k) {
+                    // plane k+1's loads (its upper neighbour is plane k+2 <= nz+1)
+                    float ep2 = 0.f, nxl = 0.f, nxr = 0.f, nyd = 0.f, nyu = 0.f;
+                    double nxv = 0.0, nrv = 0.0;
+                    if (k < w.k1) {
+                        const long long o = sz32 * (k + 1);
+                        ep2 = ec[o + sz32];
+                        nxl = ec[o - 1];
+                        nxr = ec[o + 1];
+                        nyd = ec[o - sy32];
+                        nyu = ec[o + sy32];
+                        nxv = xc[L.sz * (k + 1)];
+                        nrv = rc[L.sz * (k + 1)];
+                    }
+                    float S = 0.f, Sl = 0.f;
+                    comp_term(cm, xl, ev, S, Sl);
+                    comp_term(cp, xr, ev, S, Sl);
+                    comp_term(cym, yd, ev, S, Sl);
+                    comp_term(cyp, yu, ev, S, Sl);
+                    comp_term(C.czm[k], em, ev, S, Sl);
+                    comp_term(C.czp[k], ep, ev, S, Sl);
+                    xc[L.sz * k] = xv + f32_to_f64(ev);
+                    const double v = __dsub_rn(__dsub_rn(rv, f32_to_f64_fast(S)), f32_to_f64_fast(Sl));
+                    rc[L.sz * k] = v;
+                    const float v32 = f64_to_f32_rn(v);
+                    rc32[sz32 * k] = v32;
+                    const float wv = v32 * nscale;
+                    acc32 = fmaf(wv, wv, acc32);
+                    em = ev;
+                    ev = ep;
+                    ep = ep2;
+                    xl = nxl;
+                    xr = nxr;
+                    yd = nyd;
+                    yu = nyu;
+                    xv = nxv;
+                    rv = nrv;
+                }
             }
         }
         const double s = warp_sum_outer((double)acc32 / ((double)nscale * (double)nscale));
@@ -511,9 +548,9 @@ struct Batch {
     struct OList {
         OItem *d = nullptr;
         int n = 0;
-    } outer;                                // row sets of the finest level
+    } outer, march;                         // row sets of the finest level; of marched columns
     std::vector<int> first_item;            // per problem range of the outer partials (kOuterWarps per item)
-    int *d_first = nullptr;
+    int *d_first = nullptr, *d_first_march = nullptr;
     double *d_partials = nullptr, *d_res0 = nullptr, *d_ratio = nullptr;
     int *d_done = nullptr, *d_cycles = nullptr, *d_ndone = nullptr;
     // the V-cycles' problem mask (done, or stopped early within a correction) and the
@@ -559,7 +596,9 @@ Batch::~Batch()
     for (auto &l : xfer_rr) dev_free(l.d);
     for (auto &l : xfer_pr) dev_free(l.d);
     dev_free(outer.d);
+    dev_free(march.d);
     dev_free(d_first);
+    dev_free(d_first_march);
     dev_free(d_partials);
     dev_free(d_res0);
     dev_free(d_ratio);
@@ -950,7 +989,25 @@ int batch_create(Batch **out, int n, const int *dims, const double *const *meshe
         PMG_TRY_B(upload(it, &B->outer.d));
         PMG_TRY_B(upload(B->first_item, &B->d_first));
     }
-    PMG_TRY_B(cuda_status(dev_malloc(&B->d_partials, (size_t)B->outer.n * kOuterWarps * sizeof(double)),
+    {
+        // items of k_batch_correct
+        std::vector<OItem> it;
+        std::vector<int> first((size_t)n + 1, 0);
+        for (int p = 0; p < n; ++p) {
+            first[p] = (int)it.size() * kOuterWarps;
+            const int *nn = B->probs[p]->lv[0].n;
+            for (int k0 = 1; k0 <= nn[2]; k0 += kMarchPlanes)
+                for (int j0 = 1; j0 <= nn[1]; j0 += kOuterWarps)
+                    it.push_back({p, j0, std::min(nn[1], j0 + kOuterWarps - 1), k0,
+                                  std::min(nn[2], k0 + kMarchPlanes - 1)});
+        }
+        first[n] = (int)it.size() * kOuterWarps;
+        B->march.n = (int)it.size();
+        PMG_TRY_B(upload(it, &B->march.d));
+        PMG_TRY_B(upload(first, &B->d_first_march));
+    }
+    PMG_TRY_B(cuda_status(dev_malloc(&B->d_partials,
+                                     (size_t)std::max(B->outer.n, B->march.n) * kOuterWarps * sizeof(double)),
                           "batch allocation"));
     PMG_TRY_B(cuda_status(dev_malloc(&B->d_res0, n * sizeof(double)), "batch allocation"));
     PMG_TRY_B(cuda_status(dev_malloc(&B->d_ratio, n * sizeof(double)), "batch allocation"));
@@ -1134,9 +1191,9 @@ static void batch_outer(Batch &B, bool first, double tol, int max_cycles)
         count_launches(3);
         return;
     }
-    k_batch_correct<<<grid_for(B.outer.n), NTB, 0, B.stream>>>(B.d_outer, B.outer.d, B.outer.n, B.d_partials,
+    k_batch_correct<<<grid_for(B.march.n), NTB, 0, B.stream>>>(B.d_outer, B.march.d, B.march.n, B.d_partials,
                                                                B.d_done, B.d_mode, B.d_res0);
-    k_batch_norms_update<<<n, NTB, 0, B.stream>>>(B.d_partials, B.d_first, B.d_res0, B.d_done, B.d_mode, B.d_cycles,
+    k_batch_norms_update<<<n, NTB, 0, B.stream>>>(B.d_partials, B.d_first_march, B.d_res0, B.d_done, B.d_mode, B.d_cycles,
                                                   B.d_check, B.d_cheap, tol, max_cycles);
     k_batch_outer_residual<<<grid_for(B.outer.n), NTB, 0, B.stream>>>(B.d_outer, B.outer.d, B.outer.n, B.d_partials,
                                                                       B.d_done, B.d_check, nullptr);
